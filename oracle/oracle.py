@@ -39,10 +39,10 @@ def reference_tree() -> str:
 
 
 def build_reference() -> bool:
-    """Build oracle/_ref from the reference tree when it is present.  Returns whether the
-    library exists afterwards."""
+    """Build oracle/_ref from the reference tree when it is present (an empty directory in its
+    place counts as absent).  Returns whether the library exists afterwards."""
     ref = reference_tree()
-    if os.path.isdir(ref):
+    if os.path.isdir(os.path.join(ref, "RTLib")):
         subprocess.check_call(["make", "-s", "-C", os.path.join(HERE, "ref"), f"REF={ref}"],
                               stdout=subprocess.DEVNULL)
     return os.path.exists(REF_SO)
