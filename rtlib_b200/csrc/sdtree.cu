@@ -61,14 +61,54 @@ __global__ void k_stree_top(SDTreeDev t) {
 }
 
 // ------------------------------------------------------------------ record
-// One thread per record (grid-stride, warp-uniform trip count so that the warp-aggregated
-// atomics run converged).  Two 64-bit fixed-point atomics per record: the DTree's stat-weight
-// and the leaf quadrant sum (RecordIrradiance, PG.h:417-428).  When the whole tree is small
-// (at most kPrivQuads quadrants and kPrivTrees DTrees) every CTA accumulates in shared memory
-// and flushes once, which removes the same-address contention of a freshly cleared tree.
-constexpr uint32_t kPrivQuads = 2048;
-constexpr uint32_t kPrivTrees = 512;
-constexpr uint32_t kStageSTreeRecord = 4096;  // 16 KB + 16 KB + 4 KB of static shared memory
+// One thread per record, grid-stride.  Two 64-bit fixed-point adds per record: the DTree's
+// stat-weight and the leaf quadrant sum (RecordIrradiance, PG.h:417-428).  Where they go depends
+// on the size of the tree, read from its device-side counts:
+//   root only (a cleared tree: one DTree, four quadrants): every thread sums its records in five
+//     registers and adds them once; the position cannot matter, so it is not read either.
+//     Shared-memory adds to five counters by every lane were all contention.
+//   small (its quadrants and DTrees fit kPrivSums counters): per-CTA sums in shared memory,
+//     flushed once per CTA;
+//   larger: the stat-weights, a few hundred counters hit by every record, still go to shared
+//     memory while they fit; the quadrant sums go to the tree with plain 64-bit atomics.  Keys
+//     spread over thousands of quadrants gain nothing from warp aggregation, and its 64-bit
+//     match costs more than the add it saves.
+// Two passes of 2^20 records (24 B each): 208.6 us when the first pass added through shared memory
+// and the second through warp-aggregated global atomics, 47.6 us now (15.1 the root-only pass,
+// 32.5 the refined one).
+constexpr uint32_t kPrivSums = 2560;
+constexpr uint32_t kStageSTreeRecord = 4096;  // 16 KB + 20 KB of static shared memory
+
+// what one record adds: its stat-weight, and its irradiance where that is finite and positive
+struct RecordIn {
+    float sw, irr;
+    bool use, use_irr;
+};
+__device__ __forceinline__ RecordIn record_in(int64_t i, const float* __restrict__ radiance,
+                                              const float* __restrict__ wo_pdf, const float* __restrict__ stat_w,
+                                              const uint8_t* __restrict__ is_delta) {
+    RecordIn r;
+    const bool delta = is_delta && is_delta[i];
+    const float wo = wo_pdf ? wo_pdf[i] : 1.0f;
+    r.sw = stat_w ? stat_w[i] : 1.0f;
+    r.irr = __fdiv_rn(radiance[i], wo);
+    r.use = !delta && isfinite(r.sw) && r.sw > 0.0f;
+    r.use_irr = r.use && isfinite(r.irr) && r.irr > 0.0f;
+    return r;
+}
+template <bool CANON>
+__device__ __forceinline__ float2 record_uv(int64_t i, const float* __restrict__ dir) {
+    if (CANON) return reinterpret_cast<const float2*>(dir)[i];
+    return dir_to_canonical(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
+}
+
+// sum of v over the warp's lanes, exact modulo 2^64 (as the counters themselves add)
+__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 template <bool CANON>
 __global__ void __launch_bounds__(kRecordBlock) k_record(SDTreeDev t, int64_t n, const float* __restrict__ pos,
                                                          const float* __restrict__ dir, const float* __restrict__ radiance,
@@ -76,65 +116,74 @@ __global__ void __launch_bounds__(kRecordBlock) k_record(SDTreeDev t, int64_t n,
                                                          const float* __restrict__ stat_w,
                                                          const uint8_t* __restrict__ is_delta) {
     __shared__ uint32_t s_st[kStageSTreeRecord];
-    __shared__ unsigned long long s_q[kPrivQuads];
-    __shared__ unsigned long long s_w[kPrivTrees];
+    __shared__ unsigned long long s_sum[kPrivSums];
     const uint32_t nst = t.counts[0];
     const uint32_t nq = t.counts[2] * 4u, ndt = t.counts[1];
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    const int64_t first = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (ndt == 1 && t.b_cnt[0] == 1) {
+        // root only: DTree 0, quadrants of its one node
+        unsigned long long w = 0, q[4] = {0, 0, 0, 0};
+        auto add = [&](const RecordIn& r, float2 c) {
+            if (!r.use) return;
+            w += to_fx(r.sw, t.fx, t.status);
+            if (!r.use_irr) return;
+            const int k = quad_child(c.x, c.y);
+            const unsigned long long v = to_fx(__fmul_rn(r.irr, r.sw), t.fx, t.status);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) q[j] += k == j ? v : 0ull;
+        };
+        int64_t i = first;
+        for (; i + 3 * stride < n; i += 4 * stride) {  // four records' loads in flight
+            RecordIn r[4];
+            float2 c[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                r[j] = record_in(i + j * stride, radiance, wo_pdf, stat_w, is_delta);
+                c[j] = record_uv<CANON>(i + j * stride, dir);
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) add(r[j], c[j]);
+        }
+        for (; i < n; i += stride) add(record_in(i, radiance, wo_pdf, stat_w, is_delta), record_uv<CANON>(i, dir));
+        // one add per CTA and counter
+        if (threadIdx.x < 5) s_sum[threadIdx.x] = 0ull;
+        __syncthreads();
+        const unsigned long long sums[5] = {w, q[0], q[1], q[2], q[3]};
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            const unsigned long long v = warp_sum_u64(sums[j]);
+            if ((threadIdx.x & 31) == 0 && v) atomicAdd(s_sum + j, v);
+        }
+        __syncthreads();
+        if (threadIdx.x < 5 && s_sum[threadIdx.x])
+            atomicAdd(threadIdx.x ? t.b_sums + size_t(t.b_off[0]) * 4 + (threadIdx.x - 1) : t.b_statw, s_sum[threadIdx.x]);
+        return;
+    }
     const bool staged = nst <= kStageSTreeRecord;
-    const bool priv = nq <= kPrivQuads && ndt <= kPrivTrees;
+    const bool priv_w = ndt <= kPrivSums;
+    const bool priv = priv_w && nq <= kPrivSums - ndt;
     if (staged)
         for (uint32_t i = threadIdx.x; i < nst; i += blockDim.x) s_st[i] = t.snode[i];
-    if (priv) {
-        for (uint32_t i = threadIdx.x; i < nq; i += blockDim.x) s_q[i] = 0ull;
-        for (uint32_t i = threadIdx.x; i < ndt; i += blockDim.x) s_w[i] = 0ull;
-    }
+    if (priv_w)
+        for (uint32_t i = threadIdx.x; i < ndt + (priv ? nq : 0u); i += blockDim.x) s_sum[i] = 0ull;
     __syncthreads();
     const uint32_t* st = staged ? s_st : t.snode;
-    unsigned long long* acc_w = priv ? s_w : t.b_statw;
-    unsigned long long* acc_q = priv ? s_q : t.b_sums;
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t base = int64_t(blockIdx.x) * blockDim.x; base < n; base += stride) {
-        const int64_t i = base + threadIdx.x;
-        unsigned long long k_w = ~0ull, k_s = ~0ull, v_w = 0, v_s = 0;
-        if (i < n && !(is_delta && is_delta[i])) {
-            const float wo = wo_pdf ? wo_pdf[i] : 1.0f;
-            const float sw = stat_w ? stat_w[i] : 1.0f;
-            const float irr = __fdiv_rn(radiance[i], wo);
-            if (isfinite(sw) && sw > 0.0f) {
-                const uint32_t d = stree_lookup(st, t.mn, t.mx, pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], t.inv_size,
-                                                staged ? nullptr : t.stop);
-                k_w = d;
-                v_w = to_fx(sw, t.fx, t.status);
-                if (isfinite(irr) && irr > 0.0f) {
-                    float u, v;
-                    if (CANON) {
-                        const float2 c = reinterpret_cast<const float2*>(dir)[i];
-                        u = c.x; v = c.y;
-                    } else {
-                        const float2 c = dir_to_canonical(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
-                        u = c.x; v = c.y;
-                    }
-                    k_s = dtree_record_slot(t.b_child, t.b_off[d], u, v);
-                    v_s = to_fx(__fmul_rn(irr, sw), t.fx, t.status);
-                }
-            }
-        }
-        if (priv) {
-            // shared-memory sums: a warp's records spread over many quadrants, so plain
-            // 64-bit shared atomics beat aggregating them first
-            if (k_w != ~0ull) atomicAdd(acc_w + k_w, v_w);
-            if (k_s != ~0ull) atomicAdd(acc_q + k_s, v_s);
-        } else {
-            warp_add_u64(k_w, v_w, acc_w);
-            warp_add_u64(k_s, v_s, acc_q);
-        }
+    for (int64_t i = first; i < n; i += stride) {
+        const RecordIn r = record_in(i, radiance, wo_pdf, stat_w, is_delta);
+        if (!r.use) continue;
+        const uint32_t d = stree_lookup(st, t.mn, t.mx, pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], t.inv_size,
+                                        staged ? nullptr : t.stop);
+        atomicAdd(priv_w ? s_sum + d : t.b_statw + d, to_fx(r.sw, t.fx, t.status));
+        if (!r.use_irr) continue;
+        const float2 c = record_uv<CANON>(i, dir);
+        const uint32_t k = dtree_record_slot(t.b_child, t.b_off[d], c.x, c.y);
+        atomicAdd(priv ? s_sum + ndt + k : t.b_sums + k, to_fx(__fmul_rn(r.irr, r.sw), t.fx, t.status));
     }
-    if (priv) {
+    if (priv_w) {
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < nq; i += blockDim.x)
-            if (s_q[i]) atomicAdd(t.b_sums + i, s_q[i]);
-        for (uint32_t i = threadIdx.x; i < ndt; i += blockDim.x)
-            if (s_w[i]) atomicAdd(t.b_statw + i, s_w[i]);
+        for (uint32_t i = threadIdx.x; i < ndt + (priv ? nq : 0u); i += blockDim.x)
+            if (s_sum[i]) atomicAdd(i < ndt ? t.b_statw + i : t.b_sums + (i - ndt), s_sum[i]);
     }
 }
 
