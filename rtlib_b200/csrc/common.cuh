@@ -94,27 +94,6 @@ __device__ __forceinline__ float fx_to_float(unsigned long long x, FixedPoint fx
     return __fmul_rn(__ll2float_rn((long long)x), fx.inv_scale);
 }
 
-// Warp-aggregated 64-bit atomic add: lanes with equal keys (match.any) reduce their values
-// with three 21-bit redux.sync partial sums (exact for 32 lanes of 63-bit values) and one
-// lane issues the atomic.  All 32 lanes must call this converged; key == ~0 means no-op.
-__device__ __forceinline__ void warp_add_u64(unsigned long long key, unsigned long long val,
-                                             unsigned long long* base) {
-    const unsigned peers = __match_any_sync(0xffffffffu, key);
-    if (key == ~0ull) return;
-    const unsigned lo = unsigned(val & 0x1FFFFFull);
-    const unsigned mid = unsigned((val >> 21) & 0x1FFFFFull);
-    const unsigned hi = unsigned(val >> 42);
-    const unsigned slo = __reduce_add_sync(peers, lo);
-    const unsigned smid = __reduce_add_sync(peers, mid);
-    const unsigned shi = __reduce_add_sync(peers, hi);
-    const int lane = threadIdx.x & 31;
-    if (lane == __ffs(peers) - 1) {
-        unsigned long long total = (unsigned long long)slo + ((unsigned long long)smid << 21) +
-                                   ((unsigned long long)shi << 42);
-        atomicAdd(base + key, total);
-    }
-}
-
 // ------------------------------------------------------------------ block scan
 // Exclusive prefix sum over a block (blockDim.x multiple of 32, <= 1024); returns the
 // exclusive prefix of `v` and writes the block total to *total (all threads).

@@ -25,25 +25,23 @@ namespace rtpg {
 
 constexpr int kMqtBuildBlock = 256;
 
+// One record per thread, one plain 64-bit atomic each: a frame's records spread over the leaves
+// of thousands of cells, where aggregating equal keys within the warp only adds its 64-bit match
+// (2^22 records into 377 k cells of 4^4 leaves: 255 us aggregated, 134 us plain).
 __global__ void __launch_bounds__(256) k_mqt_record(MqtDev t, int64_t n, const uint32_t* __restrict__ cell,
                                                     const float* __restrict__ dir, int canonical,
                                                     const float* __restrict__ value) {
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t base = int64_t(blockIdx.x) * blockDim.x; base < n; base += stride) {
-        const int64_t i = base + threadIdx.x;
-        unsigned long long key = ~0ull, v = 0;
-        if (i < n) {
-            const uint32_t c = cell[i];
-            const float x = value[i];
-            if (c != 0xffffffffu && c < t.ncells && isfinite(x) && x > 0.0f) {
-                float2 uv;
-                if (canonical) uv = reinterpret_cast<const float2*>(dir)[i];
-                else uv = dir_to_canonical_mqt(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
-                key = ((unsigned long long)c << (2 * t.level)) + mqt_leaf_code(t.level, uv.x, uv.y);
-                v = to_fx(x, t.fx, t.status);
-            }
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const uint32_t c = cell[i];
+        const float x = value[i];
+        if (c != 0xffffffffu && c < t.ncells && isfinite(x) && x > 0.0f) {
+            float2 uv;
+            if (canonical) uv = reinterpret_cast<const float2*>(dir)[i];
+            else uv = dir_to_canonical_mqt(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
+            const unsigned long long key = ((unsigned long long)c << (2 * t.level)) + mqt_leaf_code(t.level, uv.x, uv.y);
+            atomicAdd(t.leaves + key, to_fx(x, t.fx, t.status));
         }
-        warp_add_u64(key, v, t.leaves);
     }
 }
 
