@@ -5,14 +5,13 @@
 //
 // Layout in HBM: building leaves, int64 fixed point, cell-major: leaves[cell * 4^L + code]
 // (the reference records only the leaf level too, OPX7UtilsMorton.h:282-283); sampling
-// pyramid, float, per cell (4^(L+1)-1)/3 entries, level l at offset (4^l-1)/3, Morton order
-// inside a level (code = part1by1(y) << 1 | part1by1(x)).
+// pyramid, float, per cell (4^(L+1)-1)/3 entries, level l at offset (4^l-1)/3 (+ mqt_dev.cuh's
+// alignment shift), Morton order inside a level (code = part1by1(y) << 1 | part1by1(x)).
 //
 // Update (RTMortonQuadTreeWrapperT::Update + LaunchBuildKernel, :640-651, :916-941) is one
-// kernel: a warp (levels up to 5) or a CTA (levels 6, 7) per cell reads the cell's leaves,
-// reduces the pyramid in shared memory with exact integer sums, writes it as float to the
-// sampling buffer and zeroes the leaves (RTLib launches 1024x more blocks than cells and loops
-// serially per cell).
+// kernel: the leaves of every cell in use are reduced with exact integer sums, written as a float
+// pyramid to the sampling buffer and zeroed (RTLib launches 1024x more blocks than cells and
+// loops serially per cell).
 #include <algorithm>
 #include <new>
 #include <vector>
@@ -23,173 +22,269 @@
 
 namespace rtpg {
 
-constexpr int kMqtBuildBlock = 256;
+
+// what one record adds: leaf (UINT64_MAX: nothing) and fixed-point value
+__device__ __forceinline__ unsigned long long mqt_record_key(const MqtDev& t, int64_t i, const uint32_t* __restrict__ cell,
+                                                             const float* __restrict__ dir, int canonical,
+                                                             const float* __restrict__ value, unsigned long long& v) {
+    const uint32_t c = cell[i];
+    const float x = value[i];
+    if (c == 0xffffffffu || c >= t.ncells || !isfinite(x) || !(x > 0.0f)) return ~0ull;
+    float2 uv;
+    if (canonical) uv = reinterpret_cast<const float2*>(dir)[i];
+    else uv = dir_to_canonical_mqt(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
+    v = to_fx(x, t.fx, t.status);
+    return ((unsigned long long)c << (2 * t.level)) + mqt_leaf_code(t.level, uv.x, uv.y);
+}
 
 // One record per thread, one plain 64-bit atomic each: a frame's records spread over the leaves
-// of thousands of cells, where aggregating equal keys within the warp only adds its 64-bit match
-// (2^22 records into 377 k cells of 4^4 leaves: 255 us aggregated, 134 us plain).
-__global__ void __launch_bounds__(256) k_mqt_record(MqtDev t, int64_t n, const uint32_t* __restrict__ cell,
-                                                    const float* __restrict__ dir, int canonical,
-                                                    const float* __restrict__ value) {
+// of many cells, where aggregating equal keys within the warp only adds its 64-bit match.
+// The cell is marked as touched by a byte store.  Popular cells would get thousands of those, which
+// queue up in L2 behind one another (and a look at the byte first finds the L1 line of the first
+// look), so each CTA remembers the cells it marked in a direct-mapped table in shared memory; large
+// CTAs share one table among many records.  2^22 records into 377 k / 1474 cells of 4^4 leaves:
+// 258 / 255 us aggregated and without
+// marks, 150 / 97 us now (139 / 75 us without marks).
+constexpr int kRecThreads = 1024;
+constexpr uint32_t kRecTags = 8192;  // 32 KB, two CTAs per SM
+__global__ void __launch_bounds__(kRecThreads) k_mqt_record(MqtDev t, int64_t n, const uint32_t* __restrict__ cell,
+                                                            const float* __restrict__ dir, int canonical,
+                                                            const float* __restrict__ value) {
+    __shared__ uint32_t s_tag[kRecTags];
+    for (uint32_t k = threadIdx.x; k < kRecTags; k += kRecThreads) s_tag[k] = 0xffffffffu;
+    __syncthreads();
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const uint32_t c = cell[i];
-        const float x = value[i];
-        if (c != 0xffffffffu && c < t.ncells && isfinite(x) && x > 0.0f) {
-            float2 uv;
-            if (canonical) uv = reinterpret_cast<const float2*>(dir)[i];
-            else uv = dir_to_canonical_mqt(dir[3 * i], dir[3 * i + 1], dir[3 * i + 2]);
-            const unsigned long long key = ((unsigned long long)c << (2 * t.level)) + mqt_leaf_code(t.level, uv.x, uv.y);
-            atomicAdd(t.leaves + key, to_fx(x, t.fx, t.status));
-        }
+        unsigned long long v;
+        const unsigned long long key = mqt_record_key(t, i, cell, dir, canonical, value, v);
+        if (key == ~0ull) continue;
+        atomicAdd(t.leaves + key, v);
+        const uint32_t c = uint32_t(key >> (2 * t.level));
+        mqt_mark(t, c, s_tag + c % kRecTags);
     }
 }
 
-// One CTA per cell: leaves -> exact pyramid in shared memory -> float sampling pyramid.
-__global__ void __launch_bounds__(kMqtBuildBlock) k_mqt_build(MqtDev t) {
-    extern __shared__ unsigned long long sp[];  // (4^(L+1)-1)/3 entries
-    const uint32_t L = t.level;
-    const uint32_t nleaf = 1u << (2 * L);
-    const uint32_t off_leaf = mqt_level_offset(L);
-    const uint32_t per = mqt_level_offset(L + 1);
-    for (uint32_t c = blockIdx.x; c < t.ncells; c += gridDim.x) {
-        unsigned long long* lf = t.leaves + (size_t)c * nleaf;
-        for (uint32_t k = threadIdx.x; k < nleaf; k += blockDim.x) {
-            sp[off_leaf + k] = lf[k];
-            lf[k] = 0ull;
-        }
-        __syncthreads();
-        for (int l = (int)L - 1; l >= 0; --l) {
-            const uint32_t o = mqt_level_offset(l), oc = mqt_level_offset(l + 1), cnt = 1u << (2 * l);
-            for (uint32_t k = threadIdx.x; k < cnt; k += blockDim.x)
-                sp[o + k] = sp[oc + 4 * k] + sp[oc + 4 * k + 1] + sp[oc + 4 * k + 2] + sp[oc + 4 * k + 3];
-            __syncthreads();
-        }
-        float* w = t.pyramid + (size_t)c * per;
-        for (uint32_t k = threadIdx.x; k < per; k += blockDim.x) w[k] = fx_to_float(sp[k], t.fx);
-        __syncthreads();
+// The same for trees of few leaves in all (`nleaf`), where records queue up on the leaves
+// themselves: every CTA sums all leaves in shared memory and adds the nonzero ones once.  A sum is
+// two 32-bit words, the low word's carry added to the high one (64-bit shared adds are
+// compare-and-swap loops).  2^22 records into 10 cells of 16 leaves: 798 us with one atomic per
+// record, 40 us here.
+constexpr uint32_t kRecPrivLeaves = 16384;  // 128 KB
+__global__ void __launch_bounds__(kRecThreads) k_mqt_record_private(MqtDev t, int64_t n, const uint32_t* __restrict__ cell,
+                                                                    const float* __restrict__ dir, int canonical,
+                                                                    const float* __restrict__ value, uint32_t nleaf) {
+    extern __shared__ uint32_t s_sum[];
+    uint32_t *lo = s_sum, *hi = s_sum + nleaf;
+    for (uint32_t k = threadIdx.x; k < 2 * nleaf; k += kRecThreads) s_sum[k] = 0u;
+    __syncthreads();
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
+        unsigned long long v;
+        const unsigned long long key = mqt_record_key(t, i, cell, dir, canonical, value, v);
+        if (key == ~0ull) continue;
+        const uint32_t low = (uint32_t)v, old = atomicAdd(lo + key, low);
+        const uint32_t up = (uint32_t)(v >> 32) + (old + low < low ? 1u : 0u);
+        if (up) atomicAdd(hi + key, up);
+    }
+    __syncthreads();
+    // each CTA starts at another leaf, so that they do not all add to the same one at once
+    for (uint32_t j = threadIdx.x; j < nleaf; j += kRecThreads) {
+        const uint32_t k = (j + blockIdx.x * 97u) % nleaf;
+        const unsigned long long v = ((unsigned long long)hi[k] << 32) | lo[k];
+        if (!v) continue;
+        atomicAdd(t.leaves + k, v);
+        t.touched[k >> (2 * t.level)] = 1;
     }
 }
 
-// Levels 1 and 2 (up to kMqtWarpLevel): one warp per cell, kMqtWarps cells per CTA.  The warp reads the
-// cell's leaves with 16-byte loads (and zeroes them with 16-byte stores), reduces the pyramid
-// in its own shared memory with exact integer sums and writes it out with consecutive lanes on
-// consecutive floats; no block-wide barrier, so every warp of the SM keeps a cell's loads in
-// flight.  Same results as k_mqt_build (integer sums do not depend on their order).
-constexpr uint32_t kMqtWarpLevel = 2;  // levels 3 to 5 use k_mqt_build_reg
+// ------------------------------------------------------------------ build
+// Bound by HBM: a cell's leaves are read (8 B each), its pyramid written (4 B a node).  The
+// building leaves of a cell are nonzero only if it was recorded into since the last build
+// (`touched`), its pyramid only if the last build wrote sums there (`live`): a cell with neither
+// is skipped, leaves are read only where touched, and a 32-byte sector of leaves is zeroed only if
+// it holds something.  At level 4 with 36 % of 2^20 cells in use and 4 M records: 1206 us when every cell
+// was read, zeroed and rewritten (level 4: 5.7 GB), 277 us now (1.4 GB, 77 % of the copy rate).
+//
+// A lane takes four leaves (one 32-byte load and, as floats, one 16-byte store) and sums them to
+// their parent; four and sixteen lanes' parents come from butterfly shuffles, wider nodes from
+// sums over the lane's further leaves 128 apart.  Lanes are consecutive in memory at every step and
+// no shared memory is used.  Sums are exact integers, in any order the same.
 constexpr int kMqtWarps = 8;
-__global__ void __launch_bounds__(32 * kMqtWarps) k_mqt_build_warp(MqtDev t) {
-    extern __shared__ unsigned long long swarp[];  // kMqtWarps x (4^(L+1)-1)/3 entries
-    const uint32_t L = t.level;
-    const uint32_t nleaf = 1u << (2 * L);  // >= 4: 16-byte aligned rows of leaves
-    const uint32_t off_leaf = mqt_level_offset(L);
-    const uint32_t per = mqt_level_offset(L + 1);
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    unsigned long long* sp = swarp + (size_t)warp * per;
-    const uint32_t nw = gridDim.x * kMqtWarps;
-    for (uint32_t c = blockIdx.x * kMqtWarps + warp; c < t.ncells; c += nw) {
-        ulonglong2* lf = reinterpret_cast<ulonglong2*>(t.leaves + (size_t)c * nleaf);
-        for (uint32_t k = lane; k < nleaf / 2; k += 32) {
-            const ulonglong2 v = lf[k];
-            lf[k] = make_ulonglong2(0ull, 0ull);
-            sp[off_leaf + 2 * k] = v.x;
-            sp[off_leaf + 2 * k + 1] = v.y;
-        }
-        __syncwarp();
-        for (int l = (int)L - 1; l >= 0; --l) {
-            const uint32_t o = mqt_level_offset(l), oc = mqt_level_offset(l + 1), cnt = 1u << (2 * l);
-            for (uint32_t k = lane; k < cnt; k += 32)
-                sp[o + k] = sp[oc + 4 * k] + sp[oc + 4 * k + 1] + sp[oc + 4 * k + 2] + sp[oc + 4 * k + 3];
-            __syncwarp();
-        }
-        float* w = t.pyramid + (size_t)c * per;
-        for (uint32_t k = lane; k < per; k += 32) w[k] = fx_to_float(sp[k], t.fx);
-        __syncwarp();
-    }
+
+__device__ __forceinline__ void ld_leaves(const unsigned long long* p, unsigned long long* v) {
+    asm volatile("ld.global.v4.u64 {%0,%1,%2,%3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void zero_leaves(unsigned long long* p) {
+    asm volatile("st.global.v4.u64 [%0], {%1,%1,%1,%1};" ::"l"(p), "l"(0ull) : "memory");
+}
+__device__ __forceinline__ unsigned long long xor_add(unsigned long long s, int o) {
+    return s + __shfl_xor_sync(0xffffffffu, s, o);
 }
 
-// Levels 3 to 5: the reduction in registers.  Lane l owns leaves [l P, (l + 1) P) with
-// P = 4^L / 32 (2, 8 or 32), loaded and zeroed as 16-byte vectors; the levels whose nodes span
-// at most P leaves are summed inside the lane, the three levels above them span 2, 8 and 32
-// lanes and come from butterfly shuffles.  The float pyramid is assembled in a per-warp
-// shared buffer and stored with consecutive lanes on consecutive floats.
+// The subtree of S levels (4 or 5) whose root is node `sub` of level `top` of a cell: its leaves
+// (lf: its first one) are summed and zeroed, its nodes written to the cell's pyramid w; returns
+// the subtree's sum.  The whole warp calls it.  read = false: the leaves are zero.
+template <int S>
+__device__ __forceinline__ unsigned long long mqt_build_subtree(unsigned long long* lf, float* w, uint32_t top,
+                                                                uint32_t sub, bool read, FixedPoint fx) {
+    static_assert(S == 4 || S == 5, "a warp's share is 256 or 1024 leaves");
+    constexpr int NC = (1 << (2 * (S - 1))) / 32;  // four-leaf groups per lane
+    const uint32_t lane = threadIdx.x & 31u;
+    unsigned long long v[NC][4];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        if (read) ld_leaves(lf + 4 * (c * 32 + lane), v[c]);
+        else v[c][0] = v[c][1] = v[c][2] = v[c][3] = 0ull;
+    }
+    unsigned long long run = 0, all = 0;
+    float* const w0 = w + mqt_base(top + S) + (size_t(sub) << (2 * S));
+    float* const w1 = w + mqt_base(top + S - 1) + (size_t(sub) << (2 * (S - 1)));
+    float* const w2 = w + mqt_base(top + S - 2) + (size_t(sub) << (2 * (S - 2)));
+    float* const w3 = w + mqt_base(top + S - 3) + (size_t(sub) << (2 * (S - 3)));
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        const uint32_t g = c * 32 + lane;
+        if (v[c][0] | v[c][1] | v[c][2] | v[c][3]) zero_leaves(lf + 4 * g);
+        *reinterpret_cast<float4*>(w0 + 4 * g) = make_float4(fx_to_float(v[c][0], fx), fx_to_float(v[c][1], fx),
+                                                             fx_to_float(v[c][2], fx), fx_to_float(v[c][3], fx));
+        unsigned long long s = v[c][0] + v[c][1] + v[c][2] + v[c][3];
+        w1[g] = fx_to_float(s, fx);
+        s = xor_add(xor_add(s, 1), 2);
+        if ((lane & 3u) == 0) w2[g >> 2] = fx_to_float(s, fx);
+        s = xor_add(xor_add(s, 4), 8);
+        if ((lane & 15u) == 0) w3[g >> 4] = fx_to_float(s, fx);
+        run += xor_add(s, 16);
+        if (S == 5 && (c & 1)) {  // the level between: two groups of 32
+            if (lane == 0) w[mqt_base(top + 1) + (size_t(sub) << 2) + (c >> 1)] = fx_to_float(run, fx);
+        }
+        if (S == 4 || (c & 1)) {
+            all += run;
+            run = 0;
+        }
+    }
+    if (lane == 0) w[mqt_base(top) + sub] = fx_to_float(all, fx);
+    return all;
+}
+
+// Levels 1 to 3: 32, 8 or 2 cells per warp, a lane per four leaves.
 template <int L>
-__global__ void __launch_bounds__(32 * kMqtWarps) k_mqt_build_reg(MqtDev t) {
-    constexpr int NLEAF = 1 << (2 * L), P = NLEAF / 32, PER = ((1 << (2 * (L + 1))) - 1) / 3;
-    static_assert(L >= 3 && L <= 5, "levels 3..5");
-    __shared__ float sbuf[kMqtWarps][PER];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    float* fb = sbuf[warp];
-    const uint32_t nw = gridDim.x * kMqtWarps;
-    for (uint32_t c = blockIdx.x * kMqtWarps + warp; c < t.ncells; c += nw) {
-        ulonglong2* lf = reinterpret_cast<ulonglong2*>(t.leaves + (size_t)c * NLEAF) + lane * (P / 2);
-        unsigned long long v[P];
-#pragma unroll
-        for (int j = 0; j < P / 2; ++j) {
-            const ulonglong2 x = lf[j];
-            v[2 * j] = x.x;
-            v[2 * j + 1] = x.y;
+__global__ void __launch_bounds__(32 * kMqtWarps) k_mqt_build_small(MqtDev t) {
+    static_assert(L >= 1 && L <= 3, "levels 1..3");
+    constexpr uint32_t G = 1u << (2 * (L - 1));  // lanes of a cell
+    constexpr uint32_t NLEAF = 4 * G;
+    const uint32_t lane = threadIdx.x & 31u, g = lane % G;
+    const uint32_t nw = gridDim.x * kMqtWarps, per = 32 / G;
+    for (uint32_t base = (blockIdx.x * kMqtWarps + (threadIdx.x >> 5)) * per; base < t.ncells; base += nw * per) {
+        const uint32_t c = base + lane / G;
+        const bool touched = c < t.ncells && t.touched[c], live = c < t.ncells && t.live[c];
+        if (!__any_sync(0xffffffffu, touched || live)) continue;
+        unsigned long long v[4] = {0ull, 0ull, 0ull, 0ull};
+        unsigned long long* lf = t.leaves + size_t(c) * NLEAF + 4 * g;
+        if (touched) ld_leaves(lf, v);
+        if (v[0] | v[1] | v[2] | v[3]) zero_leaves(lf);
+        const bool out = touched || live;
+        float* w = t.pyramid + size_t(c) * mqt_stride(L);
+        if (out)
+            *reinterpret_cast<float4*>(w + mqt_base(L) + 4 * g) =
+                make_float4(fx_to_float(v[0], t.fx), fx_to_float(v[1], t.fx), fx_to_float(v[2], t.fx), fx_to_float(v[3], t.fx));
+        unsigned long long s = v[0] + v[1] + v[2] + v[3];
+        if (out) w[mqt_base(L - 1) + g] = fx_to_float(s, t.fx);
+        if (L >= 2) {
+            s = xor_add(xor_add(s, 1), 2);
+            if (out && (lane & 3u) == 0) w[mqt_base(L >= 2 ? L - 2 : 0) + (g >> 2)] = fx_to_float(s, t.fx);
         }
-#pragma unroll
-        for (int j = 0; j < P / 2; ++j) lf[j] = make_ulonglong2(0ull, 0ull);
-        // the leaf level, then the lane-local levels (each a quarter of the one below)
-#pragma unroll
-        for (int j = 0; j < P; ++j) fb[mqt_level_offset(L) + lane * P + j] = fx_to_float(v[j], t.fx);
-        int lvl = L - 1;
-        int n = P;  // values of the current level held by this lane
-#pragma unroll
-        for (int step = 0; step < 3 && n >= 4; ++step) {
-#pragma unroll
-            for (int j = 0; j < n / 4; ++j) v[j] = v[4 * j] + v[4 * j + 1] + v[4 * j + 2] + v[4 * j + 3];
-            n /= 4;
-#pragma unroll
-            for (int j = 0; j < n; ++j) fb[mqt_level_offset(lvl) + lane * n + j] = fx_to_float(v[j], t.fx);
-            --lvl;
+        if (L >= 3) {
+            s = xor_add(xor_add(s, 4), 8);
+            if (out && (lane & 15u) == 0) w[mqt_base(0)] = fx_to_float(s, t.fx);
         }
-        // two values are left in every lane: their sum is the lane's run
-        unsigned long long s = 0;
-#pragma unroll
-        for (int j = 0; j < n; ++j) s += v[j];
-        // nodes spanning 2, 8 and 32 lanes
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        if ((lane & 1u) == 0) fb[mqt_level_offset(lvl) + (lane >> 1)] = fx_to_float(s, t.fx);
-        --lvl;
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        s += __shfl_xor_sync(0xffffffffu, s, 4);
-        if ((lane & 7u) == 0) fb[mqt_level_offset(lvl) + (lane >> 3)] = fx_to_float(s, t.fx);
-        --lvl;
-        s += __shfl_xor_sync(0xffffffffu, s, 8);
-        s += __shfl_xor_sync(0xffffffffu, s, 16);
-        if (lane == 0) fb[0] = fx_to_float(s, t.fx);
         __syncwarp();
-        float* w = t.pyramid + (size_t)c * PER;
-        for (uint32_t k = lane; k < (uint32_t)PER; k += 32) w[k] = fb[k];
-        __syncwarp();
+        if (out && g == 0) {
+            t.touched[c] = 0;
+            t.live[c] = touched ? 1 : 0;
+        }
     }
 }
 
-__global__ void __launch_bounds__(256) k_mqt_sample(MqtDev t, int64_t n, const uint32_t* __restrict__ cell,
-                                                    const uint32_t* __restrict__ seeds, uint32_t seed_base,
-                                                    float* __restrict__ out_uv, float* __restrict__ out_pdf,
-                                                    float* __restrict__ out_dir, float* __restrict__ out_pdf_tree) {
-    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const uint32_t c = cell[i];
-        uint32_t rng = seeds ? seeds[i] : (pcg1d(seed_base + (uint32_t)i) | 1u);
-        float pdf;
-        const float2 uv = mqt_sample_and_pdf(t, c, rng, pdf);
-        if (out_uv) reinterpret_cast<float2*>(out_uv)[i] = uv;
-        if (out_pdf_tree) out_pdf_tree[i] = pdf;
-        // MortonQuadTreeWrapperT::SampleAndPdf (OPX7UtilsMorton.h:486-500):
-        // pdf *= (0.25f * RTLIB_M_INV_PI), evaluated in double as written
-        if (out_pdf) out_pdf[i] = (float)((double)pdf * (0.25 * kInvPiD));
-        if (out_dir) {
-            const float3 d = canonical_to_dir_mqt(uv.x, uv.y);
-            out_dir[3 * i] = d.x;
-            out_dir[3 * i + 1] = d.y;
-            out_dir[3 * i + 2] = d.z;
+// Levels 4 and 5: a warp per cell.  A warp looks at eight cells' flags at a time.
+template <int L>
+__global__ void __launch_bounds__(32 * kMqtWarps) k_mqt_build_warp(MqtDev t) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t nw = gridDim.x * kMqtWarps;
+    for (uint32_t base = (blockIdx.x * kMqtWarps + (threadIdx.x >> 5)) * 8; base < t.ncells; base += nw * 8) {
+        const uint32_t c0 = base + lane;
+        const bool mine = lane < 8 && c0 < t.ncells;
+        const bool touched = mine && t.touched[c0], live = mine && t.live[c0];
+        const unsigned read = __ballot_sync(0xffffffffu, touched);
+        for (unsigned todo = __ballot_sync(0xffffffffu, touched || live); todo; todo &= todo - 1) {
+            const uint32_t k = __ffs(todo) - 1;
+            mqt_build_subtree<L>(t.leaves + (size_t(base + k) << (2 * L)), t.pyramid + size_t(base + k) * mqt_stride(L), 0, 0,
+                                 (read >> k) & 1u, t.fx);
+        }
+        if (touched || live) {
+            t.touched[c0] = 0;
+            t.live[c0] = touched ? 1 : 0;
         }
     }
+}
+
+// Levels 6 and 7: a CTA of 4 or 16 warps per cell, each warp a subtree of five levels; the one or
+// two levels above come from the warps' sums in shared memory.
+template <int L>
+__global__ void __launch_bounds__(L == 6 ? 128 : 512) k_mqt_build_block(MqtDev t) {
+    static_assert(L == 6 || L == 7, "levels 6, 7");
+    constexpr uint32_t W = L == 6 ? 4 : 16, TOP = L - 5;
+    __shared__ unsigned long long s_sum[W];
+    const uint32_t warp = threadIdx.x >> 5;
+    for (uint32_t c = blockIdx.x; c < t.ncells; c += gridDim.x) {
+        const bool touched = t.touched[c], live = t.live[c];
+        if (!touched && !live) continue;
+        float* w = t.pyramid + size_t(c) * mqt_stride(L);
+        const unsigned long long s = mqt_build_subtree<5>(t.leaves + (size_t(c) << (2 * L)) + size_t(warp) * 1024, w, TOP, warp,
+                                                          touched, t.fx);
+        if ((threadIdx.x & 31u) == 0) s_sum[warp] = s;
+        __syncthreads();
+        if (L == 7 && threadIdx.x < 4) {
+            const unsigned long long* p = s_sum + 4 * threadIdx.x;
+            w[mqt_base(1) + threadIdx.x] = fx_to_float(p[0] + p[1] + p[2] + p[3], t.fx);
+        }
+        if (threadIdx.x == 0) {
+            unsigned long long r = 0;
+            for (uint32_t k = 0; k < W; ++k) r += s_sum[k];
+            w[mqt_base(0)] = fx_to_float(r, t.fx);
+            t.touched[c] = 0;
+            t.live[c] = touched ? 1 : 0;
+        }
+        __syncthreads();
+    }
+}
+
+// ------------------------------------------------------------------ sample / pdf
+struct MqtSampleOut {
+    float *uv, *pdf, *dir, *pdf_tree;
+};
+__device__ __forceinline__ void mqt_sample_one(const MqtDev& t, int64_t i, const uint32_t* __restrict__ cell,
+                                               const uint32_t* __restrict__ seeds, uint32_t seed_base, const MqtSampleOut& o) {
+    const uint32_t c = cell[i];
+    uint32_t rng = seeds ? seeds[i] : (pcg1d(seed_base + (uint32_t)i) | 1u);
+    float pdf;
+    const float2 uv = mqt_sample_and_pdf(t, c, rng, pdf);
+    if (o.uv) reinterpret_cast<float2*>(o.uv)[i] = uv;
+    if (o.pdf_tree) o.pdf_tree[i] = pdf;
+    // MortonQuadTreeWrapperT::SampleAndPdf (OPX7UtilsMorton.h:486-500):
+    // pdf *= (0.25f * RTLIB_M_INV_PI), evaluated in double as written
+    if (o.pdf) o.pdf[i] = (float)((double)pdf * (0.25 * kInvPiD));
+    if (o.dir) {
+        const float3 d = canonical_to_dir_mqt(uv.x, uv.y);
+        o.dir[3 * i] = d.x;
+        o.dir[3 * i + 1] = d.y;
+        o.dir[3 * i + 2] = d.z;
+    }
+}
+__global__ void __launch_bounds__(256) k_mqt_sample(MqtDev t, int64_t n, const uint32_t* __restrict__ cell,
+                                                    const uint32_t* __restrict__ seeds, uint32_t seed_base, MqtSampleOut o) {
+    const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
+        mqt_sample_one(t, i, cell, seeds, seed_base, o);
 }
 
 __global__ void __launch_bounds__(256) k_mqt_pdf(MqtDev t, int64_t n, const uint32_t* __restrict__ cell,
@@ -232,9 +327,6 @@ struct rtpg_mqt {
     }
 };
 
-static int mqt_smem(uint32_t level) { return int(mqt_level_offset(level + 1) * sizeof(unsigned long long)); }
-static int mqt_smem_warp(uint32_t level) { return kMqtWarps * mqt_smem(level); }
-
 extern "C" {
 
 // RTMortonQuadTreeWrapperT(ctx, maxHashSize, maxTreeLevel, fraction) + Allocate (MO.h:597-638)
@@ -251,20 +343,21 @@ int rtpg_mqt_create(uint32_t num_cells, uint32_t level, float fraction, int32_t 
     t.fraction = fraction;
     t.fx.scale = ldexpf(1.0f, fixed_point_bits);
     t.fx.inv_scale = ldexpf(1.0f, -fixed_point_bits);
-    const size_t nleaf = (size_t)num_cells << (2 * level), npyr = (size_t)num_cells * mqt_level_offset(level + 1);
+    const size_t nleaf = (size_t)num_cells << (2 * level), npyr = (size_t)num_cells * mqt_stride(level);
     int r;
-    if ((r = h->alloc(&t.leaves, nleaf)) || (r = h->alloc(&t.pyramid, npyr)) || (r = h->alloc(&t.status, 1))) {
+    if ((r = h->alloc(&t.leaves, nleaf)) || (r = h->alloc(&t.pyramid, npyr)) || (r = h->alloc(&t.status, 1)) ||
+        (r = h->alloc(&t.touched, num_cells)) || (r = h->alloc(&t.live, num_cells))) {
         delete h;
         return r;
     }
     if (cudaMemset(t.leaves, 0, nleaf * 8) != cudaSuccess || cudaMemset(t.pyramid, 0, npyr * 4) != cudaSuccess ||
-        cudaMemset(t.status, 0, 4) != cudaSuccess) {
+        cudaMemset(t.status, 0, 4) != cudaSuccess || cudaMemset(t.touched, 0, num_cells) != cudaSuccess ||
+        cudaMemset(t.live, 0, num_cells) != cudaSuccess) {
         delete h;
         return fail(RTPG_ECUDA, "rtpg_mqt_create: memset failed");
     }
-    cudaError_t e = cudaFuncSetAttribute(k_mqt_build, cudaFuncAttributeMaxDynamicSharedMemorySize, mqt_smem(kMqtMaxLevel));
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mqt_build_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, mqt_smem_warp(kMqtWarpLevel));
+    const cudaError_t e = cudaFuncSetAttribute(k_mqt_record_private, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               int(kRecPrivLeaves * 8));
     if (e != cudaSuccess) {
         delete h;
         return fail(RTPG_ECUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -285,7 +378,9 @@ int rtpg_mqt_clear(rtpg_mqt* h, void* stream) {
     cudaStream_t st = as_stream(stream);
     const MqtDev& t = h->dev;
     RTPG_CUDA(cudaMemsetAsync(t.leaves, 0, ((size_t)t.ncells << (2 * t.level)) * 8, st));
-    RTPG_CUDA(cudaMemsetAsync(t.pyramid, 0, (size_t)t.ncells * mqt_level_offset(t.level + 1) * 4, st));
+    RTPG_CUDA(cudaMemsetAsync(t.pyramid, 0, (size_t)t.ncells * mqt_stride(t.level) * 4, st));
+    RTPG_CUDA(cudaMemsetAsync(t.touched, 0, t.ncells, st));
+    RTPG_CUDA(cudaMemsetAsync(t.live, 0, t.ncells, st));
     RTPG_CUDA(cudaMemsetAsync(t.status, 0, 4, st));
     return RTPG_OK;
 }
@@ -297,7 +392,16 @@ int rtpg_mqt_record(rtpg_mqt* h, int64_t n, const uint32_t* cell, const float* d
     if (n < 0 || (n > 0 && (!cell || !dir || !value))) return fail(RTPG_EINVAL, "rtpg_mqt_record: bad arguments");
     if (dir_is_canonical && !aligned8(dir)) return fail(RTPG_EINVAL, "rtpg_mqt_record: misaligned float2 array");
     if (n == 0) return RTPG_OK;
-    k_mqt_record<<<grid_for(n, 256, 8), 256, 0, as_stream(stream)>>>(h->dev, n, cell, dir, dir_is_canonical, value);
+    const MqtDev& t = h->dev;
+    cudaStream_t st = as_stream(stream);
+    // private sums on so many CTAs that flushing them takes at most half as many adds as there
+    // are records; below sixteen records per leaf there is little to gather
+    const uint64_t nleaf = (uint64_t)t.ncells << (2 * t.level);
+    if (nleaf <= kRecPrivLeaves && (int64_t)(16 * nleaf) <= n)
+        k_mqt_record_private<<<(int)std::min<int64_t>(kSMs, n / (int64_t)(2 * nleaf)), kRecThreads, nleaf * 8, st>>>(
+            t, n, cell, dir, dir_is_canonical, value, (uint32_t)nleaf);
+    else
+        k_mqt_record<<<grid_for(n, kRecThreads, 2), kRecThreads, 0, st>>>(t, n, cell, dir, dir_is_canonical, value);
     RTPG_LAUNCH_CHECK();
     return RTPG_OK;
 }
@@ -305,18 +409,22 @@ int rtpg_mqt_record(rtpg_mqt* h, int64_t n, const uint32_t* cell, const float* d
 // Update + mortonBuildKernel: building leaves -> sampling pyramid, building cleared.
 int rtpg_mqt_update(rtpg_mqt* h, void* stream) {
     if (!h) return fail(RTPG_EINVAL, "rtpg_mqt_update: null handle");
-    const int gw = (int)std::min<uint32_t>((h->dev.ncells + kMqtWarps - 1) / kMqtWarps, kSMs * 8);
-    if (h->dev.level == 3) {
-        k_mqt_build_reg<3><<<gw, 32 * kMqtWarps, 0, as_stream(stream)>>>(h->dev);
-    } else if (h->dev.level == 4) {
-        k_mqt_build_reg<4><<<gw, 32 * kMqtWarps, 0, as_stream(stream)>>>(h->dev);
-    } else if (h->dev.level == 5) {
-        k_mqt_build_reg<5><<<gw, 32 * kMqtWarps, 0, as_stream(stream)>>>(h->dev);
-    } else if (h->dev.level <= kMqtWarpLevel) {
-        k_mqt_build_warp<<<gw, 32 * kMqtWarps, mqt_smem_warp(h->dev.level), as_stream(stream)>>>(h->dev);
-    } else {
-        const int g = (int)std::min<uint32_t>(h->dev.ncells, kSMs * 8);
-        k_mqt_build<<<g, kMqtBuildBlock, mqt_smem(h->dev.level), as_stream(stream)>>>(h->dev);
+    const MqtDev& t = h->dev;
+    cudaStream_t st = as_stream(stream);
+    // warps of `cells` cells each, at most one resident wave of 8 CTAs per SM
+    auto grid = [&](uint32_t cells) {
+        const uint32_t per = cells * kMqtWarps;
+        return (int)std::min<uint32_t>(t.ncells / per + (t.ncells % per != 0), kSMs * 8);
+    };
+    const int block = 32 * kMqtWarps, gb = (int)std::min<uint32_t>(t.ncells, kSMs * 8);
+    switch (t.level) {
+        case 1: k_mqt_build_small<1><<<grid(32), block, 0, st>>>(t); break;
+        case 2: k_mqt_build_small<2><<<grid(8), block, 0, st>>>(t); break;
+        case 3: k_mqt_build_small<3><<<grid(2), block, 0, st>>>(t); break;
+        case 4: k_mqt_build_warp<4><<<grid(8), block, 0, st>>>(t); break;
+        case 5: k_mqt_build_warp<5><<<grid(8), block, 0, st>>>(t); break;
+        case 6: k_mqt_build_block<6><<<gb, 128, 0, st>>>(t); break;
+        default: k_mqt_build_block<7><<<gb, 512, 0, st>>>(t); break;
     }
     RTPG_LAUNCH_CHECK();
     return RTPG_OK;
@@ -330,8 +438,8 @@ int rtpg_mqt_sample_pdf(rtpg_mqt* h, int64_t n, const uint32_t* cell, const uint
     if (n < 0 || (n > 0 && !cell)) return fail(RTPG_EINVAL, "rtpg_mqt_sample_pdf: bad arguments");
     if (!aligned8(out_uv)) return fail(RTPG_EINVAL, "rtpg_mqt_sample_pdf: misaligned float2 array");
     if (n == 0) return RTPG_OK;
-    k_mqt_sample<<<grid_for(n, 256, 8), 256, 0, as_stream(stream)>>>(h->dev, n, cell, seeds, seed_base, out_uv, out_pdf,
-                                                                     out_dir, out_pdf_tree);
+    const MqtSampleOut o{out_uv, out_pdf, out_dir, out_pdf_tree};
+    k_mqt_sample<<<grid_for(n, 256, 8), 256, 0, as_stream(stream)>>>(h->dev, n, cell, seeds, seed_base, o);
     RTPG_LAUNCH_CHECK();
     return RTPG_OK;
 }
@@ -354,9 +462,11 @@ int rtpg_mqt_export(rtpg_mqt* h, int64_t* host_leaves, float* host_pyramid, void
     const MqtDev& t = h->dev;
     if (host_leaves)
         RTPG_CUDA(cudaMemcpyAsync(host_leaves, t.leaves, ((size_t)t.ncells << (2 * t.level)) * 8, cudaMemcpyDeviceToHost, st));
-    if (host_pyramid)
-        RTPG_CUDA(cudaMemcpyAsync(host_pyramid, t.pyramid, (size_t)t.ncells * mqt_level_offset(t.level + 1) * 4,
-                                  cudaMemcpyDeviceToHost, st));
+    if (host_pyramid) {
+        const size_t row = (size_t)mqt_level_offset(t.level + 1) * 4;
+        RTPG_CUDA(cudaMemcpy2DAsync(host_pyramid, row, t.pyramid + kMqtShift, (size_t)mqt_stride(t.level) * 4, row, t.ncells,
+                                    cudaMemcpyDeviceToHost, st));
+    }
     RTPG_CUDA(cudaStreamSynchronize(st));
     return RTPG_OK;
 }

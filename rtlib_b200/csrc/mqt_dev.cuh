@@ -5,9 +5,8 @@
 
 namespace rtpg {
 
-// Deepest supported level: a cell's pyramid of (4^(L+1)-1)/3 int64 sums must fit in shared
-// memory during the build (level 7: 175 KB).  RTLib's configured maximum is 6
-// (OPX7/CMakeLists.txt:103).
+// Deepest supported level (the build gives a cell of level 7 sixteen warps).  RTLib's configured
+// maximum is 6 (OPX7/CMakeLists.txt:103).
 constexpr uint32_t kMqtMaxLevel = 7;
 constexpr double kInvPiD = 0.318309886183790691216444201927515678107738494873046875;
 
@@ -16,11 +15,20 @@ struct MqtDev {
     float fraction;
     FixedPoint fx;
     unsigned long long* leaves;  // ncells * 4^L, building
-    float* pyramid;              // ncells * (4^(L+1)-1)/3, sampling
+    float* pyramid;              // ncells * mqt_stride(level), sampling
+    // per cell: recorded into since the last build (its leaves may be nonzero); its pyramid may
+    // be nonzero.  The build reads and writes only the cells that need it.
+    uint8_t *touched, *live;
     unsigned* status;
 };
 
 __host__ __device__ __forceinline__ uint32_t mqt_level_offset(uint32_t l) { return ((1u << (2 * l)) - 1u) / 3u; }
+// Device layout of a cell's pyramid: the levels one after the other, shifted by three floats, so
+// that the four children of a node are one aligned 16-byte vector ((4^l - 1) / 3 = 1 mod 4) and
+// a cell starts on a 32-byte sector; root and first children share the first sector.
+constexpr uint32_t kMqtShift = 3;
+__host__ __device__ __forceinline__ uint32_t mqt_base(uint32_t l) { return mqt_level_offset(l) + kMqtShift; }
+__host__ __device__ __forceinline__ uint32_t mqt_stride(uint32_t level) { return mqt_level_offset(level + 1) + kMqtShift; }
 
 // MortonUtils::Part1By1_16 / Comp1By1_16 (OPX7UtilsMorton.h:41-89)
 __device__ __forceinline__ uint32_t part1by1(uint32_t x) {
@@ -54,56 +62,85 @@ __device__ __forceinline__ uint32_t mqt_leaf_code(uint32_t level, float u, float
 __device__ __forceinline__ float2 dir_to_canonical_mqt(float x, float y, float z) { return dir_to_canonical(x, y, z); }
 __device__ __forceinline__ float3 canonical_to_dir_mqt(float u, float v) { return canonical_to_dir(u, v); }
 
-// MortonQuadTreeT::SampleAndPdf (:286-344), float order as written
+// One level of MortonQuadTreeT::SampleAndPdf (:286-344), float order as written: the quadrant a
+// draw selects among the sums q of a node with sum `total`.
+__device__ __forceinline__ uint32_t mqt_choose_exact(float4 q, float total, float draw) {
+    const float partial_l = __fadd_rn(q.x, q.z);
+    const float boundary = __fdiv_rn(partial_l, total);
+    const bool right = !(draw < boundary);
+    const float partial = right ? __fadd_rn(q.y, q.w) : partial_l;
+    const float sample = __fdiv_rn(right ? __fsub_rn(draw, boundary) : draw,
+                                   right ? __fsub_rn(1.0f, boundary) : boundary);
+    return (right ? 1u : 0u) | (sample >= __fdiv_rn(right ? q.y : q.x, partial) ? 2u : 0u);
+}
+// The same choice without its three divisions wherever they cannot matter: the boundary is
+// approximated (2 ulp of at most 1: 2.4e-7) and the second comparison num / den >= c / partial is
+// taken as num * partial >= c * den.  num and den are then off by at most 4e-7 each, c <= partial
+// up to rounding, and the rounded quotients by 2^-24 relative each, so the products differ by at
+// most 1.1e-6 * partial from what decides.  Closer calls (about two draws in a million), and every
+// comparison that a zero or non-finite sum makes unordered, take the divisions.
+__device__ __forceinline__ uint32_t mqt_choose(float4 q, float total, float draw) {
+    const float partial_l = __fadd_rn(q.x, q.z);
+    const float b = __fdividef(partial_l, total);
+    const float off = __fsub_rn(draw, b);
+    const bool right = off >= 0.0f;
+    const float partial = right ? __fadd_rn(q.y, q.w) : partial_l;
+    const float num = right ? off : draw, den = right ? __fsub_rn(1.0f, b) : b;
+    const float d = __fsub_rn(__fmul_rn(num, partial), __fmul_rn(right ? q.y : q.x, den));
+    if (fabsf(off) > 1e-6f && fabsf(d) > __fmul_rn(2e-6f, partial)) return (right ? 1u : 0u) | (d >= 0.0f ? 2u : 0u);
+    return mqt_choose_exact(q, total, draw);
+}
+
+// MortonQuadTreeT::SampleAndPdf (:286-344)
 // A cell outside [0, ncells) (UINT32_MAX marks a hash-grid miss) samples like an empty
 // tree: uniform with pdf 1 (RTLib reads out of bounds there).
 __device__ __forceinline__ float2 mqt_sample_and_pdf(const MqtDev& t, uint32_t cell, uint32_t& rng, float& pdf) {
-    const float* w = t.pyramid + (size_t)(cell < t.ncells ? cell : 0u) * mqt_level_offset(t.level + 1);
-    float total = cell < t.ncells ? w[0] : 0.0f;
-    if (total <= 0.0f) {
+    const float* w = t.pyramid + (size_t)(cell < t.ncells ? cell : 0u) * mqt_stride(t.level);
+    const float root = cell < t.ncells ? w[mqt_base(0)] : 0.0f;
+    if (root <= 0.0f) {
         const float a = rnd1(rng);
         const float b = rnd1(rng);
         pdf = 1.0f;
         return make_float2(a, b);
     }
-    uint32_t size = 4, offset = 1, code = 0;
+    float total = root;
+    uint32_t size = 4, offset = mqt_base(1), code = 0;
     for (uint32_t l = 0; l < t.level; ++l) {
-        // level offsets (4^l-1)/3 are odd, so the four children are read one by one
-        const float* qp = w + offset + (code << 2);
-        const float4 q = make_float4(qp[0], qp[1], qp[2], qp[3]);
-        // both sides of the first choice as selects of their operands (the same divisions of
-        // the same values, without the two divergent branches)
-        const float partial_l = __fadd_rn(q.x, q.z);
-        const float boundary = __fdiv_rn(partial_l, total);
-        const float draw = rnd1(rng);
-        const bool right = !(draw < boundary);
-        const float partial = right ? __fadd_rn(q.y, q.w) : partial_l;
-        const float sample = __fdiv_rn(right ? __fsub_rn(draw, boundary) : draw,
-                                       right ? __fsub_rn(1.0f, boundary) : boundary);
-        const uint32_t cl = (right ? 1u : 0u) | (sample >= __fdiv_rn(right ? q.y : q.x, partial) ? 2u : 0u);
+        const float4 q = *reinterpret_cast<const float4*>(w + offset + (code << 2));
+        const uint32_t cl = mqt_choose(q, total, rnd1(rng));
         total = cl == 0 ? q.x : (cl == 1 ? q.y : (cl == 2 ? q.z : q.w));
         code = (code << 2) + cl;
         offset += size;
         size *= 4;
     }
-    const float nn = (float)(1u << t.level);
+    // division by 2^L as the exact product with its reciprocal
+    const float inv = __uint_as_float((127u - t.level) << 23);
     const uint32_t xi = compact1by1(code), yi = compact1by1(code >> 1);
     const float rx = rnd1(rng);
-    const float px = __fdiv_rn(__fadd_rn((float)xi, rx), nn);
+    const float px = __fmul_rn(__fadd_rn((float)xi, rx), inv);
     const float ry = rnd1(rng);
-    const float py = __fdiv_rn(__fadd_rn((float)yi, ry), nn);
-    pdf = __fmul_rn(__fdiv_rn(total, w[0]), (float)(1u << (2 * t.level)));
+    const float py = __fmul_rn(__fadd_rn((float)yi, ry), inv);
+    pdf = __fmul_rn(__fdiv_rn(total, root), (float)(1u << (2 * t.level)));
     return make_float2(px, py);
+}
+
+// Marks cell c as touched unless `tag`, its entry of a direct-mapped table of cells the CTA has
+// marked (shared memory, UINT32_MAX: none), says that was done.  Any lane's entry will do.
+__device__ __forceinline__ void mqt_mark(const MqtDev& t, uint32_t c, volatile uint32_t* tag) {
+    if (*tag == c) return;
+    *tag = c;
+    t.touched[c] = 1;
 }
 
 // MortonQuadTreeT::Pdf (:401-414)
 __device__ __forceinline__ float mqt_pdf(const MqtDev& t, uint32_t cell, float u, float v) {
     if (cell >= t.ncells) return 1.0f;
-    const float* w = t.pyramid + (size_t)cell * mqt_level_offset(t.level + 1);
-    if (w[0] <= 0.0f) return 1.0f;
+    const float* w = t.pyramid + (size_t)cell * mqt_stride(t.level);
+    const float root = w[mqt_base(0)];
+    if (root <= 0.0f) return 1.0f;
     const float nn = (float)(1u << t.level);
-    const uint32_t idx = mqt_level_offset(t.level) + mqt_leaf_code(t.level, u, v);
-    return __fmul_rn(__fmul_rn(__fdiv_rn(w[idx], w[0]), nn), nn);
+    const uint32_t idx = mqt_base(t.level) + mqt_leaf_code(t.level, u, v);
+    return __fmul_rn(__fmul_rn(__fdiv_rn(w[idx], root), nn), nn);
 }
 
 }  // namespace rtpg

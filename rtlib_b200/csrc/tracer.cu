@@ -835,7 +835,12 @@ __global__ void __launch_bounds__(kCommitThreads) k_commit(TracerDev T) {
         }
         if (G == kGuideMlp && !tree_too) {
         } else if (use_grid) {
-            if (k_s != ~0ull) atomicAdd(T.mqt.leaves + k_s, v_s);
+            if (k_s != ~0ull) {
+                atomicAdd(T.mqt.leaves + k_s, v_s);
+                // a look first: a wave's vertices meet a cell a few times each, not thousands
+                uint8_t* const touched = T.mqt.touched + (k_s >> (2 * T.mqt.level));
+                if (!*touched) *touched = 1;
+            }
         } else {
             if (k_w != ~0ull) atomicAdd(priv_w ? s_w + k_w : T.tree.b_statw + k_w, v_w);
             if (k_s != ~0ull) atomicAdd(priv ? s_q + k_s : T.tree.b_sums + k_s, v_s);

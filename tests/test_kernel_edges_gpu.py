@@ -52,3 +52,80 @@ def test_record_counter_placement(cuda, oracle, threshold):
     np.testing.assert_array_equal(eg.scalars, eo.scalars)
     np.testing.assert_array_equal(eg.dsums, eo.dsums)
     assert g.status() == 0
+
+
+@pytest.mark.parametrize("level", [1, 2, 3, 4, 5, 6, 7])
+def test_morton_build_skips_only_clean_cells(cuda, oracle, level):
+    """Few cells of an odd number recorded, then others, then none: cells in use are rebuilt,
+    cells no longer in use go back to zero, leaves end cleared; samples follow the pyramid."""
+    import torch
+    from rtlib_b200.hashgrid import MortonQuadTrees
+    rng = np.random.default_rng(level)
+    ncell = 37 if level < 6 else 5
+    m = MortonQuadTrees(ncell, level=level)
+    for used in ([0, 3, ncell - 1], [3, 4], []):
+        n = 2000 if used else 0
+        cell = np.array(used, np.uint32)[rng.integers(0, len(used), n)] if n else np.zeros(0, np.uint32)
+        uv, val = rng.random((n, 2), dtype=np.float32), rng.lognormal(0, 2, n).astype(np.float32)
+        leaves = np.zeros(ncell << (2 * level), np.int64)
+        if n:
+            m.record(_t(cell, cuda), _t(uv, cuda), _t(val, cuda))
+            oracle.mqt_record(level, 24, leaves, cell, uv, val)
+        m.update()
+        want = oracle.mqt_build(ncell, level, 24, leaves)
+        got_leaves, got = m.export()
+        np.testing.assert_array_equal(got, want)
+        assert not got_leaves.any()
+        q = np.arange(5000, dtype=np.uint32) % (ncell + 1)
+        seeds = rng.integers(1, 2**32, q.size, dtype=np.uint64).astype(np.uint32)
+        o_uv = torch.empty((q.size, 2), dtype=torch.float32, device=cuda)
+        o_pdf = torch.empty(q.size, dtype=torch.float32, device=cuda)
+        m.sample_pdf(_t(q, cuda), _t(seeds, cuda), out_uv=o_uv, out_pdf_tree=o_pdf)
+        in_range = q < ncell
+        uv_w, pdf_w, _ = oracle.mqt_sample_pdf(level, want, q[in_range], seeds[in_range])
+        np.testing.assert_array_equal(o_uv.cpu().numpy()[in_range], uv_w)
+        np.testing.assert_array_equal(o_pdf.cpu().numpy()[in_range], pdf_w)
+
+
+def test_morton_choice_at_its_margins(cuda, oracle):
+    """Quadrant sums for which boundary and second comparison fall on representable draws (equal
+    quarters and halves, zero quadrants, one quadrant alone): the divisions decide, as the oracle."""
+    import torch
+    from rtlib_b200.hashgrid import MortonQuadTrees
+    sums = [(1, 1, 1, 1), (1, 0, 0, 0), (0, 0, 0, 2), (0, 3, 0, 3), (3, 0, 1, 0), (1, 1, 0, 0), (0, 0, 1, 1), (1, 2, 3, 2),
+            (1e-6, 1, 1e-6, 1), (1, 1e-6, 1, 1e-6), (5, 0, 0, 7)]
+    m = MortonQuadTrees(len(sums), level=1)
+    cell = np.repeat(np.arange(len(sums), dtype=np.uint32), 4)
+    uv = np.tile(np.array([[0.1, 0.1], [0.9, 0.1], [0.1, 0.9], [0.9, 0.9]], np.float32), (len(sums), 1))
+    val = np.array(sums, np.float32).ravel()
+    leaves = np.zeros(4 * len(sums), np.int64)
+    m.record(_t(cell, cuda), _t(uv, cuda), _t(val, cuda))
+    oracle.mqt_record(1, 24, leaves, cell, uv, val)
+    m.update()
+    pyr = oracle.mqt_build(len(sums), 1, 24, leaves)
+    q = (np.arange(1 << 20) % len(sums)).astype(np.uint32)
+    seeds = np.random.default_rng(1).integers(1, 2**32, q.size, dtype=np.uint64).astype(np.uint32)
+    o_uv = torch.empty((q.size, 2), dtype=torch.float32, device=cuda)
+    m.sample_pdf(_t(q, cuda), _t(seeds, cuda), out_uv=o_uv)
+    np.testing.assert_array_equal(o_uv.cpu().numpy(), oracle.mqt_sample_pdf(1, pyr, q, seeds)[0])
+
+
+@pytest.mark.parametrize("ncell,level,n", [(10, 2, 16 * 160), (10, 2, 16 * 160 - 1), (64, 4, 1 << 18), (65, 4, 1 << 18),
+                                           (3, 1, 1), (16384, 4, 300001)])
+def test_morton_record_routes(cuda, oracle, ncell, level, n):
+    """Private sums (few leaves, many records) and one atomic per record, at the line between them;
+    sums past 32 bits carry into the high word; every recorded cell is rebuilt."""
+    from rtlib_b200.hashgrid import MortonQuadTrees
+    rng = np.random.default_rng(n)
+    m = MortonQuadTrees(ncell, level=level)
+    cell = np.minimum((rng.random(n) ** 2 * (ncell + 1)).astype(np.uint32), ncell)  # ncell: outside, skipped
+    cell[::17] = 0xFFFFFFFF
+    uv, val = rng.random((n, 2), dtype=np.float32), rng.lognormal(3, 3, n).astype(np.float32)
+    val[::19] = np.nan
+    leaves = np.zeros(ncell << (2 * level), np.int64)
+    m.record(_t(cell, cuda), _t(uv, cuda), _t(val, cuda))
+    ok = cell < ncell
+    oracle.mqt_record(level, 24, leaves, cell[ok], uv[ok], val[ok])
+    np.testing.assert_array_equal(m.export()[0], leaves)
+    m.update()
+    np.testing.assert_array_equal(m.export()[1], oracle.mqt_build(ncell, level, 24, leaves))
