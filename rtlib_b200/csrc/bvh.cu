@@ -1,4 +1,5 @@
-// Linear BVH build over triangles and batched hit queries (rtpg_scene_*).
+// BVH build over triangles (the binary linear hierarchy, then the eight-wide one rays walk) and
+// batched hit queries (rtpg_scene_*).
 //
 // This is the hit-query boundary of the integrator: RTLib answers closest-hit and occlusion
 // queries with OptiX (optixTrace in TraceRadiance / TraceOccluded, SimpleKernel.h:347-366,
@@ -6,6 +7,7 @@
 // machine, so queries go to this CUDA BVH instead.
 #include <cub/cub.cuh>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -77,8 +79,10 @@ __device__ __forceinline__ int bvh_delta(const unsigned long long* __restrict__ 
 }
 
 // Karras 2012: node i covers a key range whose split is found by binary search
+// (count: leaves of every node)
 __global__ void k_scene_hierarchy(const unsigned long long* __restrict__ keys, int n, BvhNode* __restrict__ nodes,
-                                  uint32_t* __restrict__ parent_i, uint32_t* __restrict__ parent_l) {
+                                  uint32_t* __restrict__ parent_i, uint32_t* __restrict__ parent_l,
+                                  uint32_t* __restrict__ count) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += gridDim.x * blockDim.x) {
         const int d = (bvh_delta(keys, n, i, i + 1) - bvh_delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
         const int dmin = bvh_delta(keys, n, i, i - d);
@@ -104,6 +108,7 @@ __global__ void k_scene_hierarchy(const unsigned long long* __restrict__ keys, i
         nodes[i].child[0] = c0;
         nodes[i].child[1] = c1;
         nodes[i].pad[0] = nodes[i].pad[1] = 0;
+        count[i] = (uint32_t)(hi - lo + 1);
     }
 }
 
@@ -141,6 +146,26 @@ __device__ __forceinline__ void tri_box(const float* __restrict__ v, const uint3
     }
 }
 
+// the leaves' boxes for the walk, and their largest finite absolute coordinate (as ordered bits: a
+// nonnegative float's bits order as it does)
+__global__ void k_scene_leaf_boxes(const float* __restrict__ v, const uint32_t* __restrict__ idx,
+                                   const uint32_t* __restrict__ prim, uint32_t nt, float4* __restrict__ box,
+                                   unsigned* __restrict__ max_abs) {
+    float m = 0.0f;
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nt; k += gridDim.x * blockDim.x) {
+        float lo[3], hi[3];
+        tri_box(v, idx, prim[k], lo, hi);
+        box[2 * size_t(k)] = make_float4(lo[0], lo[1], lo[2], hi[0]);
+        box[2 * size_t(k) + 1] = make_float4(hi[1], hi[2], 0.0f, 0.0f);
+        for (int a = 0; a < 3; ++a) {
+            if (isfinite(lo[a])) m = fmaxf(m, fabsf(lo[a]));
+            if (isfinite(hi[a])) m = fmaxf(m, fabsf(hi[a]));
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(max_abs, __float_as_uint(m));
+}
+
 // bottom-up boxes: the second thread to reach an interior node merges its children
 __global__ void k_scene_boxes(const float* __restrict__ v, const uint32_t* __restrict__ idx,
                               const uint32_t* __restrict__ prim, uint32_t nt, BvhNode* nodes, const uint32_t* parent_i,
@@ -175,17 +200,305 @@ __global__ void k_scene_boxes(const float* __restrict__ v, const uint32_t* __res
     }
 }
 
+// ------------------------------------------------------------------ walked hierarchy, binary stage
+// A second binary hierarchy over the same leaves by parallel locally-ordered clustering (Meister
+// and Bittner, IEEE TVCG 24(3), 2018): clusters stay in Morton order, each looks kPlocRadius
+// neighbours to either side for the one whose common box has the least surface area, and pairs that
+// chose each other merge.  The linear hierarchy puts a large triangle (a wall) among the small ones
+// around its centroid and so inflates every box above it; here it waits until large clusters are
+// left and ends up near the root.  Equal areas are told apart by the smaller i ^ j, which is symmetric
+// and distinct for a cluster's candidates, so the least pair always merges.
+constexpr int kPlocRadius = 16;
+constexpr int kPlocBlock = 256;
+constexpr uint32_t kPlocMaxRounds = 120;  // a round adds at most one level (see k_wide_level)
+
+__device__ __forceinline__ float box_area(float4 alo, float4 ahi, float4 blo, float4 bhi) {
+    const float x = fmaxf(ahi.x, bhi.x) - fminf(alo.x, blo.x), y = fmaxf(ahi.y, bhi.y) - fminf(alo.y, blo.y),
+                z = fmaxf(ahi.z, bhi.z) - fminf(alo.z, blo.z);
+    return x * y + y * z + z * x;
+}
+// a cluster: lo.xyz and its reference (kBvhLeafBit | leaf or node), hi.xyz
+__global__ void k_ploc_init(const float4* __restrict__ leaf_box, uint32_t n, float4* __restrict__ lo, float4* __restrict__ hi) {
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const float4 a = leaf_box[2 * size_t(k)], b = leaf_box[2 * size_t(k) + 1];
+        lo[k] = make_float4(a.x, a.y, a.z, __uint_as_float(kBvhLeafBit | k));
+        hi[k] = make_float4(a.w, b.x, b.y, 0.0f);
+    }
+}
+__global__ void __launch_bounds__(kPlocBlock) k_ploc_nearest(const float4* __restrict__ lo, const float4* __restrict__ hi,
+                                                             uint32_t n, uint32_t* __restrict__ nearest) {
+    __shared__ float4 s_lo[kPlocBlock + 2 * kPlocRadius], s_hi[kPlocBlock + 2 * kPlocRadius];
+    const int base = (int)(blockIdx.x * kPlocBlock) - kPlocRadius;
+    for (int k = threadIdx.x; k < kPlocBlock + 2 * kPlocRadius; k += kPlocBlock) {
+        const int g = min(max(base + k, 0), (int)n - 1);
+        s_lo[k] = lo[g];
+        s_hi[k] = hi[g];
+    }
+    __syncthreads();
+    const uint32_t i = blockIdx.x * kPlocBlock + threadIdx.x;
+    if (i >= n) return;
+    const int me = threadIdx.x + kPlocRadius;
+    const float4 mlo = s_lo[me], mhi = s_hi[me];
+    float best = INFINITY;
+    uint32_t arg = i ^ 1u;
+    if (arg >= n) arg = i - 1;
+    for (int d = -kPlocRadius; d <= kPlocRadius; ++d) {
+        const int j = (int)i + d;
+        if (d == 0 || j < 0 || j >= (int)n) continue;
+        const float a = box_area(mlo, mhi, s_lo[me + d], s_hi[me + d]);
+        if (a < best || (a == best && ((uint32_t)j ^ i) < (arg ^ i))) {
+            best = a;
+            arg = (uint32_t)j;
+        }
+    }
+    nearest[i] = arg;
+}
+__global__ void k_ploc_merge(float4* lo, float4* hi, uint32_t n, const uint32_t* __restrict__ nearest,
+                             BvhNode* __restrict__ nodes, uint32_t* __restrict__ count, uint32_t* __restrict__ next,
+                             uint32_t* __restrict__ keep) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t j = nearest[i];
+        const bool pair = nearest[j] == i;
+        keep[i] = !pair || i < j;
+        if (!pair || i > j) continue;
+        const float4 alo = lo[i], ahi = hi[i], blo = lo[j], bhi = hi[j];
+        const uint32_t ra = __float_as_uint(alo.w), rb = __float_as_uint(blo.w), id = atomicAdd(next, 1u);
+        BvhNode nd;
+        nd.a = make_float4(alo.x, alo.y, alo.z, ahi.x);
+        nd.b = make_float4(ahi.y, ahi.z, blo.x, blo.y);
+        nd.c = make_float4(blo.z, bhi.x, bhi.y, bhi.z);
+        nd.child[0] = ra;
+        nd.child[1] = rb;
+        nd.pad[0] = nd.pad[1] = 0;
+        nodes[id] = nd;
+        count[id] = ((ra & kBvhLeafBit) ? 1u : count[ra]) + ((rb & kBvhLeafBit) ? 1u : count[rb]);
+        lo[i] = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), __uint_as_float(id));
+        hi[i] = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
+    }
+}
+__global__ void k_ploc_compact(const float4* __restrict__ lo, const float4* __restrict__ hi, uint32_t n,
+                               const uint32_t* __restrict__ keep, const uint32_t* __restrict__ at, float4* __restrict__ lo2,
+                               float4* __restrict__ hi2, uint32_t* __restrict__ left) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        if (i == n - 1) *left = at[i] + keep[i];
+        if (!keep[i]) continue;
+        lo2[at[i]] = lo[i];
+        hi2[at[i]] = hi[i];
+    }
+}
+
+// ------------------------------------------------------------------ eight-wide hierarchy
+// One level of the collapse, one thread per node of it: starting from the two children of its
+// binary node, the child of largest surface area is replaced by its own two children until
+// there are eight; single triangles become leaves.  From level kCountLevel on
+// the child with most triangles is opened instead, which bounds the depth: on the way to any
+// triangle a level then either descends seven binary levels or at least halves the triangles
+// (at most 31 times), so a binary hierarchy of D levels takes at most kCountLevel + 31 + (D - 31) / 7
+// levels: 56 for the linear one (95: 63 key bits and the index), 60 for 120 rounds of clustering.
+// Nodes with fewer than eight children have leaves only, at least two, so there are at most 5/8 as
+// many nodes as triangles.
+constexpr uint32_t kCountLevel = 16;
+struct WideChild {
+    uint32_t ref;    // binary node or kBvhLeafBit | leaf
+    uint32_t count;  // its leaves
+    float lo[3], hi[3];
+    __device__ __forceinline__ float area() const {
+        const float x = hi[0] - lo[0], y = hi[1] - lo[1], z = hi[2] - lo[2];
+        return x * y + y * z + z * x;
+    }
+};
+__device__ __forceinline__ WideChild wide_child(const BvhNode& nd, const uint32_t* __restrict__ count, float max_abs,
+                                                int k) {
+    WideChild c;
+    c.ref = nd.child[k];
+    const float b0[6] = {nd.a.x, nd.a.y, nd.a.z, nd.a.w, nd.b.x, nd.b.y}, b1[6] = {nd.b.z, nd.b.w, nd.c.x, nd.c.y, nd.c.z, nd.c.w};
+    // a triangle with a vertex that is not finite is never hit, but its box must not spoil its
+    // neighbours' planes
+    for (int a = 0; a < 3; ++a) {
+        c.lo[a] = fminf(fmaxf(k ? b1[a] : b0[a], -max_abs), max_abs);
+        c.hi[a] = fmaxf(fminf(k ? b1[3 + a] : b0[3 + a], max_abs), -max_abs);
+    }
+    c.count = (c.ref & kBvhLeafBit) ? 1u : count[c.ref];
+    return c;
+}
+// counts: [0] nodes allocated, [1] triangles placed, [2] bits of the largest coordinate; root: the binary node of every wide node
+__global__ void __launch_bounds__(128) k_wide_level(const BvhNode* __restrict__ nodes, const uint32_t* __restrict__ count,
+                                                    const BvhTri* __restrict__ tris, const uint32_t* __restrict__ prim,
+                                                    uint32_t begin, uint32_t end, uint32_t level, uint32_t* __restrict__ root,
+                                                    uint32_t cap, WideNode* __restrict__ wide, WideTri* __restrict__ wtris,
+                                                    uint32_t* __restrict__ counts) {
+    const uint32_t w = begin + blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= end) return;
+    const float max_abs = __uint_as_float(counts[2]);
+    WideChild c[8];
+    int n = 2;
+    {
+        const BvhNode nd = nodes[root[w]];
+        c[0] = wide_child(nd, count, max_abs, 0);
+        c[1] = wide_child(nd, count, max_abs, 1);
+    }
+    while (n < 8) {
+        int best = -1;
+        float key = -1.0f;
+        for (int k = 0; k < n; ++k) {
+            if (c[k].count == 1) continue;
+            const float a = level >= kCountLevel ? (float)c[k].count : c[k].area();
+            if (best < 0 || a > key) {
+                best = k;
+                key = a;
+            }
+        }
+        if (best < 0) break;
+        const BvhNode nd = nodes[c[best].ref];
+        c[best] = wide_child(nd, count, max_abs, 0);
+        c[n++] = wide_child(nd, count, max_abs, 1);
+    }
+    float lo[3], hi[3];
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = c[0].lo[a];
+        hi[a] = c[0].hi[a];
+        for (int k = 1; k < n; ++k) {
+            lo[a] = fminf(lo[a], c[k].lo[a]);
+            hi[a] = fmaxf(hi[a], c[k].hi[a]);
+        }
+    }
+    // slots: the pair of a free slot and an unplaced child whose centre lies furthest towards the
+    // slot's octant, until all are placed
+    int slot_of[8];
+    {
+        uint32_t placed = 0, taken = 0;
+        for (int j = 0; j < n; ++j) {
+            int bk = -1, bs = 0;
+            float bv = 0.0f;
+            for (int k = 0; k < n; ++k) {
+                if (placed >> k & 1u) continue;
+                float d[3];
+                for (int a = 0; a < 3; ++a) d[a] = (c[k].lo[a] + c[k].hi[a]) - (lo[a] + hi[a]);
+                for (int q = 0; q < 8; ++q) {
+                    if (taken >> q & 1u) continue;
+                    const float val = ((q & 1) ? d[0] : -d[0]) + ((q & 2) ? d[1] : -d[1]) + ((q & 4) ? d[2] : -d[2]);
+                    if (bk < 0 || val > bv) {
+                        bk = k;
+                        bs = q;
+                        bv = val;
+                    }
+                }
+            }
+            slot_of[bk] = bs;
+            placed |= 1u << bk;
+            taken |= 1u << bs;
+        }
+    }
+    int in_slot[8];
+    for (int q = 0; q < 8; ++q) in_slot[q] = -1;
+    uint32_t imask = 0, lmask = 0;
+    for (int k = 0; k < n; ++k) {
+        in_slot[slot_of[k]] = k;
+        (c[k].count > 1 ? imask : lmask) |= 1u << slot_of[k];
+    }
+    WideNode nd;
+    // planes: a step of at least 2 ulp of the coordinates, origin one step below the box
+    double step[3];
+    nd.exp = imask << 24;
+    for (int a = 0; a < 3; ++a) {
+        int e = -100, m = 0;
+        if (hi[a] > lo[a]) frexp(((double)hi[a] - (double)lo[a]) / 250.0, &e);
+        frexp(fmax(fabs((double)lo[a]), fabs((double)hi[a])), &m);
+        e = max(max(e, m - 22), -100);
+        step[a] = ldexp(1.0, e);
+        nd.org[a] = (float)((double)lo[a] - step[a]);
+        nd.exp |= uint32_t(min(e + 127, 254)) << (8 * a);
+    }
+    nd.lmask = lmask;
+    nd.pad0 = 0;
+    for (int q = 0; q < 4; ++q) nd.pad1[q] = 0;
+    nd.child_base = imask ? atomicAdd(counts, (uint32_t)__popc(imask)) : 0u;
+    nd.tri_base = lmask ? atomicAdd(counts + 1, (uint32_t)__popc(lmask)) : 0u;
+    uint32_t child = nd.child_base, tri = nd.tri_base;
+    for (int q = 0; q < 8; ++q) {
+        const int k = in_slot[q];
+        for (int a = 0; a < 3; ++a) {
+            nd.qlo[a][q] = 0;
+            nd.qhi[a][q] = 0;
+        }
+        if (k < 0) continue;
+        for (int a = 0; a < 3; ++a) {
+            const double x0 = ((double)c[k].lo[a] - (double)nd.org[a]) / step[a], x1 = ((double)c[k].hi[a] - (double)nd.org[a]) / step[a];
+            nd.qlo[a][q] = (uint8_t)fmin(fmax(floor(x0 - 0.015625), 0.0), 255.0);
+            nd.qhi[a][q] = (uint8_t)fmin(fmax(ceil(x1 + 0.015625), 0.0), 255.0);
+        }
+        if (imask >> q & 1u) {
+            if (child < cap) root[child] = c[k].ref;
+            ++child;
+        } else {
+            const uint32_t leaf = c[k].ref & ~kBvhLeafBit;
+            WideTri t;
+            t.tr = tris[leaf];
+            t.leaf = leaf;
+            t.prim = prim[leaf];
+            t.pad[0] = t.pad[1] = 0;
+            wtris[tri++] = t;
+        }
+    }
+    wide[w] = nd;
+}
+
+struct HitOut {
+    float* t;
+    uint32_t* prim;
+    float* uv;
+    __device__ __forceinline__ void put(int64_t i, const Hit& h) const {
+        if (t) t[i] = h.prim == 0xffffffffu ? -1.0f : h.t;
+        if (prim) prim[i] = h.prim;
+        if (uv) reinterpret_cast<float2*>(uv)[i] = make_float2(h.u, h.v);
+    }
+};
 template <bool ANY>
-__global__ void __launch_bounds__(128) k_scene_intersect(SceneDev s, int64_t n, const float* __restrict__ org,
-                                                         const float* __restrict__ dir, const float* __restrict__ tmin,
-                                                         const float* __restrict__ tmax, float* __restrict__ out_t,
-                                                         uint32_t* __restrict__ out_prim, float* __restrict__ out_uv) {
+__global__ void __launch_bounds__(128) k_scene_intersect_flat(SceneDev s, int64_t n, const float* __restrict__ org,
+                                                              const float* __restrict__ dir, const float* __restrict__ tmin,
+                                                              const float* __restrict__ tmax, HitOut o) {
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
-        const Hit h = bvh_trace<ANY>(s, org[3 * i], org[3 * i + 1], org[3 * i + 2], dir[3 * i], dir[3 * i + 1],
-                                     dir[3 * i + 2], tmin ? tmin[i] : 0.0f, tmax ? tmax[i] : 1e20f);
-        if (out_t) out_t[i] = h.prim == 0xffffffffu ? -1.0f : h.t;
-        if (out_prim) out_prim[i] = h.prim;
-        if (out_uv) reinterpret_cast<float2*>(out_uv)[i] = make_float2(h.u, h.v);
+        Hit h;
+        h.prim = 0xffffffffu;
+        h.t = h.u = h.v = 0.0f;
+        if (s.ntris)
+            h = flat_trace<ANY>(s.flat, s.ntris, org[3 * i], org[3 * i + 1], org[3 * i + 2], dir[3 * i], dir[3 * i + 1],
+                                dir[3 * i + 2], tmin ? tmin[i] : 0.0f, tmax ? tmax[i] : 1e20f);
+        o.put(i, h);
+    }
+}
+// Each warp owns `share` consecutive rays.  Walks end at very different steps, so whenever fewer
+// than kRefill lanes are still walking the others take the warp's next rays.
+constexpr int kRefill = 28;
+constexpr int kWalkCtas = 8;
+template <bool ANY>
+__global__ void __launch_bounds__(128, 8) k_scene_intersect(SceneDev s, int64_t n, int64_t share, const float* __restrict__ org,
+                                                         const float* __restrict__ dir, const float* __restrict__ tmin,
+                                                         const float* __restrict__ tmax, HitOut o) {
+    const uint32_t lane = threadIdx.x & 31u;
+    int64_t next = (int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * share;
+    const int64_t end = min(next + share, n);
+    if (next >= end) return;
+    int64_t i = -1;
+    WideWalk<ANY> w(s, 0.f, 0.f, 0.f, 1.f, 1.f, 1.f, 0.f, 0.f);
+    w.g.y = 0u;
+    uint2 stack[kWideStack];
+    for (;;) {
+        const unsigned idle = __ballot_sync(0xffffffffu, !w.alive());
+        if (idle && (next < end ? __popc(idle) > 32 - kRefill : idle == 0xffffffffu)) {
+            if (!w.alive()) {
+                if (i >= 0) o.put(i, w.h);
+                i = next + __popc(idle & ((1u << lane) - 1u));
+                if (i < end)
+                    w = WideWalk<ANY>(s, org[3 * i], org[3 * i + 1], org[3 * i + 2], dir[3 * i], dir[3 * i + 1], dir[3 * i + 2],
+                                      tmin ? tmin[i] : 0.0f, tmax ? tmax[i] : 1e20f);
+                else
+                    i = -1;
+            }
+            if (next >= end) break;
+            next += __popc(idle);
+        }
+        w.step(s, stack);
     }
 }
 
@@ -196,8 +509,9 @@ using namespace rtpg;
 struct rtpg_scene {
     SceneDev dev{};
     BvhNode* nodes = nullptr;
-    BvhTri* tris = nullptr;
-    uint32_t* prim = nullptr;
+    float4* leaf_box = nullptr;
+    WideNode* wide = nullptr;
+    WideTri* wtris = nullptr;
     BvhTri* flat = nullptr;
     std::vector<void*> allocs;
     size_t bytes = 0;
@@ -240,38 +554,80 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
     uint32_t *v0 = nullptr, *v1 = nullptr, *pi = nullptr, *pl = nullptr;
     float4* ibox = nullptr;
     unsigned* flags = nullptr;
-    void* temp = nullptr;
-    size_t tb = 0;
+    BvhTri* tris = nullptr;  // the triangles in leaf order, and their scene indices
+    uint32_t *prim = nullptr, *root = nullptr, *counts = nullptr;
+    uint32_t *count = nullptr, *pcount = nullptr, *nearest = nullptr, *keep = nullptr, *at = nullptr;
+    BvhNode* pnodes = nullptr;
+    float4 *clo[2] = {nullptr, nullptr}, *chi[2] = {nullptr, nullptr};
+    uint8_t *sort_temp = nullptr, *scan_temp = nullptr;
     cub::DoubleBuffer<unsigned long long> dk(nullptr, nullptr);
     cub::DoubleBuffer<uint32_t> dv(nullptr, nullptr);
-    if ((r = s->alloc(&s->nodes, n > 1 ? n - 1 : 1)) || (r = s->alloc(&s->tris, n)) || (r = s->alloc(&s->prim, n)) ||
-        (n > 0 && n <= kFlatTris && (r = s->alloc(&s->flat, n)))) {
+    // small scenes are a flat list; the others get both hierarchies
+    const bool flat = n <= kFlatTris;
+    const uint32_t wide_cap = n / 8 * 5 + 8;
+    if (n > 0 && (flat ? (r = s->alloc(&s->flat, n))
+                       : (r = s->alloc(&s->nodes, n - 1)) || (r = s->alloc(&s->leaf_box, 2 * size_t(n))) ||
+                             (r = s->alloc(&s->wide, wide_cap)) || (r = s->alloc(&s->wtris, n)))) {
         delete s;
         return r;
     }
     s->dev.nodes = s->nodes;
-    s->dev.tris = s->tris;
-    s->dev.prim = s->prim;
+    s->dev.leaf_box = s->leaf_box;
+    s->dev.wide = s->wide;
+    s->dev.wtris = s->wtris;
     s->dev.flat = s->flat;
     s->dev.ntris = n;
     if (n == 0) {
         *out = s;
         return RTPG_OK;
     }
-    std::vector<void*> tmp;
-    auto talloc = [&](size_t bytes, void** p) -> cudaError_t {
-        cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
-        if (e == cudaSuccess) tmp.push_back(*p);
-        return e;
-    };
-    cudaError_t e = cudaSuccess;
-    if ((e = talloc(6 * 4, (void**)&bounds)) || (e = talloc(8ull * n, (void**)&k0)) || (e = talloc(8ull * n, (void**)&k1)) ||
-        (e = talloc(4ull * n, (void**)&v0)) || (e = talloc(4ull * n, (void**)&v1)) || (e = talloc(4ull * n, (void**)&pi)) ||
-        (e = talloc(4ull * n, (void**)&pl)) || (e = talloc(32ull * n, (void**)&ibox)) || (e = talloc(4ull * n, (void**)&flags))) {
-        for (void* p : tmp) cudaFree(p);
+    // all scratch in one allocation, freed at the end
+    size_t sort_bytes = 0, scan_bytes = 0;
+    cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, dk, dv, (int)n, 0, 63, st);
+    if (!e && !flat) e = cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, keep, at, (int)n, st);
+    if (e) {
         delete s;
-        cudaGetLastError();
-        return fail(RTPG_ENOMEM, "rtpg_scene_create: scratch allocation failed");
+        return fail(RTPG_ECUDA, "rtpg_scene_create: %s", cudaGetErrorString(e));
+    }
+    void* scratch = nullptr;
+    for (int pass = 0; pass < 2; ++pass) {  // sizes, then places
+        size_t at_byte = 0;
+        auto take = [&](auto** p, size_t count) {
+            if (pass) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(static_cast<char*>(scratch) + at_byte);
+            at_byte += (count * sizeof(**p) + 255) & ~size_t(255);
+        };
+        take(&bounds, 6);
+        take(&k0, n);
+        take(&k1, n);
+        take(&v0, n);
+        take(&v1, n);
+        take(&tris, n);
+        take(&prim, n);
+        take(&sort_temp, sort_bytes);
+        if (!flat) {
+            take(&pi, n);
+            take(&pl, n);
+            take(&ibox, 2 * size_t(n));
+            take(&flags, n);
+            take(&root, wide_cap);
+            take(&counts, 5);
+            take(&count, n);
+            take(&pcount, n);
+            take(&nearest, n);
+            take(&keep, n);
+            take(&at, n);
+            take(&pnodes, n);
+            for (int k = 0; k < 2; ++k) {
+                take(&clo[k], n);
+                take(&chi[k], n);
+            }
+            take(&scan_temp, scan_bytes);
+        }
+        if (!pass && (e = cudaMalloc(&scratch, at_byte))) {
+            cudaGetLastError();
+            delete s;
+            return fail(RTPG_ENOMEM, "rtpg_scene_create: scratch allocation failed");
+        }
     }
     const unsigned init[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
     const int g = grid_for(n, 256, 8);
@@ -282,26 +638,67 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
         k_scene_morton<<<g, 256, 0, st>>>(vertices, indices, n, bounds, k0, v0);
         dk = cub::DoubleBuffer<unsigned long long>(k0, k1);
         dv = cub::DoubleBuffer<uint32_t>(v0, v1);
-        if ((e = cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, dv, (int)n, 0, 63, st))) break;
-        if ((e = talloc(tb, &temp))) break;
-        if ((e = cub::DeviceRadixSort::SortPairs(temp, tb, dk, dv, (int)n, 0, 63, st))) break;
-        k_scene_leaves<<<g, 256, 0, st>>>(vertices, indices, n, dv.Current(), s->tris, s->prim);
-        if (s->flat) k_scene_flat<<<1, 64, 0, st>>>(s->tris, s->prim, n, s->flat);
-        if (n > 1) {
-            k_scene_hierarchy<<<g, 256, 0, st>>>(dk.Current(), (int)n, s->nodes, pi, pl);
+        if ((e = cub::DeviceRadixSort::SortPairs(sort_temp, sort_bytes, dk, dv, (int)n, 0, 63, st))) break;
+        k_scene_leaves<<<g, 256, 0, st>>>(vertices, indices, n, dv.Current(), tris, prim);
+        if (flat) {
+            k_scene_flat<<<1, 64, 0, st>>>(tris, prim, n, s->flat);
+        } else {
+            k_scene_hierarchy<<<g, 256, 0, st>>>(dk.Current(), (int)n, s->nodes, pi, pl, count);
             if ((e = cudaMemsetAsync(flags, 0, 4ull * n, st))) break;
-            k_scene_boxes<<<g, 256, 0, st>>>(vertices, indices, s->prim, n, s->nodes, pi, pl, ibox, flags);
+            k_scene_boxes<<<g, 256, 0, st>>>(vertices, indices, prim, n, s->nodes, pi, pl, ibox, flags);
+            // counts: wide nodes, triangles, largest absolute coordinate, clustered nodes, clusters
+            const uint32_t init_counts[5] = {1u, 0u, 0u, 0u, n};
+            if ((e = cudaMemcpyAsync(counts, init_counts, sizeof(init_counts), cudaMemcpyHostToDevice, st))) break;
+            k_scene_leaf_boxes<<<g, 256, 0, st>>>(vertices, indices, prim, n, s->leaf_box, counts + 2);
+            k_ploc_init<<<g, 256, 0, st>>>(s->leaf_box, n, clo[0], chi[0]);
+            uint32_t clusters = n, rounds = 0;
+            for (; clusters > 1 && rounds < kPlocMaxRounds && !e; ++rounds) {
+                const int a = rounds & 1, b = a ^ 1, gc = grid_for(clusters, 256, 8);
+                k_ploc_nearest<<<(clusters + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, st>>>(clo[a], chi[a], clusters, nearest);
+                k_ploc_merge<<<gc, 256, 0, st>>>(clo[a], chi[a], clusters, nearest, pnodes, pcount, counts + 3, keep);
+                if ((e = cub::DeviceScan::ExclusiveSum(scan_temp, scan_bytes, keep, at, (int)clusters, st))) break;
+                k_ploc_compact<<<gc, 256, 0, st>>>(clo[a], chi[a], clusters, keep, at, clo[b], chi[b], counts + 4);
+                if ((e = cudaMemcpyAsync(&clusters, counts + 4, 4, cudaMemcpyDeviceToHost, st))) break;
+                e = cudaStreamSynchronize(st);
+            }
+            if (e) break;
+            // the clustered hierarchy (its root was made last) or, where clustering took too many
+            // rounds (coincident triangles), the linear one
+            const bool clustered = clusters == 1;
+            const BvhNode* const bin = clustered ? pnodes : s->nodes;
+            const uint32_t* const bin_count = clustered ? pcount : count;
+            const uint32_t bin_root = clustered ? n - 2 : 0;
+            if ((e = cudaMemcpyAsync(root, &bin_root, 4, cudaMemcpyHostToDevice, st))) break;
+            uint32_t begin = 0, end = 1, now[3] = {1, 0, 0};
+            for (uint32_t level = 0; begin < end; ++level) {
+                if (level >= (uint32_t)kWideStack || end > wide_cap) {
+                    rc = fail(RTPG_ECAPACITY, "rtpg_scene_create: hierarchy of %u nodes in %u levels exceeds its bounds", end, level);
+                    break;
+                }
+                k_wide_level<<<(end - begin + 127) / 128, 128, 0, st>>>(bin, bin_count, tris, prim, begin, end, level, root,
+                                                                       wide_cap, s->wide, s->wtris, counts);
+                if ((e = cudaMemcpyAsync(now, counts, sizeof(now), cudaMemcpyDeviceToHost, st))) break;
+                if ((e = cudaStreamSynchronize(st))) break;
+                begin = end;
+                end = now[0];
+            }
+            if (e || rc) break;
+            memcpy(&s->dev.max_abs, &now[2], 4);
         }
         if ((e = cudaGetLastError())) break;
         if ((e = cudaStreamSynchronize(st))) break;
     } while (0);
-    for (void* p : tmp) cudaFree(p);
+    cudaFree(scratch);
     if (e != cudaSuccess) {
         delete s;
         return fail(RTPG_ECUDA, "rtpg_scene_create: %s", cudaGetErrorString(e));
     }
+    if (rc) {
+        delete s;
+        return rc;
+    }
     *out = s;
-    return rc;
+    return RTPG_OK;
 }
 
 int rtpg_scene_destroy(rtpg_scene* s) {
@@ -316,11 +713,20 @@ int rtpg_scene_intersect(rtpg_scene* s, int64_t n, const float* org, const float
     if (!s) return fail(RTPG_EINVAL, "rtpg_scene_intersect: null handle");
     if (n < 0 || (n > 0 && (!org || !dir))) return fail(RTPG_EINVAL, "rtpg_scene_intersect: bad arguments");
     if (n == 0) return RTPG_OK;
-    const int g = grid_for(n, 128, 16);
-    if (any_hit)
-        k_scene_intersect<true><<<g, 128, 0, as_stream(stream)>>>(s->dev, n, org, dir, tmin, tmax, out_t, out_prim, out_uv);
-    else
-        k_scene_intersect<false><<<g, 128, 0, as_stream(stream)>>>(s->dev, n, org, dir, tmin, tmax, out_t, out_prim, out_uv);
+    cudaStream_t st = as_stream(stream);
+    const HitOut o{out_t, out_prim, out_uv};
+    if (s->dev.flat || s->dev.ntris == 0) {
+        const int g = grid_for(n, 128, 16);
+        if (any_hit) k_scene_intersect_flat<true><<<g, 128, 0, st>>>(s->dev, n, org, dir, tmin, tmax, o);
+        else k_scene_intersect_flat<false><<<g, 128, 0, st>>>(s->dev, n, org, dir, tmin, tmax, o);
+    } else {
+        // a share of at least a warp's rays on at most kWalkCtas CTAs per SM
+        const int64_t warps = int64_t(kSMs) * kWalkCtas * 4;
+        const int64_t share = std::max<int64_t>(32, (n + warps - 1) / warps);
+        const int g = (int)((n + 4 * share - 1) / (4 * share));
+        if (any_hit) k_scene_intersect<true><<<g, 128, 0, st>>>(s->dev, n, share, org, dir, tmin, tmax, o);
+        else k_scene_intersect<false><<<g, 128, 0, st>>>(s->dev, n, share, org, dir, tmin, tmax, o);
+    }
     RTPG_LAUNCH_CHECK();
     return RTPG_OK;
 }

@@ -107,11 +107,11 @@ struct TracerDev {
 };
 
 // closest hit (ANY = false) or any hit (ANY = true) in (tmin, tmax): the scene's triangles from
-// the kernel parameters when it is small, else the BVH
-template <bool ANY>
+// the kernel parameters when it is small (FLAT), else the BVH
+template <bool ANY, bool FLAT>
 __device__ __forceinline__ Hit trace(const TracerDev& T, float ox, float oy, float oz, float dx, float dy, float dz,
                                      float tmin, float tmax) {
-    if (T.nflat) return flat_trace<ANY>(T.ftri, T.nflat, ox, oy, oz, dx, dy, dz, tmin, tmax);
+    if (FLAT) return flat_trace<ANY>(T.ftri, T.nflat, ox, oy, oz, dx, dy, dz, tmin, tmax);
     return bvh_trace<ANY>(T.scene, ox, oy, oz, dx, dy, dz, tmin, tmax);
 }
 
@@ -195,7 +195,7 @@ constexpr int kGuideNone = 0, kGuideTree = 1, kGuideGrid = 2, kAdjoint = 3, kGui
 // at a textured vertex it holds exactly the terms that carry the vertex's albedo as a factor
 // (its NEE term and everything after it); the albedo gradient is delta * lrem / albedo per
 // channel.  An emitter's gradient is delta * (the term's factor in front of its radiance).
-template <int G>
+template <int G, bool FLAT>
 __device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, bool build, bool recording, bool& shadow) {
     constexpr bool use_tree = G == kGuideTree, use_grid = G == kGuideGrid, adjoint = G == kAdjoint;
     constexpr bool use_mlp = G == kGuideMlp;
@@ -209,7 +209,7 @@ __device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, bool
         h.u = tuv.y;
         h.v = tuv.z;
     } else {
-        h = trace<false>(T, org.x, org.y, org.z, in_dir.x, in_dir.y, in_dir.z, 0.0001f, 1.0e20f);
+        h = trace<false, FLAT>(T, org.x, org.y, org.z, in_dir.x, in_dir.y, in_dir.z, 0.0001f, 1.0e20f);
     }
     const size_t vi = size_t(d < kTV ? d : 0) * T.npath + p;
     bool pend = false;
@@ -517,7 +517,7 @@ __device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, bool
     bool lit = false;
     if (pend) {
         shadow = true;
-        const Hit sh = trace<true>(T, position.x, position.y, position.z, sdir.x, sdir.y, sdir.z, 0.0001f, sdist);
+        const Hit sh = trace<true, FLAT>(T, position.x, position.y, position.z, sdir.x, sdir.y, sdir.z, 0.0001f, sdist);
         if (sh.prim == 0xffffffffu) {
             L = L + scontrib;
             lit = true;
@@ -561,7 +561,7 @@ __device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, bool
     if (use_mlp) {
         // the closest hit of the continuing ray, traced here rather than in a pass of its own,
         // so the network of the next bounce finds it waiting (k_hit serves the first bounce)
-        const Hit nh = trace<false>(T, position.x, position.y, position.z, direction.x, direction.y,
+        const Hit nh = trace<false, FLAT>(T, position.x, position.y, position.z, direction.x, direction.y,
                                         direction.z, 0.0001f, 1.0e20f);
         T.hit_prim[p] = nh.prim;
         T.hit_tuv[p] = make_float4(nh.t, nh.u, nh.v, 0.0f);
@@ -580,6 +580,7 @@ __host__ __device__ constexpr int guide_of(uint32_t flags) {
 
 // learned guide, stage 1 of the first bounce: closest hits of the camera rays (later bounces
 // find theirs traced at the end of the previous k_bounce)
+template <bool FLAT>
 __global__ void __launch_bounds__(kTB) k_hit(TracerDev T, uint32_t bounce) {
     grid_dependency_wait();
     const int in = int(bounce & 1);
@@ -587,7 +588,7 @@ __global__ void __launch_bounds__(kTB) k_hit(TracerDev T, uint32_t bounce) {
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
         const uint32_t p = T.queue[in][q];
         const float3 o = T.org[p], d = T.dir[p];
-        const Hit h = trace<false>(T, o.x, o.y, o.z, d.x, d.y, d.z, 0.0001f, 1.0e20f);
+        const Hit h = trace<false, FLAT>(T, o.x, o.y, o.z, d.x, d.y, d.z, 0.0001f, 1.0e20f);
         T.hit_prim[p] = h.prim;
         T.hit_tuv[p] = make_float4(h.t, h.u, h.v, 0.0f);
     }
@@ -670,8 +671,11 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_lobes(TracerDev T, uint32_t
     if (t < 32) tmem_dealloc(tmem, kEvalCols);
 }
 
-template <int G>
-__global__ void __launch_bounds__(kTB, 8) k_bounce(TracerDev T, uint32_t bounce) {
+// FLAT: the scene's triangles are in the kernel parameters.  A template argument, so that neither
+// variant carries the other's registers.
+constexpr int kBvhCtas = 8;
+template <int G, bool FLAT>
+__global__ void __launch_bounds__(kTB, FLAT ? 8 : kBvhCtas) k_bounce(TracerDev T, uint32_t bounce) {
     grid_dependency_wait();
     const int in = int(bounce & 1);
     uint32_t* const next_count = T.qcount + (bounce + 1) % 3;
@@ -689,7 +693,7 @@ __global__ void __launch_bounds__(kTB, 8) k_bounce(TracerDev T, uint32_t bounce)
         uint32_t p = 0;
         if (q < n) {
             p = T.queue[in][q];
-            keep = bounce_path<G>(T, p, build, recording, shadow);
+            keep = bounce_path<G, FLAT>(T, p, build, recording, shadow);
         }
         const unsigned sh = __ballot_sync(0xffffffffu, shadow);
         if ((threadIdx.x & 31) == 0 && sh) atomicAdd(T.counters + 1, (unsigned long long)__popc(sh));
@@ -939,17 +943,21 @@ struct rtpg_tracer {
 // others finish, which balances a bounce's tail better than a resident grid striding over the
 // queue (measured 4% faster on the Cornell render); CTAs past the queue's end return at once.
 static int bounce_grid(const TracerDev& T) { return (int)((T.npath + kTB - 1) / kTB); }
+template <int G>
+static void launch_bounce_of(const TracerDev& T, int g, cudaStream_t st, uint32_t b) {
+    if (T.nflat) (void)launch_dependent(k_bounce<G, true>, g, kTB, 0, st, T, b);
+    else (void)launch_dependent(k_bounce<G, false>, g, kTB, 0, st, T, b);
+}
 static void launch_bounce(const TracerDev& T, int g, cudaStream_t st, uint32_t b) {
-    if (guide_of(T.flags) == kGuideMlp) {
-        if (b == 0) (void)launch_dependent(k_hit, g, kTB, 0, st, T, b);
-        if (T.flags & RTPG_TRACE_FLAG_BUILD) (void)launch_dependent(k_mlp_lobes, kSMs * 4, kMlpThreads, kSmemEval, st, T, b);
-        (void)launch_dependent(k_bounce<kGuideMlp>, g, kTB, 0, st, T, b);
-        return;
-    }
     switch (guide_of(T.flags)) {
-        case kGuideTree: (void)launch_dependent(k_bounce<kGuideTree>, g, kTB, 0, st, T, b); break;
-        case kGuideGrid: (void)launch_dependent(k_bounce<kGuideGrid>, g, kTB, 0, st, T, b); break;
-        default: (void)launch_dependent(k_bounce<kGuideNone>, g, kTB, 0, st, T, b); break;
+        case kGuideMlp:
+            if (b == 0) (void)launch_dependent(T.nflat ? k_hit<true> : k_hit<false>, g, kTB, 0, st, T, b);
+            if (T.flags & RTPG_TRACE_FLAG_BUILD) (void)launch_dependent(k_mlp_lobes, kSMs * 4, kMlpThreads, kSmemEval, st, T, b);
+            launch_bounce_of<kGuideMlp>(T, g, st, b);
+            break;
+        case kGuideTree: launch_bounce_of<kGuideTree>(T, g, st, b); break;
+        case kGuideGrid: launch_bounce_of<kGuideGrid>(T, g, st, b); break;
+        default: launch_bounce_of<kGuideNone>(T, g, st, b); break;
     }
 }
 // accumulation, then (recording waves of a guide) the commit of the trace vertices: two CTAs
@@ -1479,9 +1487,9 @@ int rtpg_tracer_render_adjoint(rtpg_tracer* h, uint32_t spp, uint32_t flags, con
     const int g = kSMs * 8;
     for (uint32_t s = 0; s < spp; ++s) {
         k_raygen<<<g, kTB, 0, st>>>(A);
-        for (uint32_t b = 0; b < A.max_depth; ++b) k_bounce<kGuideNone><<<g, kTB, 0, st>>>(A, b);
+        for (uint32_t b = 0; b < A.max_depth; ++b) launch_bounce_of<kGuideNone>(A, g, st, b);
         k_raygen<<<g, kTB, 0, st>>>(B);
-        for (uint32_t b = 0; b < B.max_depth; ++b) k_bounce<kAdjoint><<<g, kTB, 0, st>>>(B, b);
+        for (uint32_t b = 0; b < B.max_depth; ++b) launch_bounce_of<kAdjoint>(B, g, st, b);
         k_seed_store<<<g, kTB, 0, st>>>(B);
     }
     RTPG_LAUNCH_CHECK();

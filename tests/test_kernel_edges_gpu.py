@@ -129,3 +129,55 @@ def test_morton_record_routes(cuda, oracle, ncell, level, n):
     np.testing.assert_array_equal(m.export()[0], leaves)
     m.update()
     np.testing.assert_array_equal(m.export()[1], oracle.mqt_build(ncell, level, 24, leaves))
+
+
+@pytest.mark.parametrize("n", [64, 65, 66, 73, 500, 3000])
+def test_hierarchy_hits(cuda, oracle, n):
+    """Hits of the eight-wide hierarchy against brute force over soups of mixed sizes (walls among
+    small triangles), with degenerate, duplicate, flat and non-finite triangles, rays along the axes,
+    from far outside and with their own bounds: the same distance bit for bit."""
+    import torch
+    from rtlib_b200.tracer import Scene
+    rng = np.random.default_rng(n)
+    tri = (rng.normal(size=(n, 3, 3)) * 0.15 + rng.uniform(-3, 3, (n, 1, 3))).astype(np.float32)
+    tri[0] = [[-4, -4, 3], [4, -4, 3], [4, 4, 3]]
+    tri[1] = [[-4, -3, -4], [4, -3, 4], [4, -3, -4]]
+    tri[2] = tri[3]                       # duplicates
+    tri[4, 2] = tri[4, 1]                 # no area
+    tri[5, :, 1] = 0.25                   # flat box
+    if n > 65:
+        tri[6, 0, 0], tri[7, 1, 2], tri[8, 2] = np.nan, np.inf, -np.inf
+    q = 20000
+    org = rng.uniform(-3.5, 3.5, (q, 3)).astype(np.float32)
+    org[:200] *= 100.0
+    d = rng.normal(size=(q, 3)).astype(np.float32)
+    d[200:500] = np.eye(3, dtype=np.float32)[rng.integers(0, 3, 300)] * rng.choice([-1, 1], (300, 1)).astype(np.float32)
+    d[:200] = -org[:200]
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    sc = Scene(_t(tri.reshape(n, 9), cuda))
+    t, p, occ = torch.empty(q, device=cuda), torch.empty(q, dtype=torch.int32, device=cuda), torch.empty(q, dtype=torch.int32, device=cuda)
+    for tmin, tmax in ((0.0, 1e20), (0.5, 2.0)):
+        lo, hi = _t(np.full(q, tmin, np.float32), cuda), _t(np.full(q, tmax, np.float32), cuda)
+        sc.intersect(_t(org, cuda), _t(d, cuda), lo, hi, out_t=t, out_prim=p)
+        sc.intersect(_t(org, cuda), _t(d, cuda), lo, hi, any_hit=True, out_prim=occ)
+        want_t, want_p = oracle.intersect(tri.reshape(n, 9), org, d, tmin, tmax)[:2]
+        got_p = p.cpu().numpy().view(np.uint32)
+        # duplicates may answer for one another
+        same = (got_p == want_p) | (np.isin(got_p, (2, 3)) & np.isin(want_p, (2, 3)))
+        assert same.all(), np.flatnonzero(~same)[:5]
+        hit = want_p != 0xFFFFFFFF
+        np.testing.assert_array_equal(t.cpu().numpy()[hit], want_t[hit])
+        np.testing.assert_array_equal(occ.cpu().numpy() != -1, hit)
+
+
+def test_hierarchy_of_coincident_triangles(cuda):
+    """Equal boxes everywhere: clustering still pairs, the depth stays bounded, rays end."""
+    import torch
+    from rtlib_b200.tracer import Scene
+    tri = np.tile(np.array([[0, 0, 1, 1, 0, 1, 0, 1, 1]], np.float32), (5000, 1))
+    sc = Scene(_t(tri, cuda))
+    org = _t(np.tile(np.array([[0.2, 0.2, 0.0]], np.float32), (4097, 1)), cuda)
+    d = _t(np.tile(np.array([[0, 0, 1]], np.float32), (4097, 1)), cuda)
+    t, p = torch.empty(4097, device=cuda), torch.empty(4097, dtype=torch.int32, device=cuda)
+    sc.intersect(org, d, out_t=t, out_prim=p)
+    assert (t == 1.0).all() and (p == p[0]).all()
