@@ -125,10 +125,23 @@ __global__ void k_scene_leaves(const float* __restrict__ v, const uint32_t* __re
     }
 }
 
-// the leaves back in scene order, for small scenes
+// the leaves back in scene order, as pairs, for small scenes
 __global__ void k_scene_flat(const BvhTri* __restrict__ tris, const uint32_t* __restrict__ prim, uint32_t nt,
-                             BvhTri* __restrict__ flat) {
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nt; k += gridDim.x * blockDim.x) flat[prim[k]] = tris[k];
+                             FlatPair* __restrict__ flat) {
+    auto put = [&](uint32_t i, const BvhTri& t) {
+        float* const w = reinterpret_cast<float*>(flat + i / 2) + (i & 1u);
+        const float4 r[3] = {t.r0, t.r1, t.r2};
+        for (int a = 0; a < 3; ++a) {
+            w[8 * a] = r[a].x;
+            w[8 * a + 2] = r[a].y;
+            w[8 * a + 4] = r[a].z;
+            w[8 * a + 6] = r[a].w;
+        }
+    };
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nt; k += gridDim.x * blockDim.x) put(prim[k], tris[k]);
+    // u = -1 everywhere
+    if ((nt & 1u) && blockIdx.x == 0 && threadIdx.x == 0)
+        put(nt, BvhTri{make_float4(0.f, 0.f, 0.f, -1.f), make_float4(0.f, 0.f, 0.f, 0.f), make_float4(1.f, 0.f, 0.f, 0.f)});
 }
 
 // the box of scene triangle p, widened by a relative margin so that it contains the triangle
@@ -462,7 +475,7 @@ __global__ void __launch_bounds__(128) k_scene_intersect_flat(SceneDev s, int64_
         h.prim = 0xffffffffu;
         h.t = h.u = h.v = 0.0f;
         if (s.ntris)
-            h = flat_trace<ANY>(s.flat, s.ntris, org[3 * i], org[3 * i + 1], org[3 * i + 2], dir[3 * i], dir[3 * i + 1],
+            h = flat_trace<ANY>(s.flat, flat_pairs(s.ntris), org[3 * i], org[3 * i + 1], org[3 * i + 2], dir[3 * i], dir[3 * i + 1],
                                 dir[3 * i + 2], tmin ? tmin[i] : 0.0f, tmax ? tmax[i] : 1e20f);
         o.put(i, h);
     }
@@ -512,7 +525,7 @@ struct rtpg_scene {
     float4* leaf_box = nullptr;
     WideNode* wide = nullptr;
     WideTri* wtris = nullptr;
-    BvhTri* flat = nullptr;
+    FlatPair* flat = nullptr;
     std::vector<void*> allocs;
     size_t bytes = 0;
     template <class T>
@@ -565,7 +578,7 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
     // small scenes are a flat list; the others get both hierarchies
     const bool flat = n <= kFlatTris;
     const uint32_t wide_cap = n / 8 * 5 + 8;
-    if (n > 0 && (flat ? (r = s->alloc(&s->flat, n))
+    if (n > 0 && (flat ? (r = s->alloc(&s->flat, flat_pairs(n)))
                        : (r = s->alloc(&s->nodes, n - 1)) || (r = s->alloc(&s->leaf_box, 2 * size_t(n))) ||
                              (r = s->alloc(&s->wide, wide_cap)) || (r = s->alloc(&s->wtris, n)))) {
         delete s;

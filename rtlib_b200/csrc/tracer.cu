@@ -102,8 +102,8 @@ struct TracerDev {
     // A scene of at most kFlatTris triangles travels inside the kernel parameters: every lane
     // tests the same triangle at the same time, so its rows are read from the constant bank
     // with no load instruction, no load latency and no vector registers holding them.
-    uint32_t nflat;  // 0: trace through the BVH
-    BvhTri ftri[kFlatTris];
+    uint32_t nflat;  // pairs; 0: trace through the BVH
+    FlatPair ftri[flat_pairs(kFlatTris)];
 };
 
 // closest hit (ANY = false) or any hit (ANY = true) in (tmin, tmax): the scene's triangles from
@@ -116,6 +116,37 @@ __device__ __forceinline__ Hit trace(const TracerDev& T, float ox, float oy, flo
 }
 
 // ------------------------------------------------------------------ raygen (SimpleGuide.cu:48-81)
+// a path between two bounces
+struct PathState {
+    float3 org, dir, thr;
+    uint32_t rng, depth, flags;
+};
+__device__ __forceinline__ PathState raygen_path(const TracerDev& T, uint32_t p) {
+    const uint32_t x = p % T.width, y = p / T.width;
+    PathState s;
+    s.rng = T.seeds[p];
+    const float jx = rnd1(s.rng);
+    const float jy = rnd1(s.rng);
+    const float dx = (2.0f * ((float)x + jx) / (float)T.width) - 1.0f;
+    const float dy = (2.0f * ((float)y + jy) / (float)T.height) - 1.0f;
+    s.org = T.eye;
+    s.dir = unit3(dx * T.cu + dy * T.cv + T.cw);
+    s.thr = f3(1.0f, 1.0f, 1.0f);
+    s.depth = 0;
+    s.flags = HF_COUNT_EMITTED;
+    return s;
+}
+__device__ __forceinline__ PathState load_path(const TracerDev& T, uint32_t p) {
+    return PathState{T.org[p], T.dir[p], T.thr[p], T.rng[p], T.depth[p], T.hflags[p]};
+}
+__device__ __forceinline__ void store_path(const TracerDev& T, uint32_t p, const PathState& s) {
+    T.org[p] = s.org;
+    T.dir[p] = s.dir;
+    T.thr[p] = s.thr;
+    T.rng[p] = s.rng;
+    T.depth[p] = s.depth;
+    T.hflags[p] = s.flags;
+}
 __global__ void __launch_bounds__(kTB) k_raygen(TracerDev T) {
     grid_dependency_wait();  // the wave's kernels are dependent launches (see launch_wave)
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -123,19 +154,8 @@ __global__ void __launch_bounds__(kTB) k_raygen(TracerDev T) {
         T.qcount[1] = 0;
     }
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < T.npath; p += gridDim.x * blockDim.x) {
-        const uint32_t x = p % T.width, y = p / T.width;
-        uint32_t rng = T.seeds[p];
-        const float jx = rnd1(rng);
-        const float jy = rnd1(rng);
-        const float dx = (2.0f * ((float)x + jx) / (float)T.width) - 1.0f;
-        const float dy = (2.0f * ((float)y + jy) / (float)T.height) - 1.0f;
-        T.org[p] = T.eye;
-        T.dir[p] = unit3(dx * T.cu + dy * T.cv + T.cw);
-        T.thr[p] = f3(1.0f, 1.0f, 1.0f);
+        store_path(T, p, raygen_path(T, p));
         T.col[p] = f3(0.0f, 0.0f, 0.0f);
-        T.rng[p] = rng;
-        T.depth[p] = 0;
-        T.hflags[p] = HF_COUNT_EMITTED;
         T.queue[0][p] = p;
         if (T.adj_c) T.lrem[p] = T.adj_c[p];
     }
@@ -186,7 +206,8 @@ __device__ __forceinline__ LightSample sample_light(const TracerDev& T, float3 p
 // closest-hit program does, then the raygen bookkeeping (SimpleGuide.cu:85-114): bounce
 // radiance into the color (and, recording, into the per-bounce store from which k_commit forms
 // the trace-vertex radiance), termination, compaction of the survivors into the next queue.
-// Returns whether the path continues; *shadow tells whether a shadow ray was traced.
+// Returns whether the path continues (s is then its next state; s.rng is kept up to date in any
+// case); shadow tells whether a shadow ray was traced, L is the bounce's radiance.
 constexpr int kGuideNone = 0, kGuideTree = 1, kGuideGrid = 2, kAdjoint = 3, kGuideMlp = 4;
 
 // The adjoint replay (kAdjoint) runs the unguided path again from the same random numbers and
@@ -196,11 +217,12 @@ constexpr int kGuideNone = 0, kGuideTree = 1, kGuideGrid = 2, kAdjoint = 3, kGui
 // (its NEE term and everything after it); the albedo gradient is delta * lrem / albedo per
 // channel.  An emitter's gradient is delta * (the term's factor in front of its radiance).
 template <int G, bool FLAT>
-__device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, bool build, bool recording, bool& shadow) {
+__device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, PathState& s, bool build, bool recording,
+                                            bool& shadow, float3& L) {
     constexpr bool use_tree = G == kGuideTree, use_grid = G == kGuideGrid, adjoint = G == kAdjoint;
     constexpr bool use_mlp = G == kGuideMlp;
-    const float3 org = T.org[p], in_dir = T.dir[p], prev_thr = T.thr[p];
-    const uint32_t d = T.depth[p], prev_flags = T.hflags[p];
+    const float3 org = s.org, in_dir = s.dir, prev_thr = s.thr;
+    const uint32_t d = s.depth, prev_flags = s.flags;
     Hit h;
     if (use_mlp) {  // found by k_hit ahead of the mixture inference
         const float4 tuv = T.hit_tuv[p];
@@ -219,13 +241,12 @@ __device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, bool
     float3 nee_factor = f3(0.f, 0.f, 0.f);           // adjoint: NEE term / light radiance
     if (h.prim == 0xffffffffu) {
         // __miss__radiance (SimpleGuide.cu:202-219): the ray keeps its direction
-        const float3 L = prev_thr * T.bg;
+        L = prev_thr * T.bg;
         if (recording) T.b_rad[size_t(d) * T.npath + p] = L;
-        T.col[p] = T.col[p] + L;
         if (recording && d < kTV) T.v_flags[vi] = 0;
         return false;
     }
-    uint32_t rng = T.rng[p];
+    uint32_t& rng = s.rng;
     const TriFrame& tf = T.tri_frame[h.prim];
     const float3 fn = xyz(tf.fr[0]);
     float3 position = org + h.t * in_dir;
@@ -480,11 +501,10 @@ __device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, bool
     const bool emitted = dot3(in_dir, fn) < 0.0f && count_emitted;
     if (emitted) rad = prev_thr * m.emission;
     if (m.emission.x + m.emission.y + m.emission.z > 0.0f) flags |= HF_FINISH;
-    T.org[p] = position;
-    T.dir[p] = direction;
-    T.thr[p] = cur_thr;
-    T.hflags[p] = flags;
-    T.rng[p] = rng;
+    s.org = position;
+    s.dir = direction;
+    s.thr = cur_thr;
+    s.flags = flags;
     if (recording && d < kTV) {
         if (use_mlp) {
             T.v_pos[vi] = position;
@@ -513,7 +533,7 @@ __device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, bool
             T.v_wo[vi] = f3(-in_dir.x, -in_dir.y, -in_dir.z);
         }
     }
-    float3 L = rad;
+    L = rad;
     bool lit = false;
     if (pend) {
         shadow = true;
@@ -554,10 +574,9 @@ __device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, bool
         T.lrem[p] = lr;
     }
     if (recording) T.b_rad[size_t(d) * T.npath + p] = L;
-    T.col[p] = T.col[p] + L;
     const bool bad = any_nan3(direction) || any_nan3(cur_thr) || any_nan3(L);
     if (bad || (flags & HF_FINISH) || d >= T.max_depth - 1) return false;
-    T.depth[p] = d + 1;
+    s.depth = d + 1;
     if (use_mlp) {
         // the closest hit of the continuing ray, traced here rather than in a pass of its own,
         // so the network of the next bounce finds it waiting (k_hit serves the first bounce)
@@ -693,7 +712,12 @@ __global__ void __launch_bounds__(kTB, FLAT ? 8 : kBvhCtas) k_bounce(TracerDev T
         uint32_t p = 0;
         if (q < n) {
             p = T.queue[in][q];
-            keep = bounce_path<G, FLAT>(T, p, build, recording, shadow);
+            PathState s = load_path(T, p);
+            float3 L;
+            keep = bounce_path<G, FLAT>(T, p, s, build, recording, shadow, L);
+            T.col[p] = T.col[p] + L;
+            if (keep) store_path(T, p, s);
+            else T.rng[p] = s.rng;
         }
         const unsigned sh = __ballot_sync(0xffffffffu, shadow);
         if ((threadIdx.x & 31) == 0 && sh) atomicAdd(T.counters + 1, (unsigned long long)__popc(sh));
@@ -708,18 +732,58 @@ __global__ void __launch_bounds__(kTB, FLAT ? 8 : kBvhCtas) k_bounce(TracerDev T
     }
 }
 
-// ------------------------------------------------------------------ finish
 // Per path: FP64 accumulation and the seed write-back.
+__device__ __forceinline__ void finish_path(const TracerDev& T, uint32_t p, float3 c, uint32_t rng) {
+    double* a = T.accum + 3 * size_t(p);
+    a[0] += (double)c.x;
+    a[1] += (double)c.y;
+    a[2] += (double)c.z;
+    T.seeds[p] = rng;
+}
+
+// A whole path per thread: camera ray, bounces and accumulation in one kernel, the state in
+// registers.  Where the image is small the launches of a wave of bounces, each a latency-bound tail
+// on a part of the SMs, take most of its time; a path that ends leaves its lane idle instead of
+// being replaced.  Passes of one sample of the Cornell box, a launch per bounce -> here: 96 x 54
+// 130 -> 90 us, 256 x 256 150 -> 116 us, 400 x 400 208 -> 220 us.
+template <int G, bool FLAT>
+__global__ void __launch_bounds__(kTB, 8) k_path(TracerDev T) {
+    grid_dependency_wait();
+    const bool build = (T.flags & RTPG_TRACE_FLAG_BUILD) != 0;
+    const bool recording = (G == kGuideTree || G == kGuideGrid) && !(T.flags & RTPG_TRACE_FLAG_FINAL);
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    bool alive = p < T.npath;
+    PathState s;
+    float3 col = f3(0.0f, 0.0f, 0.0f);
+    if (alive) s = raygen_path(T, p);
+    uint32_t visits = 0, shadows = 0;
+    while (__any_sync(0xffffffffu, alive)) {
+        if (alive) {
+            bool shadow = false;
+            float3 L;
+            alive = bounce_path<G, FLAT>(T, p, s, build, recording, shadow, L);
+            col = col + L;
+            ++visits;
+            shadows += shadow;
+        }
+        __syncwarp();
+    }
+    visits = __reduce_add_sync(0xffffffffu, visits);
+    shadows = __reduce_add_sync(0xffffffffu, shadows);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(T.counters, (unsigned long long)visits);
+        atomicAdd(T.counters + 1, (unsigned long long)shadows);
+    }
+    if (p >= T.npath) return;
+    T.depth[p] = s.depth;  // for the commit
+    finish_path(T, p, col, s.rng);
+}
+
+// ------------------------------------------------------------------ finish
 __global__ void __launch_bounds__(kTB) k_finish(TracerDev T) {
     grid_dependency_wait();
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < T.npath; p += gridDim.x * blockDim.x) {
-        const float3 c = T.col[p];
-        double* a = T.accum + 3 * size_t(p);
-        a[0] += (double)c.x;
-        a[1] += (double)c.y;
-        a[2] += (double)c.z;
-        T.seeds[p] = T.rng[p];
-    }
+    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < T.npath; p += gridDim.x * blockDim.x)
+        finish_path(T, p, T.col[p], T.rng[p]);
 }
 
 // The commit of the trace vertices of recording waves (TraceVertexT::Commit,
@@ -960,10 +1024,9 @@ static void launch_bounce(const TracerDev& T, int g, cudaStream_t st, uint32_t b
         default: launch_bounce_of<kGuideNone>(T, g, st, b); break;
     }
 }
-// accumulation, then (recording waves of a guide) the commit of the trace vertices: two CTAs
-// of kCommitThreads per SM, each walking every vertex row over its share of the paths
-static void launch_finish(const TracerDev& T, int g, cudaStream_t st) {
-    (void)launch_dependent(k_finish, g, kTB, 0, st, T);
+// recording waves of a guide: the commit of the trace vertices, two CTAs of kCommitThreads per SM,
+// each walking every vertex row over its share of the paths
+static void launch_commit(const TracerDev& T, cudaStream_t st) {
     if (T.flags & RTPG_TRACE_FLAG_FINAL) return;
     const int gc = kSMs * 2;
     switch (guide_of(T.flags)) {
@@ -972,6 +1035,11 @@ static void launch_finish(const TracerDev& T, int g, cudaStream_t st) {
         case kGuideMlp: (void)launch_dependent(k_commit<kGuideMlp>, gc, kCommitThreads, 0, st, T); break;
         default: break;
     }
+}
+// accumulation and the commit
+static void launch_finish(const TracerDev& T, int g, cudaStream_t st) {
+    (void)launch_dependent(k_finish, g, kTB, 0, st, T);
+    launch_commit(T, st);
 }
 
 // One wave with CUDA events around every kernel group; synchronises and accumulates the
@@ -1009,9 +1077,29 @@ static int timed_wave(rtpg_tracer* h, cudaStream_t st) {
     return RTPG_OK;
 }
 
+// Whether waves of this tracer run a path per thread (k_path) instead of a launch per bounce: while
+// the paths fit seven of the eight CTAs an SM holds.  Guided Cornell passes (63 spp): 65 k paths 12.7
+// -> 10.5 ms, 144 k 16.4 -> 16.8 ms; hash-grid passes over 100 k triangles: 14 k paths 18.2 -> 14.0
+// ms, 130 k 29.2 -> 27.1 ms.  The learned guide needs its network between bounces.
+constexpr uint32_t kWholePaths = kSMs * 7 * kTB;
+static bool whole_paths(const TracerDev& T) { return T.npath <= kWholePaths && guide_of(T.flags) != kGuideMlp; }
+template <int G>
+static void launch_path_of(const TracerDev& T, cudaStream_t st) {
+    if (T.nflat) (void)launch_dependent(k_path<G, true>, bounce_grid(T), kTB, 0, st, T);
+    else (void)launch_dependent(k_path<G, false>, bounce_grid(T), kTB, 0, st, T);
+}
 static void launch_wave(rtpg_tracer* h, cudaStream_t st) {
     TracerDev& T = h->dev;
     const int g = kSMs * 8;
+    if (whole_paths(T)) {
+        switch (guide_of(T.flags)) {
+            case kGuideTree: launch_path_of<kGuideTree>(T, st); break;
+            case kGuideGrid: launch_path_of<kGuideGrid>(T, st); break;
+            default: launch_path_of<kGuideNone>(T, st); break;
+        }
+        launch_commit(T, st);
+        return;
+    }
     (void)launch_dependent(k_raygen, g, kTB, 0, st, T);
     for (uint32_t b = 0; b < T.max_depth; ++b) launch_bounce(T, bounce_grid(T), st, b);
     launch_finish(T, g, st);
@@ -1039,12 +1127,12 @@ int rtpg_tracer_create(rtpg_scene* scene, const float* tri_vertices, const uint3
     T.nflat = 0;
     if (T.scene.flat && T.scene.ntris <= kFlatTris) {
         // the scene's triangles (scene order) into the kernel parameters
-        const cudaError_t e = cudaMemcpy(T.ftri, T.scene.flat, sizeof(BvhTri) * T.scene.ntris, cudaMemcpyDeviceToHost);
+        const cudaError_t e = cudaMemcpy(T.ftri, T.scene.flat, sizeof(FlatPair) * flat_pairs(T.scene.ntris), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) {
             delete h;
             return fail(RTPG_ECUDA, "rtpg_tracer_create: %s", cudaGetErrorString(e));
         }
-        T.nflat = T.scene.ntris;
+        T.nflat = flat_pairs(T.scene.ntris);
     }
     T.tri_v = tri_vertices;
     T.tri_mat = tri_material;

@@ -181,3 +181,21 @@ def test_hierarchy_of_coincident_triangles(cuda):
     t, p = torch.empty(4097, device=cuda), torch.empty(4097, dtype=torch.int32, device=cuda)
     sc.intersect(org, d, out_t=t, out_prim=p)
     assert (t == 1.0).all() and (p == p[0]).all()
+
+
+@pytest.mark.parametrize("w,h,spp", [(1, 1, 3), (33, 7, 2), (148 * 7, 128, 1), (148 * 7, 129, 1)])
+def test_whole_path_waves_equal_bounce_waves(cuda, w, h, spp):
+    """Images, path depths and counters on both sides of the path-per-thread limit (7 CTAs of 128 per
+    SM): the same as a launch per bounce gives."""
+    from rtlib_b200 import scenes
+    from rtlib_b200.tracer import FLAG_NEE, Tracer
+    sc = scenes.cornell_box(w, h)
+    tr = Tracer(sc, cuda, max_depth=6, width=w, height=h, seed=3)
+    tr.render(spp, FLAG_NEE)
+    img, depth, cnt = tr.image64().cpu().numpy(), tr.path_depths().cpu().numpy(), tr.counters()
+    ref = Tracer(sc, cuda, max_depth=6, width=w, height=h, seed=3)
+    ref.set_timing(True)  # measures the groups of a wave: always a launch per bounce
+    ref.render(spp, FLAG_NEE)
+    np.testing.assert_array_equal(img, ref.image64().cpu().numpy())
+    np.testing.assert_array_equal(depth, ref.path_depths().cpu().numpy())
+    assert cnt == ref.counters()
