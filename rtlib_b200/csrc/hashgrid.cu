@@ -10,12 +10,15 @@
 //
 // RTLib inserts with atomicCAS, so which key wins which slot depends on thread timing.  Here
 // a batch insert reproduces the slots of inserting the batch sequentially in index order:
-// new keys are sorted (stable radix sort), each distinct key takes its first occurrence, the
-// keys of a bucket are ranked by first occurrence and appended after the bucket's occupied
-// prefix.  Lookups (FindFromPrv) read the previous snapshot and stop at the first empty slot.
+// each distinct new key takes its first occurrence, the keys of a bucket are ranked by first
+// occurrence and appended after the bucket's occupied prefix.  Usually the distinct keys come from
+// a temporary hash table and the ranks from a list per bucket (k_hash_stage and on); batches of
+// far more points than slots are sorted instead (k_hash_prepare and on).  Lookups (FindFromPrv) read the previous snapshot and stop at the first empty slot.
+#include <algorithm>
 #include <cub/cub.cuh>
 #include <mutex>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -35,14 +38,8 @@ __global__ void k_hash_prepare(HashGridDev g, int64_t base, int64_t n, const flo
         uint32_t b;
         const unsigned long long key = hash_key(g, pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], b);
         if (out_key) out_key[i] = key;
-        const unsigned long long* row = g.cur + size_t(b) * kHashBlock;
-        uint32_t k = 0;
-        bool found = false;
-        for (; k < kHashBlock; ++k) {
-            const unsigned long long v = row[k];
-            if (v == 0ull) break;
-            if (v == key) { found = true; break; }
-        }
+        bool found;
+        const uint32_t k = hash_probe(g.cur + size_t(b) * kHashBlock, key, found);
         bucket_of[j] = b;
         occ_of[j] = (uint8_t)k;
         if (found) {
@@ -111,7 +108,122 @@ __global__ void k_hash_scatter(int64_t base, int64_t n, const unsigned long long
     }
 }
 
-__global__ void k_hash_lookup(HashGridDev g, int64_t n, const float* __restrict__ pos, uint32_t* __restrict__ out_slot) {
+// ------------------------------------------------------------------ insert by hashing
+// Scratch of a batch of up to `cap` points.  table, first and head are one run of bytes, set to
+// all ones before the batch: no key is UINT64_MAX.
+struct StageDev {
+    unsigned long long* table;  // size entries: the batch's distinct new keys, linear probing
+    uint32_t* first;            // per entry: its first point
+    uint32_t* head;             // per bucket: a list of its distinct new keys' first points
+    uint32_t* slot;             // per entry: the slot it is given
+    uint32_t *entry, *next, *bucket;  // per point: its entry (kFull: key known), list link, bucket
+    uint8_t* occ;               // per point: occupied slots of its bucket
+    uint32_t size;              // a power of two, at least 1.5 points
+};
+static uint32_t stage_size(uint32_t points) {
+    uint32_t h = 32;
+    while (h < points + points / 2) h <<= 1;
+    return h;
+}
+static size_t stage_ones(uint32_t size, uint32_t nbuckets) { return size_t(size) * 12 + size_t(nbuckets) * 4; }
+static size_t stage_bytes(uint32_t cap, uint32_t nbuckets) {
+    return ((stage_ones(stage_size(cap), nbuckets) + 255) & ~size_t(255)) + size_t(stage_size(cap)) * 4 + size_t(cap) * 13;
+}
+static StageDev stage_view(unsigned char* p, uint32_t points, uint32_t nbuckets) {
+    StageDev s;
+    s.size = stage_size(points);
+    s.table = reinterpret_cast<unsigned long long*>(p);
+    s.first = reinterpret_cast<uint32_t*>(s.table + s.size);
+    s.head = s.first + s.size;
+    s.slot = reinterpret_cast<uint32_t*>(p + ((stage_ones(s.size, nbuckets) + 255) & ~size_t(255)));
+    s.entry = s.slot + s.size;
+    s.next = s.entry + points;
+    s.bucket = s.next + points;
+    s.occ = reinterpret_cast<uint8_t*>(s.bucket + points);
+    return s;
+}
+
+// Known keys get their slot; the others are entered in the temporary table with their least point.
+__global__ void __launch_bounds__(256) k_hash_stage(HashGridDev g, StageDev s, int64_t base, uint32_t n,
+                                                    const float* __restrict__ pos, uint32_t* __restrict__ out_slot,
+                                                    unsigned long long* __restrict__ out_key) {
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        const int64_t i = base + j;
+        uint32_t b;
+        const unsigned long long key = hash_key(g, pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], b);
+        if (out_key) out_key[i] = key;
+        bool found;
+        const uint32_t k = hash_probe(g.cur + size_t(b) * kHashBlock, key, found);
+        uint32_t e = kFull;
+        if (found) {
+            out_slot[i] = b * kHashBlock + k;
+        } else {
+            e = (uint32_t)(mix64(key) >> 32) & (s.size - 1);
+            for (;; e = (e + 1) & (s.size - 1)) {  // fewer keys than entries: ends
+                unsigned long long v = *reinterpret_cast<volatile unsigned long long*>(s.table + e);
+                if (v == ~0ull) v = atomicCAS(s.table + e, ~0ull, key);
+                if (v == ~0ull || v == key) break;
+            }
+            if (*reinterpret_cast<volatile uint32_t*>(s.first + e) > j) atomicMin(s.first + e, j);
+            s.bucket[j] = b;
+            s.occ[j] = (uint8_t)k;
+        }
+        s.entry[j] = e;
+    }
+}
+// the first point of every entry joins its bucket's list
+__global__ void __launch_bounds__(256) k_hash_chain(StageDev s, uint32_t n) {
+    grid_dependency_wait();
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        const uint32_t e = s.entry[j];
+        if (e != kFull && s.first[e] == j) s.next[j] = atomicExch(s.head + s.bucket[j], j);
+    }
+}
+// its rank among them gives its slot
+__global__ void __launch_bounds__(256) k_hash_rank(HashGridDev g, StageDev s, uint32_t n) {
+    grid_dependency_wait();
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        const uint32_t e = s.entry[j];
+        if (e == kFull || s.first[e] != j) continue;
+        const uint32_t b = s.bucket[j];
+        uint32_t at = s.occ[j];
+        for (uint32_t k = s.head[b]; k != 0xffffffffu && at < kHashBlock; k = s.next[k]) at += k < j;
+        if (at < kHashBlock) {
+            const uint32_t slot = b * kHashBlock + at;
+            g.cur[slot] = s.table[e];
+            s.slot[e] = slot;
+        } else {
+            s.slot[e] = kFull;
+            atomicOr(g.status, RTPG_STATUS_HASH_FULL);
+        }
+    }
+}
+__global__ void __launch_bounds__(256) k_hash_give(StageDev s, int64_t base, uint32_t n, uint32_t* __restrict__ out_slot) {
+    grid_dependency_wait();
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+        const uint32_t e = s.entry[j];
+        if (e != kFull) out_slot[base + j] = s.slot[e];
+    }
+}
+// One batch.  A bucket's list is as long as the distinct new keys that fall into it, walked once per
+// key: with at most kStagePerSlot points per slot that is at most 128 on average.  2^19 points (373 k
+// cells) into 2^20 slots: 253 us with two 64-bit radix sorts, 48 us here.
+constexpr uint32_t kStagePerSlot = 4;
+static bool stage_fits(const HashGridDev& g, int64_t n) { return (uint64_t)n <= (uint64_t)g.nslots * kStagePerSlot; }
+static int stage_insert(const HashGridDev& g, unsigned char* scratch, int64_t base, uint32_t n, const float* pos,
+                        uint32_t* out_slot, uint64_t* out_key, cudaStream_t st) {
+    const StageDev s = stage_view(scratch, n, g.nbuckets);
+    const int grid = grid_for(n, 256, 8);
+    RTPG_CUDA(cudaMemsetAsync(s.table, 0xff, stage_ones(s.size, g.nbuckets), st));
+    k_hash_stage<<<grid, 256, 0, st>>>(g, s, base, n, pos, out_slot, reinterpret_cast<unsigned long long*>(out_key));
+    RTPG_LAUNCH_CHECK();
+    RTPG_CUDA(launch_dependent(k_hash_chain, grid, 256, 0, st, s, n));
+    RTPG_CUDA(launch_dependent(k_hash_rank, grid, 256, 0, st, g, s, n));
+    RTPG_CUDA(launch_dependent(k_hash_give, grid, 256, 0, st, s, base, n, out_slot));
+    return RTPG_OK;
+}
+
+__global__ void __launch_bounds__(256) k_hash_lookup(HashGridDev g, int64_t n, const float* __restrict__ pos, uint32_t* __restrict__ out_slot) {
     for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
         out_slot[i] = hash_find_prv(g, pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]);
 }
@@ -144,8 +256,9 @@ struct rtpg_hashgrid {
     uint32_t *sval[2] = {nullptr, nullptr}, *cval[2] = {nullptr, nullptr};
     uint32_t *bucket_of = nullptr, *run_slot = nullptr;
     uint8_t* occ_of = nullptr;
-    void* temp = nullptr;
+    uint8_t* temp = nullptr;
     size_t temp_bytes = 0;
+    unsigned char* stage = nullptr;  // the scratch run: either the arrays above or the staging's
     std::vector<void*> allocs;
     size_t bytes = 0;
     template <class T>
@@ -194,21 +307,38 @@ int rtpg_hashgrid_create(const float* aabb_min, const float* aabb_max, const uin
     h->max_batch = max_batch ? max_batch : (1u << 22);
     const size_t B = h->max_batch;
     int r;
-    if ((r = h->alloc(&g.cur, num_slots)) || (r = h->alloc(&g.prv, num_slots)) || (r = h->alloc(&g.status, 1)) ||
-        (r = h->alloc(&h->skey[0], B)) || (r = h->alloc(&h->skey[1], B)) || (r = h->alloc(&h->comp[0], B)) ||
-        (r = h->alloc(&h->comp[1], B)) || (r = h->alloc(&h->sval[0], B)) || (r = h->alloc(&h->sval[1], B)) ||
-        (r = h->alloc(&h->cval[0], B)) || (r = h->alloc(&h->cval[1], B)) || (r = h->alloc(&h->bucket_of, B)) ||
-        (r = h->alloc(&h->run_slot, B)) || (r = h->alloc(&h->occ_of, B))) {
-        delete h;
-        return r;
-    }
-    cub::DoubleBuffer<unsigned long long> dk(h->skey[0], h->skey[1]);
-    cub::DoubleBuffer<uint32_t> dv(h->sval[0], h->sval[1]);
+    // one scratch run serves both ways of inserting: the sort's arrays, or the staging's
+    cub::DoubleBuffer<unsigned long long> dk(nullptr, nullptr);
+    cub::DoubleBuffer<uint32_t> dv(nullptr, nullptr);
     size_t tb = 0;
     cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, dv, (int)B);
-    if (e != cudaSuccess || (r = h->alloc(reinterpret_cast<uint8_t**>(&h->temp), tb))) {
+    if (e != cudaSuccess) {
         delete h;
-        return e != cudaSuccess ? fail(RTPG_ECUDA, "cub temp size: %s", cudaGetErrorString(e)) : r;
+        return fail(RTPG_ECUDA, "cub temp size: %s", cudaGetErrorString(e));
+    }
+    // a staged batch may be as large as max_batch
+    const uint32_t stage_cap = (uint32_t)std::min<uint64_t>(B, (uint64_t)num_slots * kStagePerSlot);
+    for (int pass = 0; pass < 2; ++pass) {  // sizes, then places
+        size_t at = 0;
+        auto take = [&](auto** p, size_t count) {
+            if (pass) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(h->stage + at);
+            at += (count * sizeof(**p) + 255) & ~size_t(255);
+        };
+        for (int k = 0; k < 2; ++k) {
+            take(&h->skey[k], B);
+            take(&h->comp[k], B);
+            take(&h->sval[k], B);
+            take(&h->cval[k], B);
+        }
+        take(&h->bucket_of, B);
+        take(&h->run_slot, B);
+        take(&h->occ_of, B);
+        take(&h->temp, tb);
+        if (!pass && ((r = h->alloc(&g.cur, num_slots)) || (r = h->alloc(&g.prv, num_slots)) || (r = h->alloc(&g.status, 1)) ||
+                      (r = h->alloc(&h->stage, std::max(at, stage_bytes(stage_cap, g.nbuckets)))))) {
+            delete h;
+            return r;
+        }
     }
     h->temp_bytes = tb;
     if (cudaMemset(g.cur, 0, num_slots * 8ull) != cudaSuccess || cudaMemset(g.prv, 0, num_slots * 8ull) != cudaSuccess ||
@@ -252,6 +382,11 @@ int rtpg_hashgrid_insert(rtpg_hashgrid* h, int64_t n, const float* pos, uint32_t
     // chunks are inserted in order, which keeps the sequential-insertion semantics
     for (int64_t base = 0; base < n; base += h->max_batch) {
         const int64_t m = std::min<int64_t>(h->max_batch, n - base);
+        if (stage_fits(h->dev, m)) {
+            const int r = stage_insert(h->dev, h->stage, base, (uint32_t)m, pos, out_slot, out_key, st);
+            if (r) return r;
+            continue;
+        }
         const int g = grid_for(m, 256, 8);
         k_hash_prepare<<<g, 256, 0, st>>>(h->dev, base, m, pos, h->skey[0], h->sval[0], h->bucket_of, h->occ_of,
                                            out_slot, reinterpret_cast<unsigned long long*>(out_key));
@@ -425,6 +560,9 @@ extern "C" int rtpg_hashgrid_insert_noalloc(const float* aabb_min, const float* 
     auto* run_slot = reinterpret_cast<uint32_t*>(s + kNA_run);
     auto* occ_of = reinterpret_cast<uint8_t*>(s + kNA_occ);
     void* temp = s + kNA_temp;
+    // the staging scratch lies where the sort's would (the status word apart)
+    if (stage_fits(g, n) && stage_bytes((uint32_t)n, g.nbuckets) <= kNA_status)
+        return stage_insert(g, s, 0, (uint32_t)n, pos, out_slot, nullptr, as_stream(stream));
     // every scratch word read below is written earlier in the same call, so nothing left
     // by a previous call needs clearing
     cudaStream_t st = as_stream(stream);

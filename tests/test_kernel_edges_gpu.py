@@ -220,3 +220,48 @@ def test_emitter_gradients_add_up(cuda, grid, w, h):
     got = (g.double().cpu().numpy() * np.asarray(sc["light_emission"], np.float64).reshape(-1, 3)).sum(0)
     want = (img * d_img.double()).sum(dim=(0, 1)).cpu().numpy()
     np.testing.assert_allclose(got, want, rtol=1e-4)
+
+
+@pytest.mark.parametrize("n,slots", [(1, 32), (128, 32), (129, 32), (5000, 1024), (4096, 1024), (4097, 1024), (70000, 1 << 16),
+                                     (3000, 96), (300, 96)])
+def test_hashgrid_insert_routes(cuda, oracle, n, slots):
+    """Batches staged in the temporary table (at most four points per slot) and sorted ones give the
+    slots of sequential insertion: overfull buckets, repeated cells, a table that is half full, a
+    number of buckets that is no power of two."""
+    from rtlib_b200.hashgrid import KEY_MORTON, HashGrid
+    rng = np.random.default_rng(n)
+    mn, mx, bounds = np.zeros(3, np.float32), np.full(3, 5, np.float32), [300, 40, 2000]
+    hg = HashGrid(mn, mx, bounds, slots, keying=KEY_MORTON)
+    cur = np.zeros(slots, np.uint64)
+    import torch
+    full = False
+    for batch in range(3):
+        pos = (rng.random((n, 3), dtype=np.float32) * 6 - 0.5).astype(np.float32)
+        pos[n // 2:] = pos[rng.integers(0, n // 2 + 1, n - n // 2)]
+        out = torch.empty(n, dtype=torch.int32, device=cuda)
+        hg.insert(_t(pos, cuda), out)
+        want, _ = oracle.mhash_insert(pos, mn, mx - mn, bounds, slots, cur)
+        full |= bool((want == 0xFFFFFFFF).any())
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), want)
+        np.testing.assert_array_equal(hg.export(), cur)
+    assert bool(hg.status() & 0x10) == full
+
+
+@pytest.mark.parametrize("offset", [0, 1, 3])
+def test_hashgrid_noalloc_table_alignment(cuda, oracle, offset):
+    """A caller's table need not lie on a 32-byte boundary."""
+    import torch
+    from rtlib_b200.hashgrid import KEY_MORTON, insert_noalloc
+    rng = np.random.default_rng(offset)
+    mn, mx, bounds, slots, n = np.zeros(3, np.float32), np.ones(3, np.float32), [64, 64, 64], 4096, 2500
+    store = torch.zeros(slots + 8, dtype=torch.int64, device=cuda)
+    table = store[offset:offset + slots]
+    cur = np.zeros(slots, np.uint64)
+    for _ in range(2):
+        pos = rng.random((n, 3), dtype=np.float32)
+        out = torch.empty(n, dtype=torch.int32, device=cuda)
+        insert_noalloc(mn, mx, bounds, table, _t(pos, cuda), out, keying=KEY_MORTON)
+        want, _ = oracle.mhash_insert(pos, mn, mx - mn, bounds, slots, cur)
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), want)
+    np.testing.assert_array_equal(table.cpu().numpy().view(np.uint64), cur)
+    assert not store[:offset].any() and not store[offset + slots:].any()
