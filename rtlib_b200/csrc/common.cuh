@@ -146,6 +146,10 @@ int scan_exclusive_u32x2(const uint32_t* in0, uint32_t* out0, uint32_t* total0, 
 // launched the ordinary way the wait returns at once.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// lets the next dependent launch of the stream be scheduled from here on (it still waits for this
+// grid in grid_dependency_wait); without it that happens when this grid ends
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                     Args... args) {

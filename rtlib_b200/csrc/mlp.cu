@@ -30,95 +30,89 @@ __device__ __forceinline__ void store_row(float* dst, const float* v) {
 }
 
 // out_raw: 48 floats per sample (the network output); out_lobes: 40 floats per sample, lobe k
-// = (mu xyz, kappa, weight).  Either may be null.
-__global__ void __launch_bounds__(kMlpThreads) k_mlp_eval(MlpDev P, int64_t n, const float* __restrict__ pos,
-                                                         const float* __restrict__ nrm, const float* __restrict__ wo,
-                                                         float* __restrict__ out_raw, float* __restrict__ out_lobes) {
+// = (mu xyz, kappa, weight).  Either may be null.  Bound by the phases of the four tiles an SM holds
+// (issue slots 58 % busy).  2^20 samples: 148.6 us with one thread per sample, 136.9 with two and the
+// next tile's inputs fetched ahead; eight tiles per SM sharing weights, one thread per sample: 133,
+// but 6 % slower at 10^5 samples.
+__global__ void __launch_bounds__(kMlpThreads, 4) k_mlp_eval(MlpDev P, int64_t n, const float* __restrict__ pos,
+                                                            const float* __restrict__ nrm, const float* __restrict__ wo,
+                                                            float* __restrict__ out_raw, float* __restrict__ out_lobes) {
     extern __shared__ __align__(128) uint8_t sm[];
-    __nv_bfloat16* ws = reinterpret_cast<__nv_bfloat16*>(sm);
-    __nv_bfloat16* x0 = reinterpret_cast<__nv_bfloat16*>(sm + kSmemW);
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kSmemW + kSmemX);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kSmemW + kSmemX + 8);
-    const int t = threadIdx.x;
-    if (t < 32) tmem_alloc(tslot, kEvalCols);
-    if (t == 0) mbar_init(mbar, 1);
-    load_weights(ws, P.wq);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tslot;
-    const uint32_t sw = smem_u32(ws);
-    uint32_t phase = 0;
+    EvalCta c = eval_begin(sm, P.wq);
     bool ok = true;
-    for (int64_t base = int64_t(blockIdx.x) * kMlpTile; base < n; base += int64_t(gridDim.x) * kMlpTile) {
-        const int64_t i = base + t;
-        float f[kMlpIn];
-        if (i < n) {
-            mlp_features(f3(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]), f3(nrm[3 * i], nrm[3 * i + 1], nrm[3 * i + 2]),
-                         f3(wo[3 * i], wo[3 * i + 1], wo[3 * i + 2]), P.mn, P.inv_ext, f);
-        } else {
-#pragma unroll
-            for (int k = 0; k < kMlpIn; ++k) f[k] = 0.0f;
+    const bool hi = threadIdx.x >= kMlpTile;
+    const int64_t stride = int64_t(gridDim.x) * kMlpTile;
+    int64_t i = int64_t(blockIdx.x) * kMlpTile + threadIdx.x % kMlpTile;
+    float3 x = f3(0.f, 0.f, 0.f), nv = x, wv = x;
+    auto fetch = [&](int64_t k) {
+        if (k >= n) return;
+        x = f3(pos[3 * k], pos[3 * k + 1], pos[3 * k + 2]);
+        if (!hi) return;  // the upper half holds these features
+        nv = f3(nrm[3 * k], nrm[3 * k + 1], nrm[3 * k + 2]);
+        wv = f3(wo[3 * k], wo[3 * k + 1], wo[3 * k + 2]);
+    };
+    fetch(i);
+    for (int64_t base = int64_t(blockIdx.x) * kMlpTile; base < n; base += stride, i += stride) {
+        store_features(c.x0, i < n, x, nv, wv, P.mn, P.inv_ext);
+        fetch(i + stride);  // the next tile's inputs arrive while this one is evaluated
+        if (!mlp_forward_tile(P, c.d, c.sw, c.x0, c.mbar, c.phase, ok)) break;  // uniform: issue nothing more
+        // half of a sample's row (192 or 160 bytes) in 16-byte stores when the array allows it; the
+        // loads from tensor memory take the whole warp
+        if (out_raw) {
+            float q[kMlpOut / 2];
+            ld_row<kMlpOut / 2>(c.d, hi ? kMlpOut / 2 : 0, q);
+            if (i < n && ok) store_row<kMlpOut / 2>(out_raw + i * kMlpOut + (hi ? kMlpOut / 2 : 0), q);
         }
-        store_features(x0, t, f);
-        float o[kMlpOut];
-        if (!mlp_forward_tile(P, tmem, sw, x0, mbar, phase, o)) {
-            ok = false;  // uniform over the CTA: issue nothing more
-            break;
-        }
-        if (i < n) {
-            // a sample's row (192 or 160 bytes) in 16-byte stores when the array allows it
-            if (out_raw) store_row<kMlpOut>(out_raw + i * kMlpOut, o);
-            if (out_lobes) {
-                VmfLobe L[kMlpLobes];
-                mlp_head(o, L);
-                float q[40];
+        if (out_lobes) {
+            float o[kMlpOut];
+            ld_row<kMlpOut>(c.d, 0, o);
+            if (i < n && ok) {
+                VmfLobe L[kMlpLobes / 2];
+                mlp_head_half(o, hi, L);
+                float q[20];
 #pragma unroll
-                for (int k = 0; k < kMlpLobes; ++k) {
+                for (int k = 0; k < kMlpLobes / 2; ++k) {
                     q[5 * k] = L[k].mu.x; q[5 * k + 1] = L[k].mu.y; q[5 * k + 2] = L[k].mu.z;
                     q[5 * k + 3] = L[k].kappa; q[5 * k + 4] = L[k].weight;
                 }
-                store_row<40>(out_lobes + i * 40, q);
+                store_row<20>(out_lobes + i * 40 + (hi ? 20 : 0), q);
             }
         }
     }
-    if (!ok) {
-        if (t == 0) atomicOr(P.status, RTPG_STATUS_TIMEOUT);
-        mma_drain(mbar, phase, P.poll_limit);
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (t < 32) tmem_dealloc(tmem, kEvalCols);
+    eval_end(c, ok, P.poll_limit, P.status);
 }
 
 // ------------------------------------------------------------------ training
 // d(loss)/d(raw outputs) of one record: loss = -w log q(wi) (scaled by inv_wsum), q the mixture
-// of mlp_head.  Returns -log q.
-__device__ __forceinline__ float head_grad(const float* o, float3 wi, float scale, float* g) {
-    VmfLobe L[kMlpLobes];
-    mlp_head(o, L);
-    float fk[kMlpLobes], q = 0.0f;
+// of mlp_head.  Each of the record's two threads forms its half of the lobes; q is the sum of both
+// halves, exchanged through s_q.  The thread's 20 gradients go to g; returns -log q.
+__device__ __forceinline__ float head_grad(const float* o, bool hi, float3 wi, float scale, float* s_q, float* g) {
+    VmfLobe L[kMlpLobes / 2];
+    mlp_head_half(o, hi, L);
+    float fk[kMlpLobes / 2], q = 0.0f;
 #pragma unroll
-    for (int k = 0; k < kMlpLobes; ++k) {
+    for (int k = 0; k < kMlpLobes / 2; ++k) {
         fk[k] = vmf_pdf(L[k], wi);
         q += L[k].weight * fk[k];
     }
-    q = fmaxf(q, 1e-30f);
+    s_q[threadIdx.x] = q;
+    __syncthreads();
+    const int row = threadIdx.x & (kMlpTile - 1);
+    q = fmaxf(s_q[row] + s_q[row + kMlpTile], 1e-30f);
 #pragma unroll
-    for (int c = 0; c < kMlpOut; ++c) g[c] = 0.0f;
-#pragma unroll
-    for (int k = 0; k < kMlpLobes; ++k) {
+    for (int k = 0; k < kMlpLobes / 2; ++k) {
         const float r = L[k].weight * fk[k] / q;  // responsibility
-        const float3 m = f3(o[5 * k], o[5 * k + 1], o[5 * k + 2]);
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = hi ? o[5 * (k + 4) + j] : o[5 * k + j];
+        const float3 m = f3(v[0], v[1], v[2]);
         const float len = fmaxf(sqrtf(dot3(m, m)), 1e-12f);
         const float kap = L[k].kappa, mw = dot3(L[k].mu, wi);
         // d log q / d m = r kappa (wi - (mu.wi) mu) / |m|
         const float3 gm = (wi - L[k].mu * mw) * (r * kap / len);
         const float e = __expf(-2.0f * kap);
         const float dlk = 1.0f / kap - 2.0f * e / (1.0f - e) + (mw - 1.0f);
-        const float s = o[5 * k + 3];
-        const float gs = (s > kLogKappaMin && s < kLogKappaMax) ? r * kap * dlk : 0.0f;
+        const float gs = (v[3] > kLogKappaMin && v[3] < kLogKappaMax) ? r * kap * dlk : 0.0f;
         g[5 * k] = -scale * gm.x;
         g[5 * k + 1] = -scale * gm.y;
         g[5 * k + 2] = -scale * gm.z;
@@ -130,6 +124,12 @@ __device__ __forceinline__ float head_grad(const float* o, float3 wi, float scal
 
 // One pass over n records: forward, loss gradient, backward; dW of all layers accumulate in
 // TMEM across the CTA's tiles and are added to grads (fp32, [in][out] per layer) at the end.
+// A minibatch gives each CTA one tile, so its time is that tile's chain of phases: features, eight
+// dependent MMA phases with an epilogue each, the gradient flush.  Launched as a dependent of the
+// previous step's Adam it forms the first tile's features, which do not depend on the weights, while
+// that still runs (records and wsum are ready before the first launch of a call).  16 steps of 16384
+// records: 574 us with 128 threads per tile and a memset, a weight sum and an Adam launched one after
+// the other around it, 320 us now.
 __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t n, Records R, const float* wsum,
                                                             float* __restrict__ grads, float* __restrict__ loss_sum) {
     extern __shared__ __align__(128) uint8_t sm[];
@@ -140,140 +140,150 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t 
     __nv_bfloat16* dy = reinterpret_cast<__nv_bfloat16*>(sm + kSmemW + kSmemX + 3 * kSmemH);
     uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kSmemW + kSmemX + 4 * kSmemH);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kSmemW + kSmemX + 4 * kSmemH + 8);
-    const int t = threadIdx.x;
+    __shared__ float s_q[kMlpThreads];
+    grid_launch_dependents();
+    const int t = threadIdx.x, row = t & (kMlpTile - 1);
+    const bool hi = t >= kMlpTile;
     if (t < 32) tmem_alloc(tslot, kTrainCols);
     if (t == 0) mbar_init(mbar, 1);
-    load_weights(ws, P.wq);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tslot;
     const uint32_t sw = smem_u32(ws), sx = smem_u32(x0), sdy = smem_u32(dy);
     const uint32_t sh[3] = {smem_u32(hs[0]), smem_u32(hs[1]), smem_u32(hs[2])};
     const float scale = (wsum && *wsum > 0.0f) ? 1.0f / *wsum : 0.0f;
     // record weights are Monte Carlo estimates with a heavy tail: clamp at kWeightClamp times
     // their mean so that single rare paths do not dominate a step
     const float wmax = (wsum && n > 0) ? kWeightClamp * (*wsum / (float)n) : 0.0f;
-    uint32_t phase = 0;
+    uint32_t phase = 0, tmem = 0;
     bool ok = true, first = true;
     float lsum = 0.0f;
-    // commit the MMAs thread 0 issued and wait for them; false (uniform over the CTA) when the
-    // wait gave up, after which nothing more is issued
-    auto sync_mma = [&]() -> bool {
+    auto commit_wait = [&] {
         if (t == 0 && !P.skip_mma) umma_commit(mbar);
-        return mma_complete(mbar, phase, P.poll_limit);
+        ok = mma_complete(mbar, phase, P.poll_limit);
     };
     for (int64_t base = int64_t(blockIdx.x) * kMlpTile; base < n; base += int64_t(gridDim.x) * kMlpTile) {
-        const int64_t i = base + t;
-        float f[kMlpIn];
-        float3 wi = f3(0.f, 0.f, 1.f);
+        const int64_t i = base + row;
+        const bool live = i < n;
+        float3 x = f3(0.f, 0.f, 0.f), nv = x, wv = x, wi = f3(0.f, 0.f, 1.f);
         float w = 0.0f;
-        if (i < n) {
-            mlp_features(f3(R.pos[3 * i], R.pos[3 * i + 1], R.pos[3 * i + 2]),
-                         f3(R.nrm[3 * i], R.nrm[3 * i + 1], R.nrm[3 * i + 2]),
-                         f3(R.wo[3 * i], R.wo[3 * i + 1], R.wo[3 * i + 2]), P.mn, P.inv_ext, f);
+        if (live) {
+            x = f3(R.pos[3 * i], R.pos[3 * i + 1], R.pos[3 * i + 2]);
+            nv = f3(R.nrm[3 * i], R.nrm[3 * i + 1], R.nrm[3 * i + 2]);
+            wv = f3(R.wo[3 * i], R.wo[3 * i + 1], R.wo[3 * i + 2]);
             wi = f3(R.wi[3 * i], R.wi[3 * i + 1], R.wi[3 * i + 2]);
             w = fminf(fmaxf(R.w[i], 0.0f), wmax);
-        } else {
-#pragma unroll
-            for (int k = 0; k < kMlpIn; ++k) f[k] = 0.0f;
         }
-        store_features(x0, t, f);
+        store_features(x0, live, x, nv, wv, P.mn, P.inv_ext);
+        if (first) {
+            grid_dependency_wait();  // the weights
+            load_weights(ws, P.wq);
+        }
         // forward, keeping H1..H3
-        for (int l = 0; l < 4; ++l) {
-            mma_barrier();
+        bool go = true;
+        for (int l = 0; l < 4 && go; ++l) {
+            if (!(go = mma_barrier(ok))) break;
+            if (l == 0 && first) tmem = *tslot;
             if (t == 0 && !P.skip_mma) {
                 if (l == 0) issue_fwd(tmem + kColD, sx, kMlpIn, kMlpIn, sw + 2 * kW0, kMlpHidden);
                 else if (l < 3) issue_fwd(tmem + kColD, sh[l - 1], kMlpHidden, kMlpHidden, sw + 2 * (l == 1 ? kW1 : kW2), kMlpHidden);
                 else issue_fwd(tmem + kColD, sh[2], kMlpHidden, kMlpHidden, sw + 2 * kW3, kMlpOut);
             }
-            if (!(ok = sync_mma())) break;
-            if (l < 3) epilogue_relu(tmem, hs[l]);
+            commit_wait();
+            if (l < 3) epilogue_relu(tmem + kColD, hs[l]);
         }
-        if (!ok) break;
+        if (!go) break;
         // loss gradient at the outputs -> dY [128 x 64] (columns 40..63 zero)
         {
-            float o[kMlpOut], g[kMlpHidden];
+            float o[kMlpOut], g[20];
             ld_row<kMlpOut>(tmem, kColD, o);
-            const float nl = head_grad(o, wi, w * scale, g);
-            if (w > 0.0f) lsum += w * nl;
+            const float nl = head_grad(o, hi, wi, w * scale, s_q, g);
+            if (w > 0.0f && !hi) lsum += w * nl;
+            const int c0 = hi ? 20 : 0;
 #pragma unroll
-            for (int c = kMlpOut; c < kMlpHidden; ++c) g[c] = 0.0f;
+            for (int c = 0; c < 20; c += 4) {
+                __nv_bfloat162 p[2] = {__floats2bfloat162_rn(g[c], g[c + 1]), __floats2bfloat162_rn(g[c + 2], g[c + 3])};
+                *reinterpret_cast<uint2*>(dy + blk(row, c0 + c, kMlpHidden)) = *reinterpret_cast<const uint2*>(p);
+            }
+            if (hi)
 #pragma unroll
-            for (int c = 0; c < kMlpHidden; c += 8) st_bf16x8(dy + blk(t, c, kMlpHidden), g + c);
+                for (int c = 40; c < kMlpHidden; c += 8)
+                    *reinterpret_cast<uint4*>(dy + blk(row, c, kMlpHidden)) = make_uint4(0u, 0u, 0u, 0u);
         }
         // backward: layer 3 .. 0
         for (int l = 3; l >= 0; --l) {
-            mma_barrier();
+            if (!(go = mma_barrier(ok))) break;
             if (t == 0 && !P.skip_mma) {
                 const uint32_t cw = l == 3 ? kColW3 : (l == 2 ? kColW2 : (l == 1 ? kColW1 : kColW0));
                 if (l > 0) {
-                    issue_dw(tmem + cw, sdy, sh[l - 1], kMlpHidden, kMlpHidden, !first);
                     const uint32_t wl = l == 3 ? kW3 : (l == 2 ? kW2 : kW1);
                     issue_dx(tmem + kColD, sdy, l == 3 ? kMlpOut : kMlpHidden, sw + 2 * wl, kMlpHidden);
+                    issue_dw(tmem + cw, sdy, sh[l - 1], kMlpHidden, kMlpHidden, !first);
                 } else {
                     issue_dw(tmem + cw, sdy, sx, kMlpIn, kMlpIn, !first);
                 }
             }
-            if (!(ok = sync_mma())) break;
+            commit_wait();
             if (l > 0) {
                 // dH = dX masked by ReLU' of the activation it came from, back into dY
                 const __nv_bfloat16* hl = hs[l - 1];
-                float v[kMlpHidden];
-                ld_row<kMlpHidden>(tmem, kColD, v);
+                const int c0 = hi ? 32 : 0;
+                float v[32];
+                ld_row<32>(tmem, kColD + c0, v);
 #pragma unroll
-                for (int c = 0; c < kMlpHidden; c += 8) {
+                for (int c = 0; c < 32; c += 8) {
                     // the activation's 8 bf16 of this chunk in one 16-byte load
-                    const uint4 hv = *reinterpret_cast<const uint4*>(hl + blk(t, c, kMlpHidden));
+                    const uint4 hv = *reinterpret_cast<const uint4*>(hl + blk(row, c0 + c, kMlpHidden));
                     const __nv_bfloat16* hb = reinterpret_cast<const __nv_bfloat16*>(&hv);
 #pragma unroll
                     for (int k = 0; k < 8; ++k)
                         if (!(__bfloat162float(hb[k]) > 0.0f)) v[c + k] = 0.0f;
-                    st_bf16x8(dy + blk(t, c, kMlpHidden), v + c);
+                    st_bf16x8(dy + blk(row, c0 + c, kMlpHidden), v + c);
                 }
             }
         }
-        if (!ok) break;
+        if (!go) break;
         first = false;
     }
-    // flush dW^T (M = 64 rows in lanes 16w .. 16w+15 of warp w's quarter) into grads; after a
-    // wait gave up the accumulators are incomplete and nothing is flushed
-    if (!first && ok) {
+    // flush dW^T (M = 64 rows in lanes 16w .. 16w+15 of warp w's quarter, the two warps of a quarter
+    // taking alternate column groups) into grads; after a wait gave up the accumulators are
+    // incomplete and nothing is flushed
+    const bool done = mma_barrier(ok);
+    if (!first && done) {
         const int warp = t >> 5, lane = t & 31;
-        const int row = 16 * warp + lane;  // output feature
+        const int out = 16 * (warp & 3) + lane;  // output feature
         const uint32_t cols[4] = {kColW0, kColW1, kColW2, kColW3};
         const int nin[4] = {kMlpIn, kMlpHidden, kMlpHidden, kMlpHidden};
         const int nout[4] = {kMlpHidden, kMlpHidden, kMlpHidden, kMlpOut};
         const int off[4] = {kW0, kW1, kW2, kW3};
         for (int l = 0; l < 4; ++l) {
-            for (int c = 0; c < nin[l]; c += 16) {
+            for (int c = hi ? 16 : 0; c < nin[l]; c += 32) {
                 float v[16];
-                ld_row16(tmem, cols[l] + c, v);
-                if (lane < 16 && row < nout[l])
+                ld_row<16>(tmem, cols[l] + c, v);
+                if (lane < 16 && out < nout[l])
                     for (int k = 0; k < 16; ++k)
-                        if (v[k] != 0.0f) atomicAdd(grads + off[l] + (c + k) * nout[l] + row, v[k]);
+                        if (v[k] != 0.0f) atomicAdd(grads + off[l] + (c + k) * nout[l] + out, v[k]);
             }
         }
     }
     // loss
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
     if ((t & 31) == 0 && lsum != 0.0f) atomicAdd(loss_sum, lsum * scale);
-    if (!ok) {
+    if (!done) {
         if (t == 0) atomicOr(P.status, RTPG_STATUS_TIMEOUT);
         mma_drain(mbar, phase, P.poll_limit);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (t < 32) tmem_dealloc(tmem, kTrainCols);
+    if (t < 32) tmem_dealloc(*tslot, kTrainCols);
 }
 
-__global__ void k_wsum(int64_t n, const float* w, float* out) {
+// sums of the nonnegative weights of gridDim.y minibatches of `batch` records (the last shorter)
+__global__ void k_wsum(int64_t n, int64_t batch, const float* w, float* out) {
+    const int64_t b0 = blockIdx.y * batch, m = min(batch, n - b0);
     float s = 0.0f;
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x)
-        s += fmaxf(w[i], 0.0f);
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < m; i += int64_t(gridDim.x) * blockDim.x)
+        s += fmaxf(w[b0 + i], 0.0f);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0 && s != 0.0f) atomicAdd(out, s);
+    if ((threadIdx.x & 31) == 0 && s != 0.0f) atomicAdd(out + blockIdx.y, s);
 }
 
 // fp32 master [in][out] -> bf16 core-matrix layout of each matrix
@@ -291,6 +301,8 @@ __global__ void k_mlp_pack(const float* w, __nv_bfloat16* wq) {
 // Adam (Kingma & Ba 2015) with bias correction; grads zeroed after use
 __global__ void k_mlp_adam(float* w, float* g, float* m, float* v, __nv_bfloat16* wq, float lr, float b1, float b2,
                            float eps, float c1, float c2) {
+    grid_launch_dependents();
+    grid_dependency_wait();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpParams; i += gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.0f - b1) * gi;
@@ -308,12 +320,16 @@ __global__ void k_mlp_adam(float* w, float* g, float* m, float* v, __nv_bfloat16
 
 using namespace rtpg;
 
+constexpr int64_t kMlpGroup = 256;  // minibatches whose weights are summed in one launch
+
 struct rtpg_mlp {
     MlpDev dev{};
-    float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr, *scratch = nullptr;  // scratch: wsum, loss
+    float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
+    float* scratch = nullptr;  // of kMlpGroup minibatches: weight sums, then losses
     __nv_bfloat16* wq = nullptr;
     float lr = 1e-3f, b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     uint32_t step = 0;
+    int64_t last = 0;  // the newest loss's place in scratch's second half
     float mn[3], mx[3];
     // record buffer (filled by the tracer or rtpg_mlp_add_records)
     uint32_t capacity = 0;
@@ -376,7 +392,7 @@ int rtpg_mlp_create(const float* aabb_min, const float* aabb_max, uint32_t seed,
     h->capacity = record_capacity;
     const size_t C = std::max<uint32_t>(record_capacity, 1);
     if ((r = h->alloc(&h->w, kMlpParams)) || (r = h->alloc(&h->g, kMlpParams)) || (r = h->alloc(&h->m, kMlpParams)) ||
-        (r = h->alloc(&h->v, kMlpParams)) || (r = h->alloc(&h->wq, kMlpParams)) || (r = h->alloc(&h->scratch, 4)) ||
+        (r = h->alloc(&h->v, kMlpParams)) || (r = h->alloc(&h->wq, kMlpParams)) || (r = h->alloc(&h->scratch, 2 * kMlpGroup)) ||
         (r = h->alloc(&h->r_pos, 3 * C)) || (r = h->alloc(&h->r_nrm, 3 * C)) || (r = h->alloc(&h->r_wo, 3 * C)) ||
         (r = h->alloc(&h->r_wi, 3 * C)) || (r = h->alloc(&h->r_w, C)) || (r = h->alloc(&h->r_pdf, C)) ||
         (r = h->alloc(&h->r_count, 1)) ||
@@ -469,14 +485,27 @@ int rtpg_mlp_eval(rtpg_mlp* h, int64_t n, const float* pos, const float* nrm, co
 // Gradient of the loss over n records (device arrays) ADDED to host_grads-sized device buffer
 // `grads` (16384 floats, NULL: the handle's own accumulator); returns the loss through
 // host_loss (NULL: none).  The loss is -sum w log q(wi) / sum w.
-static int mlp_grad(rtpg_mlp* h, int64_t n, const float* pos, const float* nrm, const float* wo, const float* wi,
-                    const float* w, float* grads, cudaStream_t st) {
-    RTPG_CUDA(cudaMemsetAsync(h->scratch, 0, 8, st));
-    k_wsum<<<grid_for(n, 256, 4), 256, 0, st>>>(n, w, h->scratch);
-    const int g = (int)std::min<int64_t>((n + kMlpTile - 1) / kMlpTile, kSMs);
-    k_mlp_train<<<g, kMlpThreads, kSmemTrain, st>>>(h->dev, n, Records{pos, nrm, wo, wi, w}, h->scratch, grads,
-                                                   h->scratch + 1);
+// weight sums of up to kMlpGroup minibatches of `batch` records (n records in all), losses zeroed
+static int mlp_group(rtpg_mlp* h, int64_t n, int64_t batch, const float* w, cudaStream_t st) {
+    const int64_t nb = (n + batch - 1) / batch;
+    RTPG_CUDA(cudaMemsetAsync(h->scratch, 0, sizeof(float) * 2 * kMlpGroup, st));
+    k_wsum<<<dim3((unsigned)std::max<int64_t>(1, grid_for(std::min(n, batch), 256, 4) / nb), (unsigned)nb), 256, 0, st>>>(
+        n, batch, w, h->scratch);
     RTPG_LAUNCH_CHECK();
+    return RTPG_OK;
+}
+// gradient over minibatch k of the group; chained: a dependent of the previous step's Adam, before
+// which records and weight sums were complete
+static int mlp_grad(rtpg_mlp* h, int64_t k, int64_t n, const Records& R, float* grads, bool chained, cudaStream_t st) {
+    const int g = (int)std::min<int64_t>((n + kMlpTile - 1) / kMlpTile, kSMs);
+    const float* const wsum = h->scratch + k;
+    float* const loss = h->scratch + kMlpGroup + k;
+    if (chained) {
+        RTPG_CUDA(launch_dependent(k_mlp_train, g, kMlpThreads, kSmemTrain, st, h->dev, n, R, wsum, grads, loss));
+    } else {
+        k_mlp_train<<<g, kMlpThreads, kSmemTrain, st>>>(h->dev, n, R, wsum, grads, loss);
+        RTPG_LAUNCH_CHECK();
+    }
     return RTPG_OK;
 }
 
@@ -484,10 +513,11 @@ int rtpg_mlp_loss_grad(rtpg_mlp* h, int64_t n, const float* pos, const float* nr
                        const float* w, float* grads, float* host_loss, void* stream) {
     if (!h || n <= 0 || !pos || !nrm || !wo || !wi || !w) return fail(RTPG_EINVAL, "rtpg_mlp_loss_grad: bad arguments");
     cudaStream_t st = as_stream(stream);
-    int r = mlp_grad(h, n, pos, nrm, wo, wi, w, grads ? grads : h->g, st);
-    if (r) return r;
+    h->last = 0;
+    int r = mlp_group(h, n, n, w, st);
+    if (r || (r = mlp_grad(h, 0, n, Records{pos, nrm, wo, wi, w}, grads ? grads : h->g, false, st))) return r;
     if (host_loss) {
-        RTPG_CUDA(cudaMemcpyAsync(host_loss, h->scratch + 1, 4, cudaMemcpyDeviceToHost, st));
+        RTPG_CUDA(cudaMemcpyAsync(host_loss, h->scratch + kMlpGroup, 4, cudaMemcpyDeviceToHost, st));
         RTPG_CUDA(cudaStreamSynchronize(st));
     }
     return RTPG_OK;
@@ -509,17 +539,24 @@ int rtpg_mlp_train(rtpg_mlp* h, int64_t n, const float* pos, const float* nrm, c
         return fail(RTPG_EINVAL, "rtpg_mlp_train: record arrays missing");
     }
     for (uint32_t e = 0; e < epochs; ++e)
-        for (int64_t b = 0; b < n; b += batch) {
-            const int64_t m = std::min<int64_t>(batch, n - b);
-            int r = mlp_grad(h, m, pos + 3 * b, nrm + 3 * b, wo + 3 * b, wi + 3 * b, w + b, h->g, st);
+        for (int64_t g0 = 0; g0 < n; g0 += kMlpGroup * batch) {
+            const int64_t in_group = std::min<int64_t>(kMlpGroup * batch, n - g0);
+            int r = mlp_group(h, in_group, batch, w + g0, st);
             if (r) return r;
-            ++h->step;
-            const float c1 = 1.0f - std::pow(h->b1, (float)h->step), c2 = 1.0f - std::pow(h->b2, (float)h->step);
-            k_mlp_adam<<<64, 256, 0, st>>>(h->w, h->g, h->m, h->v, h->wq, h->lr, h->b1, h->b2, h->eps, c1, c2);
-            RTPG_LAUNCH_CHECK();
+            for (int64_t b = 0; b < in_group; b += batch) {
+                const int64_t at = g0 + b;
+                h->last = b / batch;
+                r = mlp_grad(h, h->last, std::min<int64_t>(batch, in_group - b),
+                             Records{pos + 3 * at, nrm + 3 * at, wo + 3 * at, wi + 3 * at, w + at}, h->g, b > 0, st);
+                if (r) return r;
+                ++h->step;
+                const float c1 = 1.0f - std::pow(h->b1, (float)h->step), c2 = 1.0f - std::pow(h->b2, (float)h->step);
+                RTPG_CUDA(launch_dependent(k_mlp_adam, 64, 256, 0, st, h->w, h->g, h->m, h->v, h->wq, h->lr, h->b1, h->b2,
+                                           h->eps, c1, c2));
+            }
         }
     if (host_last_loss) {
-        RTPG_CUDA(cudaMemcpyAsync(host_last_loss, h->scratch + 1, 4, cudaMemcpyDeviceToHost, st));
+        RTPG_CUDA(cudaMemcpyAsync(host_last_loss, h->scratch + kMlpGroup + h->last, 4, cudaMemcpyDeviceToHost, st));
         RTPG_CUDA(cudaStreamSynchronize(st));
     }
     return RTPG_OK;

@@ -2,9 +2,11 @@
 // run on the 5th-generation tensor cores (tcgen05.mma, BF16 operands in shared memory, FP32
 // accumulators in tensor memory).
 //
-// One CTA of 128 threads owns a tile of 128 samples: thread t computes the features of sample
-// t, one elected thread issues the MMAs of a layer, and thread t reads row t of the
-// accumulator back from tensor memory (TMEM lane t) for the epilogue.  Matrices live in shared
+// One CTA of 256 threads owns a tile of 128 samples, two threads per sample: threads t and t + 128
+// compute one half each of the features of sample t, one elected thread issues the MMAs of a
+// layer, and both read half of row t of the accumulator back from tensor memory (TMEM lane t) for
+// the epilogue.  The layers depend on one another, so a tile's time is the sum of its phases; two
+// threads per sample halve what a phase does between its MMAs.  Matrices live in shared
 // memory in the no-swizzle "core matrix" layout of the UMMA descriptors: 8 rows x 16 bytes
 // (8 bf16) per 128-byte core matrix, core matrices of a row group adjacent (128 B apart), row
 // groups (C / 8) * 128 B apart for a C-column matrix.  The same storage serves as a K-major
@@ -116,6 +118,11 @@ __device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t* r) {
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
 }
+__device__ __forceinline__ void tmem_ld8_async(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
     uint32_t r[16];
@@ -124,12 +131,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
-// `n` (a multiple of 16, at most 64) columns with the loads in flight together
+// N (a multiple of 8, at most 64) columns with the loads in flight together
 template <int N>
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, float* v) {
     uint32_t r[N];
 #pragma unroll
-    for (int c = 0; c < N; c += 16) tmem_ld16_async(taddr + c, r + c);
+    for (int c = 0; c + 16 <= N; c += 16) tmem_ld16_async(taddr + c, r + c);
+    if (N % 16) tmem_ld8_async(taddr + N - 8, r + N - 8);
     tmem_wait_ld();
 #pragma unroll
     for (int i = 0; i < N; ++i) v[i] = __uint_as_float(r[i]);
@@ -145,24 +153,40 @@ __device__ __forceinline__ void st_bf16x8(__nv_bfloat16* dst, const float* v) {
 
 // ------------------------------------------------------------------ features
 // Position normalised to the AABB, 12 frequencies of sin / cos of pi 2^j u per axis, then the
-// shading normal, the outgoing direction, a constant 1 (the first layer's bias) and a zero.
-__device__ __forceinline__ void mlp_features(float3 pos, float3 nrm, float3 wo, float3 mn, float3 inv_ext, float* f) {
+// shading normal, the outgoing direction, a constant 1 (the first layer's bias) and a zero: 80
+// features, of which half 0 forms the first 40 and half 1 the rest, eight at a time straight into
+// row `row` of the shared-memory operand.  live = false: a row of zeros.
+template <int HALF>
+__device__ __forceinline__ void store_features_of(__nv_bfloat16* x0, int row, bool live, float3 pos, float3 nrm, float3 wo,
+                                                  float3 mn, float3 inv_ext) {
     const float u[3] = {(pos.x - mn.x) * inv_ext.x, (pos.y - mn.y) * inv_ext.y, (pos.z - mn.z) * inv_ext.z};
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        float a = u[c];
+    for (int c8 = HALF * 5; c8 < HALF * 5 + 5; ++c8) {
+        float f[8];
+        if (c8 < 9) {  // four frequencies of one axis
+            const int axis = c8 / 3, j0 = (c8 % 3) * 4;
+            float a = u[axis] * (float)(1 << j0);
 #pragma unroll
-        for (int j = 0; j < kMlpFreqs; ++j) {
-            float s, co;
-            sincospif(a, &s, &co);
-            f[c * 24 + 2 * j] = s;
-            f[c * 24 + 2 * j + 1] = co;
-            a = a * 2.0f;
+            for (int j = 0; j < 4; ++j) {
+                sincospif(a, &f[2 * j], &f[2 * j + 1]);
+                a = a * 2.0f;
+            }
+        } else {
+            f[0] = nrm.x; f[1] = nrm.y; f[2] = nrm.z;
+            f[3] = wo.x; f[4] = wo.y; f[5] = wo.z;
+            f[6] = 1.0f; f[7] = 0.0f;
         }
+        if (!live)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) f[k] = 0.0f;
+        st_bf16x8(x0 + blk(row, c8 * 8, kMlpIn), f);
     }
-    f[72] = nrm.x; f[73] = nrm.y; f[74] = nrm.z;
-    f[75] = wo.x; f[76] = wo.y; f[77] = wo.z;
-    f[78] = 1.0f; f[79] = 0.0f;
+}
+__device__ __forceinline__ void store_features(__nv_bfloat16* x0, bool live, float3 pos, float3 nrm, float3 wo, float3 mn,
+                                               float3 inv_ext) {
+    const int row = threadIdx.x & (kMlpTile - 1);
+    if (threadIdx.x < kMlpTile) store_features_of<0>(x0, row, live, pos, nrm, wo, mn, inv_ext);
+    else store_features_of<1>(x0, row, live, pos, nrm, wo, mn, inv_ext);
 }
 
 // ------------------------------------------------------------------ vMF mixture
@@ -188,6 +212,30 @@ __device__ __forceinline__ void mlp_head(const float* o, VmfLobe* L) {
     const float inv = 1.0f / se;
 #pragma unroll
     for (int k = 0; k < kMlpLobes; ++k) L[k].weight *= inv;
+}
+// the same for the four lobes of one half (k = 4 half .. 4 half + 3) only
+__device__ __forceinline__ void mlp_head_half(const float* o, bool hi, VmfLobe* L) {
+    float mx = -1e30f;
+#pragma unroll
+    for (int k = 0; k < kMlpLobes; ++k) mx = fmaxf(mx, o[5 * k + 4]);
+    float se = 0.0f, w[kMlpLobes];
+#pragma unroll
+    for (int k = 0; k < kMlpLobes; ++k) {
+        w[k] = __expf(o[5 * k + 4] - mx);
+        se += w[k];
+    }
+    const float inv = 1.0f / se;
+#pragma unroll
+    for (int k = 0; k < kMlpLobes / 2; ++k) {
+        float q[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) q[j] = hi ? o[5 * (k + 4) + j] : o[5 * k + j];
+        const float3 m = f3(q[0], q[1], q[2]);
+        const float len = sqrtf(dot3(m, m));
+        L[k].mu = len > 1e-12f ? m * (1.0f / len) : f3(0.f, 0.f, 1.f);
+        L[k].kappa = __expf(fminf(fmaxf(q[3], kLogKappaMin), kLogKappaMax));
+        L[k].weight = (hi ? w[k + 4] : w[k]) * inv;
+    }
 }
 // density of one lobe at w: kappa / (2 pi (1 - e^{-2 kappa})) exp(kappa (mu.w - 1))
 __device__ __forceinline__ float vmf_pdf(const VmfLobe& l, float3 w) {
@@ -228,7 +276,7 @@ __device__ __forceinline__ float3 vmf_mixture_sample(const VmfLobe* L, float u0,
 }
 
 // ------------------------------------------------------------------ network building blocks
-constexpr int kMlpThreads = kMlpTile;
+constexpr int kMlpThreads = 2 * kMlpTile;
 constexpr size_t kSmemW = size_t(kMlpParams) * 2;             // 32 KB of bf16 weights
 constexpr size_t kSmemX = size_t(kMlpTile) * kMlpIn * 2;       // 20 KB input features
 constexpr size_t kSmemH = size_t(kMlpTile) * kMlpHidden * 2;   // 16 KB per hidden activation
@@ -280,18 +328,15 @@ __device__ __forceinline__ void load_weights(__nv_bfloat16* ws, const __nv_bfloa
     uint4* d = reinterpret_cast<uint4*>(ws);
     for (int i = threadIdx.x; i < kMlpParams / 8; i += blockDim.x) d[i] = __ldg(s + i);
 }
-// features of sample t into row t of X0
-__device__ __forceinline__ void store_features(__nv_bfloat16* x0, int t, const float* f) {
-#pragma unroll
-    for (int c = 0; c < kMlpIn; c += 8) st_bf16x8(x0 + blk(t, c, kMlpIn), f + c);
-}
-// all threads: make the shared-memory operands written by this CTA visible to the tensor
-// cores and order earlier TMEM loads before the next MMA
-__device__ __forceinline__ void mma_barrier() {
+// All threads: make the shared-memory operands written by this CTA visible to the tensor cores and
+// order earlier TMEM loads before the next MMA.  ok: the thread's last wait; returns whether no
+// thread's wait gave up (uniform over the CTA), false: issue nothing more.
+__device__ __forceinline__ bool mma_barrier(bool ok) {
     fence_async_smem();
     tc_fence_before();
-    __syncthreads();
+    ok = __syncthreads_and(ok) != 0;
     tc_fence_after();
+    return ok;
 }
 // D[128 x n] (+)= A[128 x k] (K-major, a_cols columns) x W[k x n] (MN-major, n columns)
 __device__ __forceinline__ void issue_fwd(uint32_t d, uint32_t a, uint32_t a_cols, uint32_t k, uint32_t w, uint32_t n) {
@@ -310,59 +355,92 @@ __device__ __forceinline__ void issue_dw(uint32_t d, uint32_t dy, uint32_t x, ui
     for (uint32_t kk = 0; kk < kMlpTile; kk += 16)
         umma_f16(d, desc_mnmajor(dy, kk, kMlpHidden), desc_mnmajor(x, kk, x_cols), id, (acc || kk > 0) ? 1u : 0u);
 }
-// thread t: accumulator row t, columns c0 .. c0+15
-__device__ __forceinline__ void ld_row16(uint32_t tmem, uint32_t col, float* v) {
-    const uint32_t lane = (threadIdx.x & ~31u);
-    tmem_ld16(tmem + (lane << 16) + col, v);
-}
-// thread t: accumulator row t, columns c0 .. c0+N-1 in one batch of loads
+// thread t: accumulator row t mod 128, columns c0 .. c0+N-1 in one batch of loads
 template <int N>
 __device__ __forceinline__ void ld_row(uint32_t tmem, uint32_t col, float* v) {
-    const uint32_t lane = (threadIdx.x & ~31u);
+    const uint32_t lane = threadIdx.x & (kMlpTile - 32);
     tmem_ld_cols<N>(tmem + (lane << 16) + col, v);
 }
-// hidden epilogue: ReLU, bf16, row t of h [128 x 64]
-__device__ __forceinline__ void epilogue_relu(uint32_t tmem, __nv_bfloat16* h) {
-    const int t = threadIdx.x;
-    float v[kMlpHidden];
-    ld_row<kMlpHidden>(tmem, kColD, v);
+// hidden epilogue: ReLU, bf16, the thread's 32 columns of its row of h [128 x 64]
+__device__ __forceinline__ void epilogue_relu(uint32_t d, __nv_bfloat16* h) {
+    const uint32_t row = threadIdx.x & (kMlpTile - 1), c0 = threadIdx.x / kMlpTile * 32;
+    float v[32];
+    ld_row<32>(d, c0, v);
+    // rounded first, then two activations per maximum: the same values
+    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.0f, 0.0f);
 #pragma unroll
-    for (int i = 0; i < kMlpHidden; ++i) v[i] = fmaxf(v[i], 0.0f);
+    for (int c = 0; c < 32; c += 8) {
+        __align__(16) __nv_bfloat162 p[4];
 #pragma unroll
-    for (int c = 0; c < kMlpHidden; c += 8) st_bf16x8(h + blk(t, c, kMlpHidden), v + c);
+        for (int i = 0; i < 4; ++i) p[i] = __hmax2(__floats2bfloat162_rn(v[c + 2 * i], v[c + 2 * i + 1]), zero);
+        *reinterpret_cast<uint4*>(h + blk(row, c0 + c, kMlpHidden)) = *reinterpret_cast<const uint4*>(p);
+    }
 }
-
-// Completion of the MMAs thread 0 committed to `mbar`: every thread waits (bounded), and the
-// outcome is made uniform over the CTA.  On success the phase flips; on a timeout it stays,
-// so mma_drain can wait for the same phase before TMEM is freed.
+// wait for the MMAs thread 0 committed to `mbar` (bounded).  On success the phase flips; on a
+// timeout it stays, so mma_drain can wait for the same phase before TMEM is freed.  The outcome
+// becomes uniform in the next mma_barrier.
 __device__ __forceinline__ bool mma_complete(uint64_t* mbar, uint32_t& phase, uint32_t limit) {
-    const bool ok = __syncthreads_and(mbar_wait(mbar, phase, limit)) != 0;
+    const bool ok = mbar_wait(mbar, phase, limit);
     if (ok) phase ^= 1u;
     tc_fence_after();
     return ok;
 }
 
 // Forward pass of one tile: the features of sample t are in row t of x0 (which the hidden
-// activations then overwrite); returns sample t's 48 raw outputs in o.  Every thread of the
-// 128-thread CTA calls it; thread 0 issues the MMAs.  False (uniformly over the CTA, with o
-// not written) if a wait on the tensor cores gave up: the caller then issues nothing more,
-// drains with mma_drain and frees its TMEM.
-__device__ __forceinline__ bool mlp_forward_tile(const MlpDev& P, uint32_t tmem, uint32_t sw, __nv_bfloat16* x0,
-                                                 uint64_t* mbar, uint32_t& phase, float* o) {
+// activations then overwrite), the accumulator is in TMEM columns d .. d + 63.  Every thread calls
+// it; thread 0 issues the MMAs.  ok: the thread's last wait, on return its newest one; false if any
+// thread's wait gave up before (uniformly over the CTA): the caller then issues nothing more,
+// drains with mma_drain and frees its TMEM.  The outputs are in columns d .. d + 47 of row t mod 128,
+// valid where ok.
+__device__ __forceinline__ bool mlp_forward_tile(const MlpDev& P, uint32_t d, uint32_t sw, __nv_bfloat16* x0,
+                                                 uint64_t* mbar, uint32_t& phase, bool& ok) {
     const uint32_t sx = smem_u32(x0);
     for (int l = 0; l < 4; ++l) {
-        mma_barrier();
+        if (!mma_barrier(ok)) return false;
         if (threadIdx.x == 0 && !P.skip_mma) {
-            if (l == 0) issue_fwd(tmem + kColD, sx, kMlpIn, kMlpIn, sw + 2 * kW0, kMlpHidden);
-            else if (l < 3) issue_fwd(tmem + kColD, sx, kMlpHidden, kMlpHidden, sw + 2 * (l == 1 ? kW1 : kW2), kMlpHidden);
-            else issue_fwd(tmem + kColD, sx, kMlpHidden, kMlpHidden, sw + 2 * kW3, kMlpOut);
+            if (l == 0) issue_fwd(d, sx, kMlpIn, kMlpIn, sw + 2 * kW0, kMlpHidden);
+            else if (l < 3) issue_fwd(d, sx, kMlpHidden, kMlpHidden, sw + 2 * (l == 1 ? kW1 : kW2), kMlpHidden);
+            else issue_fwd(d, sx, kMlpHidden, kMlpHidden, sw + 2 * kW3, kMlpOut);
             umma_commit(mbar);
         }
-        if (!mma_complete(mbar, phase, P.poll_limit)) return false;
-        if (l < 3) epilogue_relu(tmem, x0);
+        ok = mma_complete(mbar, phase, P.poll_limit);
+        if (l < 3) epilogue_relu(d, x0);
     }
-    ld_row<kMlpOut>(tmem, kColD, o);
     return true;
+}
+
+// What an inference CTA sets up once: TMEM, mbarrier, weights.  Every thread calls it, and eval_end
+// with its last wait.
+struct EvalCta {
+    __nv_bfloat16* x0;
+    uint64_t* mbar;
+    uint32_t d, sw, phase;
+};
+__device__ __forceinline__ EvalCta eval_begin(uint8_t* sm, const __nv_bfloat16* wq) {
+    EvalCta c;
+    c.x0 = reinterpret_cast<__nv_bfloat16*>(sm + kSmemW);
+    c.mbar = reinterpret_cast<uint64_t*>(sm + kSmemW + kSmemX);
+    uint32_t* const slot = reinterpret_cast<uint32_t*>(c.mbar + 1);
+    if (threadIdx.x < 32) tmem_alloc(slot, kEvalCols);
+    if (threadIdx.x == 0) mbar_init(c.mbar, 1);
+    load_weights(reinterpret_cast<__nv_bfloat16*>(sm), wq);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    c.d = *slot + kColD;
+    c.sw = smem_u32(sm);
+    c.phase = 0;
+    return c;
+}
+__device__ __forceinline__ void eval_end(const EvalCta& c, bool ok, uint32_t limit, unsigned* status) {
+    if (!mma_barrier(ok)) {
+        if (threadIdx.x == 0) atomicOr(status, RTPG_STATUS_TIMEOUT);
+        mma_drain(c.mbar, c.phase, limit);
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+    }
+    if (threadIdx.x < 32) tmem_dealloc(c.d - kColD, kEvalCols);
 }
 
 }  // namespace rtpg

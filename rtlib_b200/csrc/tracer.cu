@@ -641,30 +641,18 @@ __global__ void __launch_bounds__(kTB) k_hit(TracerDev T, uint32_t bounce) {
 
 // learned guide, stage 2: the mixture of every queued path that hit a Phong surface, 128
 // paths per tile on the tensor cores (features of path q in row q of the tile)
-__global__ void __launch_bounds__(kMlpThreads) k_mlp_lobes(TracerDev T, uint32_t bounce) {
+__global__ void __launch_bounds__(kMlpThreads, 4) k_mlp_lobes(TracerDev T, uint32_t bounce) {
     grid_dependency_wait();
     const int in = int(bounce & 1);
     extern __shared__ __align__(128) uint8_t sm[];
-    __nv_bfloat16* ws = reinterpret_cast<__nv_bfloat16*>(sm);
-    __nv_bfloat16* x0 = reinterpret_cast<__nv_bfloat16*>(sm + kSmemW);
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kSmemW + kSmemX);
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kSmemW + kSmemX + 8);
-    const int t = threadIdx.x;
-    if (t < 32) tmem_alloc(tslot, kEvalCols);
-    if (t == 0) mbar_init(mbar, 1);
-    load_weights(ws, T.ml.dev.wq);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tslot, sw = smem_u32(ws);
-    uint32_t phase = 0;
+    EvalCta c = eval_begin(sm, T.ml.dev.wq);
     bool ok = true;
     const uint32_t n = T.qcount[bounce % 3];
     for (uint32_t base = blockIdx.x * kMlpTile; base < n; base += gridDim.x * kMlpTile) {
-        const uint32_t q = base + t;
+        const uint32_t q = base + threadIdx.x % kMlpTile;
         bool live = false;
         uint32_t p = 0;
-        float f[kMlpIn];
+        float3 x = f3(0.f, 0.f, 0.f), fn = x, wo = x;
         if (q < n) {
             p = T.queue[in][q];
             const uint32_t prim = T.hit_prim[p];
@@ -675,45 +663,35 @@ __global__ void __launch_bounds__(kMlpThreads) k_mlp_lobes(TracerDev T, uint32_t
             if (live) {
                 const float4 tuv = T.hit_tuv[p];
                 const float3 o = T.org[p], d = T.dir[p];
-                const float3 fn = xyz(T.tri_frame[prim].fr[0]);
-                mlp_features(o + tuv.x * d, fn, f3(-d.x, -d.y, -d.z), T.ml.dev.mn, T.ml.dev.inv_ext, f);
+                fn = xyz(T.tri_frame[prim].fr[0]);
+                x = o + tuv.x * d;
+                wo = f3(-d.x, -d.y, -d.z);
             }
         }
-        if (!live)
-#pragma unroll
-            for (int k = 0; k < kMlpIn; ++k) f[k] = 0.0f;
-        store_features(x0, t, f);
+        store_features(c.x0, live, x, fn, wo, T.ml.dev.mn, T.ml.dev.inv_ext);
+        if (!mlp_forward_tile(T.ml.dev, c.d, c.sw, c.x0, c.mbar, c.phase, ok)) break;  // uniform: issue nothing more
         float o[kMlpOut];
-        if (!mlp_forward_tile(T.ml.dev, tmem, sw, x0, mbar, phase, o)) {
-            ok = false;  // uniform over the CTA: issue nothing more
-            break;
-        }
-        if (live) {
-            VmfLobe L[kMlpLobes];
-            mlp_head(o, L);
-            __align__(16) __half lp[40];
+        ld_row<kMlpOut>(c.d, 0, o);
+        if (live && ok) {
+            const bool hi = threadIdx.x >= kMlpTile;
+            VmfLobe L[kMlpLobes / 2];
+            mlp_head_half(o, hi, L);
+            __align__(8) __half lp[20];
 #pragma unroll
-            for (int k = 0; k < kMlpLobes; ++k) {
+            for (int k = 0; k < kMlpLobes / 2; ++k) {
                 lp[5 * k] = __float2half_rn(L[k].mu.x);
                 lp[5 * k + 1] = __float2half_rn(L[k].mu.y);
                 lp[5 * k + 2] = __float2half_rn(L[k].mu.z);
                 lp[5 * k + 3] = __float2half_rn(L[k].kappa);
                 lp[5 * k + 4] = __float2half_rn(L[k].weight);
             }
-            // 80 bytes per path: five 16-byte stores
-            uint4* dst = reinterpret_cast<uint4*>(T.lobes + size_t(p) * 40);
+            // 40 of the path's 80 bytes: five 8-byte stores
+            uint2* dst = reinterpret_cast<uint2*>(T.lobes + size_t(p) * 40 + (hi ? 20 : 0));
 #pragma unroll
-            for (int k = 0; k < 5; ++k) dst[k] = reinterpret_cast<const uint4*>(lp)[k];
+            for (int k = 0; k < 5; ++k) dst[k] = reinterpret_cast<const uint2*>(lp)[k];
         }
     }
-    if (!ok) {
-        if (t == 0) atomicOr(T.status, RTPG_STATUS_TIMEOUT);
-        mma_drain(mbar, phase, T.ml.dev.poll_limit);
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (t < 32) tmem_dealloc(tmem, kEvalCols);
+    eval_end(c, ok, T.ml.dev.poll_limit, T.status);
 }
 
 // FLAT: the scene's triangles are in the kernel parameters.  A template argument, so that neither

@@ -265,3 +265,69 @@ def test_hashgrid_noalloc_table_alignment(cuda, oracle, offset):
         np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), want)
     np.testing.assert_array_equal(table.cpu().numpy().view(np.uint64), cur)
     assert not store[:offset].any() and not store[offset + slots:].any()
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 592 * 128 + 5])
+def test_network_tile_edges(cuda, n):
+    """Partial tiles, one tile per CTA and a CTA's second tile: each sample's row equals the one a
+    single-tile call gives, raw outputs and lobes, into arrays with and without 16-byte alignment."""
+    import torch
+    from rtlib_b200._lib import call, ptr, stream_ptr
+    from rtlib_b200.mlp import MLPGuide
+    rng = np.random.default_rng(n)
+    g = MLPGuide((0, 0, 0), (1, 1, 1), seed=4)
+    unit = lambda: (lambda v: (v / np.linalg.norm(v, axis=1, keepdims=True)).astype(np.float32))(rng.normal(size=(n, 3)))
+    pos, nrm, wo = _t(rng.random((n, 3), dtype=np.float32), cuda), _t(unit(), cuda), _t(unit(), cuda)
+    raw, lobes = g.eval(pos, nrm, wo), g.eval(pos, nrm, wo, raw=False)
+    for a in sorted({0, n // 2, max(0, n - 100)}):
+        sl = slice(a, min(n, a + 100))
+        one = [x[sl].contiguous() for x in (pos, nrm, wo)]
+        assert torch.equal(g.eval(*one), raw[sl]) and torch.equal(g.eval(*one, raw=False), lobes[sl])
+    store = torch.full((n * 48 + 8,), 7.0, device=cuda)
+    call("rtpg_mlp_eval", g.h, n, ptr(pos), ptr(nrm), ptr(wo), ptr(store) + 4, None, stream_ptr())
+    assert torch.equal(store[1:1 + n * 48].view(n, 48), raw) and (store[1 + n * 48:] == 7.0).all()
+    assert g.status() == 0
+
+
+@pytest.mark.parametrize("steps", [255, 256, 257, 600])
+def test_training_groups_of_minibatches(cuda, steps):
+    """Weight sums are formed for 256 minibatches at a time and launches chained within them: steps
+    taken in one call equal the same steps taken in several, bit for bit (one record per step: every
+    gradient element is added once, so nothing depends on the order of atomics)."""
+    from rtlib_b200.mlp import MLPGuide
+    rng = np.random.default_rng(steps)
+    unit = lambda: (lambda v: (v / np.linalg.norm(v, axis=1, keepdims=True)).astype(np.float32))(rng.normal(size=(steps, 3)))
+    rec = [_t(a, cuda) for a in (rng.random((steps, 3), dtype=np.float32), unit(), unit(), unit(),
+                                 rng.lognormal(0, 1, steps).astype(np.float32))]
+    a, b = MLPGuide((0, 0, 0), (1, 1, 1), seed=9), MLPGuide((0, 0, 0), (1, 1, 1), seed=9)
+    la = a.train(rec, batch=1, epochs=1)
+    for s in (0, 100, 101, steps):
+        if s == steps:
+            break
+        e = {0: 100, 100: 101, 101: steps}[s]
+        lb = b.train([x[s:e].contiguous() for x in rec], batch=1, epochs=1)
+    np.testing.assert_array_equal(a.params(), b.params())
+    assert la == lb and a.status() == 0 and b.status() == 0
+
+
+@pytest.mark.parametrize("n", [1, 128, 129, 148 * 128 + 77])
+def test_gradient_is_the_sum_of_its_tiles(cuda, n):
+    """Partial tiles and a CTA's second tile: the gradient over all records is the weighted sum of the
+    gradients over single tiles, up to the rounding of float sums."""
+    import torch
+    from rtlib_b200.mlp import MLPGuide
+    rng = np.random.default_rng(n)
+    unit = lambda: (lambda v: (v / np.linalg.norm(v, axis=1, keepdims=True)).astype(np.float32))(rng.normal(size=(n, 3)))
+    w = np.ones(n, np.float32)  # equal weights: no clamp, and the same scale in both sums
+    rec = [_t(a, cuda) for a in (rng.random((n, 3), dtype=np.float32), unit(), unit(), unit(), w)]
+    g = MLPGuide((0, 0, 0), (1, 1, 1), seed=2)
+    loss, grad = g.loss_grad(*rec)
+    want, wloss = torch.zeros(16384, device=cuda, dtype=torch.float64), 0.0
+    for s in range(0, n, 128):
+        part = [x[s:s + 128].contiguous() for x in rec]
+        l, p = g.loss_grad(*part)
+        want += p.double() * len(part[0]) / n
+        wloss += l * len(part[0]) / n
+    # the output gradients enter as bf16 (2^-9 relative) at another scale per call
+    assert (grad.double() - want).norm() < 0.01 * want.norm()
+    assert abs(loss - wloss) < 1e-4 * abs(wloss) and g.status() == 0
