@@ -145,8 +145,15 @@ def lib():
     return _lib
 
 
+# bound functions by name: a CDLL attribute look-up per call costs as much as the call
+_fns = {}
+
+
 def call(name, *args):
-    r = getattr(lib(), name)(*args)
+    fn = _fns.get(name)
+    if fn is None:
+        fn = _fns[name] = getattr(lib(), name)
+    r = fn(*args)
     if r != 0:
         msg = lib().rtpg_last_error()
         raise RtpgError(name, r, msg.decode() if msg else "")
@@ -168,15 +175,26 @@ def ptr(x):
     raise TypeError(f"cannot take a pointer of {type(x)}")
 
 
+_torch_cuda = None  # torch.cuda once a device was seen: asking for one again costs microseconds
+_raw_stream = None  # torch's own accessor of the current stream's handle, where it has one
+
+
 def stream_ptr(stream=None):
+    """cudaStream_t of a torch stream, an int, or (None) the current stream of the current device."""
+    global _torch_cuda, _raw_stream
     if stream is None:
-        try:
-            import torch
-            if torch.cuda.is_available():
-                return torch.cuda.current_stream().cuda_stream
-        except ImportError:
-            pass
-        return None
+        if _torch_cuda is None:
+            try:
+                import torch
+                if not torch.cuda.is_available():
+                    return None
+                _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+                _torch_cuda = torch.cuda
+            except ImportError:
+                return None
+        if _raw_stream is not None:
+            return _raw_stream(_torch_cuda.current_device())
+        return _torch_cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
