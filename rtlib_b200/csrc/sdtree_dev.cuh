@@ -76,11 +76,22 @@ __host__ __device__ inline bool sq_choice(int side, float s, float bnd, float b)
     const float q = side == 1 ? sq_div(s, bnd) : sq_div(sq_sub(s, bnd), sq_sub(1.0f, bnd));
     return q >= b;
 }
-// the smallest k for which sq_choice holds at draw k 2^-23, kNever when none does (bisection
-// over the draws; sq_choice is non-decreasing in s where that side is reachable)
+// The smallest k for which sq_choice holds at draw k 2^-23, kNever when none does (bisection
+// over the draws; sq_choice is non-decreasing in s where that side is reachable).  Each rounding in
+// sq_choice moves its quotient by 2^-24, so k is within a step or two of where the exact quotient
+// meets b: the bisection starts from four steps to either side if the choice changes there, else
+// (an empty side, a boundary past 1) from the whole range.  5 instead of 24 evaluations of up to two
+// dependent divisions: the build of a lone node 8.0 -> 4.3 us, of 64 trees 25.5 -> 19.2.
 __host__ __device__ inline uint32_t sq_threshold(int side, float bnd, float b) {
-    uint32_t lo = 0, hi = kDrawSteps - 1;
-    if (!sq_choice(side, draw_value(hi), bnd, b)) return kNever;
+    const float at = side == 0 ? bnd : side == 1 ? b * bnd : bnd + b * sq_sub(1.0f, bnd);
+    const float g = at * 8388608.0f;
+    const bool near = g >= 0.0f && g < 8388608.0f;  // false for NaN
+    uint32_t lo = near && g > 4.0f ? (uint32_t)g - 4 : 0, hi = near && g < 8388600.0f ? (uint32_t)g + 4 : kDrawSteps - 1;
+    if (!near || !sq_choice(side, draw_value(hi), bnd, b) || (lo > 0 && sq_choice(side, draw_value(lo), bnd, b))) {
+        lo = 0;
+        hi = kDrawSteps - 1;
+        if (!sq_choice(side, draw_value(hi), bnd, b)) return kNever;
+    }
     while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
         if (sq_choice(side, draw_value(mid), bnd, b)) hi = mid;

@@ -331,3 +331,30 @@ def test_gradient_is_the_sum_of_its_tiles(cuda, n):
     # the output gradients enter as bf16 (2^-9 relative) at another scale per call
     assert (grad.double() - want).norm() < 0.01 * want.norm()
     assert abs(loss - wloss) < 1e-4 * abs(wloss) and g.status() == 0
+
+
+def test_sampling_thresholds_near_and_past_boundaries(cuda, oracle):
+    """Quadrant sums whose boundary or second quotient lies on a draw, at 0 or at 1, on one side only
+    or many orders apart: samples and pdfs of single-node trees equal the oracle's divisions."""
+    import torch
+    from rtlib_b200.sdtree import SDTree
+    rng = np.random.default_rng(8)
+    sums = [(1, 1, 1, 1), (1, 0, 0, 0), (0, 1, 0, 0), (0, 0, 1, 0), (0, 0, 0, 1), (1, 0, 1, 0), (0, 1, 0, 1), (3, 1, 0, 2),
+            (1e-5, 1, 1e-5, 1), (1, 1e-5, 1, 1e-5), (1e-6, 1, 3e-6, 1e5), (0.1, 0.2, 0.3, 0.4), (1e-7, 1e-7, 1e-7, 4e6)]
+    sums += [tuple(rng.lognormal(0, 6, 4)) for _ in range(24)]
+    uv = np.array([[0.2, 0.2], [0.7, 0.2], [0.2, 0.7], [0.7, 0.7]], np.float32)
+    pos = np.full((4, 3), 0.5, np.float32)
+    q = W.sdtree_queries(20000, 3)
+    for s in sums:
+        g, o = SDTree((0, 0, 0), (1, 1, 1)), oracle.sdtree((0, 0, 0), (1, 1, 1))
+        r = np.array(s, np.float32)
+        g.record(_t(pos, cuda), _t(uv, cuda), _t(r, cuda))
+        o.record(pos, uv, r)
+        g.build()
+        o.build()
+        a = torch.empty((20000, 2), device=cuda)
+        p = torch.empty(20000, device=cuda)
+        g.sample_pdf(_t(q["pos"], cuda), _t(q["seeds"], cuda), out_uv=a, out_pdf_uv=p)
+        wa, wp = o.sample_pdf(q["pos"], q["seeds"])[:2]
+        np.testing.assert_array_equal(a.cpu().numpy(), wa)
+        np.testing.assert_array_equal(p.cpu().numpy(), wp)
