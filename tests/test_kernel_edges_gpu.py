@@ -201,6 +201,33 @@ def test_whole_path_waves_equal_bounce_waves(cuda, w, h, spp):
     assert cnt == ref.counters()
 
 
+@pytest.mark.parametrize("counts", [[578], [1, 6, 571], [2] * 256 + [3, 63], [1] * 64])
+def test_packed_lights_sample_like_indexed_ones(cuda, counts):
+    """Light meshes of one and of many triangles, powers of two and not.  Entries in front of the
+    lights, more than there are paths, rule the packed copy out; the image is the same.  The caller's
+    index array is read at each render."""
+    from rtlib_b200 import scenes
+    from rtlib_b200.tracer import FLAG_NEE, FLAG_RIS, Tracer
+    w, h = 148 * 7, 129  # past the path-per-thread limit
+    sc = scenes.cornell_box(w, h, light_grid=17)
+    rng = np.random.default_rng(len(counts))
+    sc["light_tris"] = sc["light_tris"][:sum(counts)]
+    sc["light_count"] = np.array(counts, np.uint32)
+    sc["light_first"] = (np.cumsum(counts) - counts).astype(np.uint32)
+    sc["light_emission"] = rng.uniform(1, 9, (len(counts), 3)).astype(np.float32)
+    flags = FLAG_NEE | FLAG_RIS
+    tr = Tracer(sc, cuda, max_depth=3, seed=4)
+    far = dict(sc, light_tris=np.concatenate([np.zeros(w * h, np.uint32), sc["light_tris"]]),
+               light_first=sc["light_first"] + np.uint32(w * h))
+    ref = Tracer(far, cuda, max_depth=3, seed=4)
+    for _ in range(2):
+        tr.render(1, flags)
+        ref.render(1, flags)
+        np.testing.assert_array_equal(tr.image64().cpu().numpy(), ref.image64().cpu().numpy())
+        tr.light_tris.copy_(tr.light_tris.flip(0))
+        ref.light_tris[w * h:] = tr.light_tris
+
+
 @pytest.mark.parametrize("grid,w,h", [(1, 40, 40), (16, 33, 20), (17, 33, 20), (2, 1100, 1)])
 def test_emitter_gradients_add_up(cuda, grid, w, h):
     """The image is linear in the emitters' radiances, so gradients times radiances add up to the
