@@ -44,23 +44,17 @@ namespace rtpg {
 constexpr int kTV = 10;  // trace vertices per path (kTraceVertexSize, OPX7/CMakeLists.txt:90)
 constexpr int kTB = 128;
 
-// What a light sample reads, packed for 32-byte loads (RIS draws 32 lights per shading point, every
-// lane another one; a load instruction costs a cycle per lane whatever its width): the mesh, then
-// the triangle's vertices, its unit normal and half its cross length (the area MeshLight::Sample
-// weighs by) from the frame of the triangle.  Against one index, vertex and normal component at a
-// time: 1.05 M-triangle hash-grid render (1280 x 720, 4096 lights) 207 -> 196 ms, learned guide
-// (640 x 360) 15.7 -> 14.7 ms.  With a few lights the lanes read the same words and there is nothing
-// to gain: Cornell box (2 light triangles, 512 x 512) 25.5 -> 26.2 ms, so flat scenes stay unpacked.
-struct __align__(32) LightMesh {
-    uint32_t first, count;  // its triangles in light_tri
-    float emission[3];
-    uint32_t pad[3];
-};
+// What a light sample reads, packed for two 32-byte loads: the triangle's vertices, its unit normal
+// and half its cross length (the area MeshLight::Sample weighs by) from the frame of the triangle,
+// and the radiance of its mesh.  RIS draws 32 lights per shading point, every lane another one: a
+// load instruction costs a cycle per lane whatever its width, and lights past the L1 come from the
+// L2 a sector at a time.  1.05 M-triangle hash-grid render (1280 x 720, 4096 lights): one index,
+// vertex and normal component at a time 207 ms, packed apart from the radiance 195.6, packed 195.0;
+// learned guide (640 x 360) 15.7, 14.65 and 14.45 ms.
 struct __align__(32) LightTri {
-    float v[9], n[3], area;
-    uint32_t pad[3];
+    float v[9], n[3], area, emission[3];
 };
-static_assert(sizeof(LightMesh) == 32 && sizeof(LightTri) == 64, "whole sectors");
+static_assert(sizeof(LightTri) == 64, "two sectors");
 
 struct TracerDev {
     SceneDev scene;
@@ -71,9 +65,10 @@ struct TracerDev {
     const Material* mats;
     const float* const* tex;  // per texture: RGB float, tex_wh[t] = (w, h)
     const uint2* tex_wh;
-    const LightMesh* light_mesh;
-    const uint32_t* light_tris;  // triangle of every light entry
-    const LightTri* light_tri;   // their packed copies, or null (pack_lights)
+    const uint32_t* light_tris;
+    const uint2* light_mesh;  // (first, count) into light_tris
+    const float3* light_emit;
+    const LightTri* light_tri;  // packed copies of the entries, or null (pack_lights)
     uint32_t light_count;
     uint32_t num_materials;
     float3 eye, cu, cv, cw, bg;
@@ -195,27 +190,19 @@ struct LightSample {
 };
 // MeshLightList::Sample -> MeshLight::Sample (SimpleKernel.h:81-98, 114-120): mesh and
 // triangle by next() % count, barycentrics by random_in_unit_triangle.
-// PACKED: the mesh in one load, and the triangles from T.light_tri where that is set.
+// PACKED: the triangle from T.light_tri where that is set.
 template <bool PACKED>
 __device__ __forceinline__ LightSample sample_light(const TracerDev& T, float3 p_in, uint32_t& rng) {
     const uint32_t mi = PACKED ? mod_u32(xs32_next(rng), T.light_count) : xs32_next(rng) % T.light_count;
-    uint32_t w[16], count;
+    const uint2 mesh = T.light_mesh[mi];
+    const uint32_t k = mesh.x + (PACKED ? mod_u32(xs32_next(rng), mesh.y) : xs32_next(rng) % mesh.y);
     float t[16];  // a LightTri
-    float3 emission;
-    if (PACKED) {
-        ld32(T.light_mesh + mi, w);
-        count = w[1];
-        emission = f3(__uint_as_float(w[2]), __uint_as_float(w[3]), __uint_as_float(w[4]));
-    } else {
-        w[0] = T.light_mesh[mi].first;
-        count = T.light_mesh[mi].count;
-    }
-    const uint32_t k = w[0] + (PACKED ? mod_u32(xs32_next(rng), count) : xs32_next(rng) % count);
     if (PACKED && T.light_tri) {
+        uint32_t w[16];
         ld32(T.light_tri + k, w);
         ld32(reinterpret_cast<const char*>(T.light_tri + k) + 32, w + 8);
 #pragma unroll
-        for (int j = 0; j < 13; ++j) t[j] = __uint_as_float(w[j]);
+        for (int j = 0; j < 16; ++j) t[j] = __uint_as_float(w[j]);
     } else {
         const uint32_t ti = min(T.light_tris[k], T.scene.ntris - 1);
         const float* tv = T.tri_v + 9 * size_t(ti);
@@ -223,6 +210,7 @@ __device__ __forceinline__ LightSample sample_light(const TracerDev& T, float3 p
         for (int j = 0; j < 9; ++j) t[j] = tv[j];
         const float4 f0 = T.tri_frame[ti].fr[0];  // unit3(cross(v1 - v0, v2 - v0)), half its length
         t[9] = f0.x; t[10] = f0.y; t[11] = f0.z; t[12] = f0.w;
+        if (PACKED) t[13] = T.light_emit[mi].x, t[14] = T.light_emit[mi].y, t[15] = T.light_emit[mi].z;
     }
     const float3 v0 = f3(t[0], t[1], t[2]), v1 = f3(t[3], t[4], t[5]), v2 = f3(t[6], t[7], t[8]);
     const float r0 = rnd1(rng);
@@ -234,10 +222,9 @@ __device__ __forceinline__ LightSample sample_light(const TracerDev& T, float3 p
     l.pos = p;
     l.dist = len3(d);
     l.dir = unit3(d);
-    if (!PACKED) emission = f3(T.light_mesh[mi].emission[0], T.light_mesh[mi].emission[1], T.light_mesh[mi].emission[2]);
-    l.emission = emission;
+    l.emission = PACKED ? f3(t[13], t[14], t[15]) : T.light_emit[mi];
     l.normal = f3(t[9], t[10], t[11]);
-    l.inv_pdf = t[12] * (float)count * (float)T.light_count;
+    l.inv_pdf = t[12] * (float)mesh.y * (float)T.light_count;
     l.mesh = mi;
     return l;
 }
@@ -1036,17 +1023,18 @@ __global__ void k_tri_frames(const float* __restrict__ tri_v, uint32_t n, TriFra
     }
 }
 
-// the packed triangles of the lights: entry k from triangle index[k] (clamped to the scene)
-__global__ void k_light_tris(const float* __restrict__ tri_v, const TriFrame* __restrict__ frame, uint32_t ntris,
-                             const uint32_t* __restrict__ index, uint32_t n, LightTri* __restrict__ out) {
+// the packed lights: entry k from triangle light_tris[k] (clamped to the scene) and its mesh
+__global__ void k_light_tris(TracerDev T, const uint32_t* __restrict__ mesh_of, uint32_t n, LightTri* __restrict__ out) {
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
-        const uint32_t ti = min(index[k], ntris - 1);
+        const uint32_t ti = min(T.light_tris[k], T.scene.ntris - 1), mi = mesh_of[k];
+        if (mi >= T.light_count) continue;  // of no mesh
         LightTri t;
-        for (int j = 0; j < 9; ++j) t.v[j] = tri_v[9 * size_t(ti) + j];
-        const float4 f = frame[ti].fr[0];
+        for (int j = 0; j < 9; ++j) t.v[j] = T.tri_v[9 * size_t(ti) + j];
+        const float4 f = T.tri_frame[ti].fr[0];
+        const float3 e = T.light_emit[mi];
         t.n[0] = f.x; t.n[1] = f.y; t.n[2] = f.z;
         t.area = f.w;
-        t.pad[0] = t.pad[1] = t.pad[2] = 0;
+        t.emission[0] = e.x; t.emission[1] = e.y; t.emission[2] = e.z;
         out[k] = t;
     }
 }
@@ -1072,8 +1060,9 @@ struct rtpg_tracer {
     std::vector<void*> allocs;
     // host copies for parameter updates and the adjoint
     std::vector<Material> hmats;
-    std::vector<LightMesh> hlight;
-    LightTri* light_tri = nullptr;  // num_light_tris entries, written by pack_lights
+    std::vector<float3> hemit;
+    LightTri* light_tri = nullptr;  // num_light_tris entries, written by pack_lights; null: never packed
+    uint32_t* light_mesh_of = nullptr;  // mesh of every entry
     uint32_t num_light_tris = 0;
     std::vector<int32_t> light_mat;  // material of every light mesh (-1: its triangles differ)
     bool light_mat_shared = false;   // some material belongs to two light meshes
@@ -1270,10 +1259,11 @@ int rtpg_tracer_create(rtpg_scene* scene, const float* tri_vertices, const uint3
     h->seed = D.seed ? D.seed : 1;
     const size_t P = T.npath;
     Material* mats = nullptr;
-    LightMesh* lmesh = nullptr;
+    uint2* lmesh = nullptr;
+    float3* lemit = nullptr;
     int r;
     if ((r = h->alloc(&mats, num_materials)) || (r = h->alloc(&lmesh, std::max(num_light_meshes, 1u))) ||
-        (r = h->alloc(&T.org, P)) ||
+        (r = h->alloc(&lemit, std::max(num_light_meshes, 1u))) || (r = h->alloc(&T.org, P)) ||
         (r = h->alloc(&T.dir, P)) || (r = h->alloc(&T.thr, P)) || (r = h->alloc(&T.col, P)) ||
         (r = h->alloc(&T.rng, P)) || (r = h->alloc(&T.depth, P)) ||
         (r = h->alloc(&T.hflags, P)) || (r = h->alloc(&T.queue[0], P)) ||
@@ -1287,6 +1277,7 @@ int rtpg_tracer_create(rtpg_scene* scene, const float* tri_vertices, const uint3
         return r;
     }
     std::vector<Material> hm(num_materials);
+    std::vector<float3> he(std::max(num_light_meshes, 1u));
     for (uint32_t i = 0; i < num_materials; ++i) {
         const rtpg_material& s = host_materials[i];
         Material& m = hm[i];
@@ -1299,19 +1290,21 @@ int rtpg_tracer_create(rtpg_scene* scene, const float* tri_vertices, const uint3
         m.tex = s.diffuse_texture;
         m.pad[0] = m.pad[1] = m.pad[2] = 0;
     }
-    std::vector<LightMesh> hl(std::max(num_light_meshes, 1u), LightMesh{0, 1, {0.f, 0.f, 0.f}, {0, 0, 0}});
+    std::vector<uint2> hl(std::max(num_light_meshes, 1u), make_uint2(0, 1));
     for (uint32_t i = 0; i < num_light_meshes; ++i) {
-        hl[i].first = host_light_mesh_first[i];
-        hl[i].count = host_light_mesh_count[i];
+        hl[i] = make_uint2(host_light_mesh_first[i], host_light_mesh_count[i]);
         if (!host_light_mesh_count[i]) {
             delete h;
             return fail(RTPG_EINVAL, "rtpg_tracer_create: empty light mesh %u", i);
         }
-        for (int c = 0; c < 3; ++c) hl[i].emission[c] = host_desc->light_emission ? host_desc->light_emission[3 * i + c] : 0.f;
+        he[i] = make_float3(host_desc->light_emission ? host_desc->light_emission[3 * i] : 0.f,
+                            host_desc->light_emission ? host_desc->light_emission[3 * i + 1] : 0.f,
+                            host_desc->light_emission ? host_desc->light_emission[3 * i + 2] : 0.f);
     }
     cudaError_t e;
     if ((e = cudaMemcpy(mats, hm.data(), sizeof(Material) * num_materials, cudaMemcpyHostToDevice)) ||
-        (e = cudaMemcpy(lmesh, hl.data(), sizeof(LightMesh) * hl.size(), cudaMemcpyHostToDevice))) {
+        (e = cudaMemcpy(lmesh, hl.data(), sizeof(uint2) * hl.size(), cudaMemcpyHostToDevice)) ||
+        (e = cudaMemcpy(lemit, he.data(), sizeof(float3) * he.size(), cudaMemcpyHostToDevice))) {
         delete h;
         return fail(RTPG_ECUDA, "rtpg_tracer_create: %s", cudaGetErrorString(e));
     }
@@ -1319,25 +1312,21 @@ int rtpg_tracer_create(rtpg_scene* scene, const float* tri_vertices, const uint3
     T.num_materials = num_materials;
     for (uint32_t i = 0; i < num_materials; ++i) h->mat_tex.push_back(host_materials[i].diffuse_texture);
     T.light_mesh = lmesh;
+    T.light_emit = lemit;
     T.light_tris = light_tris;
     T.light_count = num_light_meshes;
     // light mesh <-> emissive material, for emitter parameters and their gradients
     h->hmats = hm;
-    h->hlight = hl;
+    h->hemit = he;
     {
         std::vector<int32_t> ml(num_materials, -1);
         h->light_mat.assign(num_light_meshes, -1);
         uint32_t nlt = 0;
-        for (uint32_t i = 0; i < num_light_meshes; ++i) nlt = std::max(nlt, hl[i].first + hl[i].count);
+        for (uint32_t i = 0; i < num_light_meshes; ++i) nlt = std::max(nlt, hl[i].x + hl[i].y);
         std::vector<uint32_t> lt(nlt), tm;
         if (nlt && (e = cudaMemcpy(lt.data(), light_tris, 4ull * nlt, cudaMemcpyDeviceToHost))) {
             delete h;
             return fail(RTPG_ECUDA, "rtpg_tracer_create: %s", cudaGetErrorString(e));
-        }
-        h->num_light_tris = nlt;
-        if (nlt <= T.npath && (r = h->alloc(&h->light_tri, std::max(nlt, 1u)))) {
-            delete h;
-            return r;
         }
         const uint32_t nt = T.scene.ntris;
         tm.resize(nt);
@@ -1347,8 +1336,8 @@ int rtpg_tracer_create(rtpg_scene* scene, const float* tri_vertices, const uint3
         }
         for (uint32_t i = 0; i < num_light_meshes; ++i) {
             int32_t mat = -1;
-            for (uint32_t k = 0; k < hl[i].count; ++k) {
-                const uint32_t t = lt[hl[i].first + k];
+            for (uint32_t k = 0; k < hl[i].y; ++k) {
+                const uint32_t t = lt[hl[i].x + k];
                 const int32_t mk = t < nt ? (int32_t)std::min(tm[t], num_materials - 1) : -1;
                 mat = (k == 0) ? mk : (mat == mk ? mat : -1);
             }
@@ -1356,6 +1345,25 @@ int rtpg_tracer_create(rtpg_scene* scene, const float* tri_vertices, const uint3
             if (mat >= 0) {
                 if (ml[mat] >= 0 && ml[mat] != (int32_t)i) h->light_mat_shared = true;
                 ml[mat] = (int32_t)i;
+            }
+        }
+        // packed copies (pack_lights): where every entry belongs to one mesh at most
+        h->num_light_tris = nlt;
+        std::vector<uint32_t> mesh_of(nlt <= T.npath && !T.nflat ? nlt : 0, 0xffffffffu);
+        bool one_mesh = !mesh_of.empty();
+        for (uint32_t i = 0; i < num_light_meshes && one_mesh; ++i)
+            for (uint32_t k = 0; k < hl[i].y; ++k) {
+                one_mesh &= mesh_of[hl[i].x + k] == 0xffffffffu;
+                mesh_of[hl[i].x + k] = i;
+            }
+        if (one_mesh) {
+            if ((r = h->alloc(&h->light_mesh_of, nlt)) || (r = h->alloc(&h->light_tri, nlt))) {
+                delete h;
+                return r;
+            }
+            if ((e = cudaMemcpy(h->light_mesh_of, mesh_of.data(), 4ull * nlt, cudaMemcpyHostToDevice))) {
+                delete h;
+                return fail(RTPG_ECUDA, "rtpg_tracer_create: %s", cudaGetErrorString(e));
             }
         }
         if (h->light_mat_shared) std::fill(ml.begin(), ml.end(), -1);
@@ -1441,15 +1449,16 @@ static int check_render(rtpg_tracer* h, uint32_t flags, const char* fn) {
 }
 
 // The lights packed for the render's samples, anew for each render: the arrays are the caller's.
-// Where a sample reads them often enough: RIS (one light sample per shading point otherwise), waves
-// with a launch per bounce, and no more light triangles than paths.
+// Where they are read often enough: RIS (one light sample per shading point otherwise), waves with a
+// launch per bounce, and no more light triangles than paths (rtpg_tracer_create keeps no room else).
+// Not in flat scenes: with a few lights the lanes read the same words (2 light triangles, Cornell box
+// 512 x 512: 25.5 ms indexed, 26.2 ms packed).
 static void pack_lights(rtpg_tracer* h, cudaStream_t st) {
     TracerDev& T = h->dev;
     T.light_tri = nullptr;
-    if (!(T.flags & RTPG_TRACE_FLAG_RIS) || T.nflat || whole_paths(T) || !h->light_tri || !h->num_light_tris) return;
+    if (!(T.flags & RTPG_TRACE_FLAG_RIS) || whole_paths(T) || !h->light_tri) return;
     T.light_tri = h->light_tri;
-    k_light_tris<<<grid_for(h->num_light_tris, 256, 8), 256, 0, st>>>(T.tri_v, T.tri_frame, T.scene.ntris, T.light_tris,
-                                                                      h->num_light_tris, h->light_tri);
+    k_light_tris<<<grid_for(h->num_light_tris, 256, 8), 256, 0, st>>>(T, h->light_mesh_of, h->num_light_tris, h->light_tri);
 }
 
 // `spp` waves with the flags and guide views already in h->dev.  A captured wave bakes in
@@ -1653,10 +1662,10 @@ int rtpg_tracer_set_light_emission(rtpg_tracer* h, const float* host_rgb, uint32
     for (uint32_t i = 0; i < num_lights; ++i) {
         if (h->light_mat[i] < 0)
             return fail(RTPG_EINVAL, "rtpg_tracer_set_light_emission: light mesh %u has triangles of several materials", i);
-        for (int c = 0; c < 3; ++c) h->hlight[i].emission[c] = host_rgb[3 * i + c];
-        h->hmats[h->light_mat[i]].emission = make_float3(host_rgb[3 * i], host_rgb[3 * i + 1], host_rgb[3 * i + 2]);
+        h->hemit[i] = make_float3(host_rgb[3 * i], host_rgb[3 * i + 1], host_rgb[3 * i + 2]);
+        h->hmats[h->light_mat[i]].emission = h->hemit[i];
     }
-    RTPG_CUDA(cudaMemcpy(const_cast<LightMesh*>(h->dev.light_mesh), h->hlight.data(), sizeof(LightMesh) * num_lights,
+    RTPG_CUDA(cudaMemcpy(const_cast<float3*>(h->dev.light_emit), h->hemit.data(), sizeof(float3) * num_lights,
                          cudaMemcpyHostToDevice));
     RTPG_CUDA(cudaMemcpy(const_cast<Material*>(h->dev.mats), h->hmats.data(), sizeof(Material) * h->hmats.size(),
                          cudaMemcpyHostToDevice));

@@ -228,6 +228,23 @@ def test_packed_lights_sample_like_indexed_ones(cuda, counts):
         ref.light_tris[w * h:] = tr.light_tris
 
 
+def test_lights_that_share_triangles(cuda):
+    """Two meshes over the same entries, each with its own radiance: as the same entries twice."""
+    from rtlib_b200 import scenes
+    from rtlib_b200.tracer import FLAG_NEE, FLAG_RIS, Tracer
+    w, h = 148 * 7, 129
+    sc = scenes.cornell_box(w, h, light_grid=17)
+    lt = sc["light_tris"]
+    sc["light_emission"] = np.array([[9, 1, 1], [1, 1, 9]], np.float32)
+    sc["light_count"] = np.full(2, len(lt), np.uint32)
+    img = []
+    for tris, first in ((lt, [0, 0]), (np.concatenate([lt, lt]), [0, len(lt)])):
+        tr = Tracer(dict(sc, light_tris=tris, light_first=np.array(first, np.uint32)), cuda, max_depth=3, seed=4)
+        tr.render(1, FLAG_NEE | FLAG_RIS)
+        img.append(tr.image64().cpu().numpy())
+    np.testing.assert_array_equal(img[0], img[1])
+
+
 @pytest.mark.parametrize("grid,w,h", [(1, 40, 40), (16, 33, 20), (17, 33, 20), (2, 1100, 1)])
 def test_emitter_gradients_add_up(cuda, grid, w, h):
     """The image is linear in the emitters' radiances, so gradients times radiances add up to the
