@@ -729,7 +729,7 @@ def bench_occluded_ours(args, rank, world):
                      "note": "bounce = BVH closest hit over 1M triangles + shading + RIS over 32 light samples + "
                              "one shadow ray; bound by traversal latency and issue"},
         "clocks": clk,
-        "gpu_launches": ((1 + O_DEPTH + 1) * samples + _recording_launches(O_BUDGET, 1)) * args.steps,
+        "gpu_launches": ((1 + O_DEPTH + 2) * samples + _recording_launches(O_BUDGET, 1)) * args.steps,
         "counters_per_step": cnt,
         "unguided_nee_ris_Mpaths_s": O_W * O_H * samples / (plain_ms * 1e-3) / 1e6,
         "grid_cells": cells, "spp_per_step": samples,
@@ -749,7 +749,7 @@ HG_LOOKUP_BYTES, HG_RECORD_BYTES, HG_SAMPLE_BYTES = 16, 16, 24
 
 
 def _hg_cell_bytes(level=HG_LEVEL):
-    """Algorithmic bytes of one cell's pyramid build: every int64 leaf read and zeroed (16 B)
+    """Algorithmic bytes of one recorded cell's pyramid build: every int64 leaf read and zeroed (16 B)
     and every float of the (4^(L+1)-1)/3-entry pyramid written (4 B)."""
     return (1 << (2 * level)) * 16 + (((1 << (2 * (level + 1))) - 1) // 3) * 4
 
@@ -827,6 +827,7 @@ def bench_hashgrid_ours(args, rank, world):
     ms = _max_over_ranks(statistics.mean(e[0].elapsed_time(e[-1]) for e in ev), world, dev)
     found = int((slot_q >= 0).sum().item())
     cells = int(torch.unique(slot_p).numel())
+    built = int(torch.unique(slot_q[slot_q >= 0]).numel())  # the cells with records
     grid_status = grid.status()  # RTPG_STATUS_HASH_FULL if a bucket of 32 overflowed
     assert trees.status() == 0
 
@@ -856,7 +857,7 @@ def bench_hashgrid_ours(args, rank, world):
     ops = (HG_POINTS + 3 * HG_QUERIES) * world
     peak, peak_kind = _peaks()
     gbs = lambda b, t: b / (t * 1e-3) / 1e9
-    build_bytes = HG_SLOTS * _hg_cell_bytes()
+    build_bytes = built * _hg_cell_bytes()
     achieved = gbs(build_bytes, ph["build"])
     return {
         "metric": "hash-grid guide insert+lookup+record+build+sample throughput (config-3 grid)",
@@ -868,9 +869,8 @@ def bench_hashgrid_ours(args, rank, world):
                      "traffic": _traffic("k_mqt_build"), "algorithmic_bytes_per_launch": build_bytes,
                      "launch_ms": ph["build"]},
         "clocks": clk,
-        # clear 1 + insert (prepare, 2 sorts, heads, assign, scatter) + swap 1; lookup 1; record 1;
-        # build 1; sample 1 (cub sorts counted as one launch each)
-        "gpu_launches": 12 * args.steps,
+        # insert 4 (stage, chain, rank, give); lookup, record, build, sample 1 each
+        "gpu_launches": 8 * args.steps,
         "phases": {"insert_Mpts_s": HG_POINTS / (ph["insert"] * 1e-3) / 1e6,
                    "lookup_Mq_s": HG_QUERIES / (ph["lookup"] * 1e-3) / 1e6,
                    "lookup_GBs": gbs(HG_LOOKUP_BYTES * HG_QUERIES, ph["lookup"]),
@@ -1108,7 +1108,8 @@ def bench_mlp_ours(args, rank, world):
         "inference": {"Msamples_s": MLP_N_EVAL / (e_ms * 1e-3) / 1e6, "ms": e_ms,
                       "tflops": MLP_FWD_FLOP * MLP_N_EVAL / (e_ms * 1e-3) / 1e12},
         "clocks": clk,
-        "gpu_launches": (3 * steps + 1) * args.steps,
+        # weight sums of the epoch 1; gradient and Adam per minibatch; evaluation 1
+        "gpu_launches": (2 * steps + 2) * args.steps,
     }
 
 
@@ -1159,7 +1160,7 @@ def bench_adjoint(args):
             "vector_rel_err": float(np.linalg.norm(adj - fd) / np.linalg.norm(fd)),
             "forward_Mpaths_s": paths / (r["forward_ms"] * 1e-3) / 1e6,
             "adjoint_Mpaths_s": paths / (r["adjoint_ms"] * 1e-3) / 1e6,
-            "note": "adjoint = one primal and one adjoint replay wave per sample", "clocks": clk}
+            "note": "adjoint = one launch per sample: a primal pass and its replay", "clocks": clk}
 
 
 # ---------------------------------------------------------------------------- plumbing

@@ -6,7 +6,7 @@
 //     reports: a leaf's box must pass box_hit, and of triangles at exactly the same distance
 //     the one a near-first walk of this hierarchy meets first wins;
 //   - the hierarchy that rays walk: eight children per node, their boxes quantised to eight bits
-//     per plane (see WideNode), collapsed from the binary one.
+//     per plane (see WideNode), collapsed from a binary hierarchy that clustering builds (k_ploc_*).
 #pragma once
 #include "common.cuh"
 
