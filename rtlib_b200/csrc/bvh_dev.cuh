@@ -181,7 +181,10 @@ __device__ __forceinline__ float min3_nan(float a, float b, float c) {  // NaN i
 // same roundings, half the multiply-adds to issue.  u >= 0, v >= 0 and u + v <= 1 are one comparison
 // of the least of u, v and 1 - (u + v), whose sign is exact.  k_bounce of the guided Cornell render
 // (36 triangles, 512 launches at 512 x 512): 25.0 -> 22.1 ms; unrolled by 1, 3, 4: 24.9, 22.4, 22.6.
-template <bool ANY>
+// LANES > 1: that many neighbouring lanes hold the same ray and test every LANES-th pair each; all of
+// them return the hit.  The pairs come from memory then (the constant bank serves one address at a
+// time).
+template <bool ANY, int LANES = 1>
 __device__ __forceinline__ Hit flat_trace(const FlatPair* pairs, uint32_t npairs, float ox, float oy, float oz, float dx,
                                           float dy, float dz, float tmin, float tmax) {
     Hit h;
@@ -192,7 +195,7 @@ __device__ __forceinline__ Hit flat_trace(const FlatPair* pairs, uint32_t npairs
     const unsigned long long qx = pack2(dx, dx), qy = pack2(dy, dy), qz = pack2(dz, dz);
     const unsigned long long one = pack2(1.0f, 1.0f), minus = pack2(-1.0f, -1.0f);
 #pragma unroll 2
-    for (uint32_t k = 0; k < npairs; ++k) {
+    for (uint32_t k = LANES > 1 ? threadIdx.x % LANES : 0; k < npairs; k += LANES) {
         const FlatPair& p = pairs[k];
         const float2 den = unpack2(fma2(p.r2[0], qx, fma2(p.r2[1], qy, mul2(p.r2[2], qz))));
         const float2 num = unpack2(fma2(p.r2[0], px, fma2(p.r2[1], py, fma2(p.r2[2], pz, p.r2[3]))));
@@ -211,15 +214,22 @@ __device__ __forceinline__ Hit flat_trace(const FlatPair* pairs, uint32_t npairs
             h.u = u.x;
             h.v = v.x;
             h.prim = 2 * k;
-            if (ANY) return h;
+            if (ANY) break;
         }
         if (inb & (tb > tmin) & (tb < h.t) & (tb > 0.0f)) {
             h.t = tb;
             h.u = u.y;
             h.v = v.y;
             h.prim = 2 * k + 1;
-            if (ANY) return h;
+            if (ANY) break;
         }
+    }
+    const uint32_t group = ((1u << (LANES % 32)) - 1u) << (threadIdx.x % 32 / LANES * LANES);
+#pragma unroll
+    for (int o = 1; o < LANES; o *= 2) {  // the nearest, of equal distances the lowest index
+        const float t = __shfl_xor_sync(group, h.t, o), u = __shfl_xor_sync(group, h.u, o), v = __shfl_xor_sync(group, h.v, o);
+        const uint32_t prim = __shfl_xor_sync(group, h.prim, o);
+        if (t < h.t || (t == h.t && prim < h.prim)) h = Hit{t, u, v, prim};
     }
     return h;
 }

@@ -119,10 +119,10 @@ struct TracerDev {
 
 // closest hit (ANY = false) or any hit (ANY = true) in (tmin, tmax): the scene's triangles from
 // the kernel parameters when it is small (FLAT), else the BVH
-template <bool ANY, bool FLAT>
+template <bool ANY, bool FLAT, int LANES = 1>
 __device__ __forceinline__ Hit trace(const TracerDev& T, float ox, float oy, float oz, float dx, float dy, float dz,
                                      float tmin, float tmax) {
-    if (FLAT) return flat_trace<ANY>(T.ftri, T.nflat, ox, oy, oz, dx, dy, dz, tmin, tmax);
+    if (FLAT) return flat_trace<ANY, LANES>(LANES > 1 ? T.scene.flat : T.ftri, T.nflat, ox, oy, oz, dx, dy, dz, tmin, tmax);
     return bvh_trace<ANY>(T.scene, ox, oy, oz, dx, dy, dz, tmin, tmax);
 }
 
@@ -262,7 +262,7 @@ __device__ __forceinline__ uint32_t& kept_prim(const TracerDev& T, uint32_t d, u
     return row[p];
 }
 
-template <int G, bool FLAT, int HITS = kTrace>
+template <int G, bool FLAT, int HITS = kTrace, int LANES = 1>
 __device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, PathState& s, bool build, bool recording,
                                             bool& shadow, float3& L, Adjoint* adj = nullptr) {
     constexpr bool use_tree = G == kGuideTree, use_grid = G == kGuideGrid, adjoint = G == kAdjoint;
@@ -285,7 +285,7 @@ __device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, Path
         h.u = tuv.y;
         h.v = tuv.z;
     } else {
-        h = trace<false, FLAT>(T, org.x, org.y, org.z, in_dir.x, in_dir.y, in_dir.z, 0.0001f, 1.0e20f);
+        h = trace<false, FLAT, LANES>(T, org.x, org.y, org.z, in_dir.x, in_dir.y, in_dir.z, 0.0001f, 1.0e20f);
     }
     const size_t vi = size_t(d < kTV ? d : 0) * T.npath + p;
     bool pend = false;
@@ -593,7 +593,7 @@ __device__ __forceinline__ bool bounce_path(const TracerDev& T, uint32_t p, Path
     if (pend) {
         shadow = true;
         lit = HITS == kReuse ? kept >> 31
-                             : trace<true, FLAT>(T, position.x, position.y, position.z, sdir.x, sdir.y, sdir.z, 0.0001f, sdist)
+                             : trace<true, FLAT, LANES>(T, position.x, position.y, position.z, sdir.x, sdir.y, sdir.z, 0.0001f, sdist)
                                        .prim == 0xffffffffu;
         if (lit) L = L + scontrib;
     }
@@ -777,17 +777,17 @@ __device__ __forceinline__ void finish_path(const TracerDev& T, uint32_t p, floa
     T.seeds[p] = rng;
 }
 
-// A whole path per thread: camera ray, bounces and accumulation in one kernel, the state in
+// A whole path per thread, or per LANES of them (kPathLanes): camera ray, bounces and accumulation in one kernel, the state in
 // registers.  Where the image is small the launches of a wave of bounces, each a latency-bound tail
 // on a part of the SMs, take most of its time; a path that ends leaves its lane idle instead of
 // being replaced.  Passes of one sample of the Cornell box, a launch per bounce -> here: 96 x 54
 // 130 -> 90 us, 256 x 256 150 -> 116 us, 400 x 400 208 -> 220 us.
-template <int G, bool FLAT>
+template <int G, bool FLAT, int LANES>
 __global__ void __launch_bounds__(kTB, 8) k_path(TracerDev T) {
     grid_dependency_wait();
     const bool build = (T.flags & RTPG_TRACE_FLAG_BUILD) != 0;
     const bool recording = (G == kGuideTree || G == kGuideGrid) && !(T.flags & RTPG_TRACE_FLAG_FINAL);
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) / LANES;
     bool alive = p < T.npath;
     PathState s;
     float3 col = f3(0.0f, 0.0f, 0.0f);
@@ -797,20 +797,22 @@ __global__ void __launch_bounds__(kTB, 8) k_path(TracerDev T) {
         if (alive) {
             bool shadow = false;
             float3 L;
-            alive = bounce_path<G, FLAT>(T, p, s, build, recording, shadow, L);
+            alive = bounce_path<G, FLAT, kTrace, LANES>(T, p, s, build, recording, shadow, L);
             col = col + L;
             ++visits;
             shadows += shadow;
         }
         __syncwarp();
     }
+    const bool first = threadIdx.x % LANES == 0;
+    if (!first) visits = shadows = 0;
     visits = __reduce_add_sync(0xffffffffu, visits);
     shadows = __reduce_add_sync(0xffffffffu, shadows);
     if ((threadIdx.x & 31) == 0) {
         atomicAdd(T.counters, (unsigned long long)visits);
         atomicAdd(T.counters + 1, (unsigned long long)shadows);
     }
-    if (p >= T.npath) return;
+    if (p >= T.npath || !first) return;
     T.depth[p] = s.depth;  // for the commit
     finish_path(T, p, col, s.rng);
 }
@@ -1191,10 +1193,19 @@ static int timed_wave(rtpg_tracer* h, cudaStream_t st) {
 // ms, 130 k 29.2 -> 27.1 ms.  The learned guide needs its network between bounces.
 constexpr uint32_t kWholePaths = kSMs * 7 * kTB;
 static bool whole_paths(const TracerDev& T) { return T.npath <= kWholePaths && guide_of(T.flags) != kGuideMlp; }
+// In flat scenes of so few paths that an SM holds ten warps of them at most, four lanes share a path:
+// each tests a quarter of the triangles, all of them shade (what else would these schedulers issue).
+// One sample of the Cornell box with a lane a path -> four, NEE and RIS with 32 candidates: 256 paths
+// 68.8 -> 37.1 us and 284 -> 242, 5184 69.9 -> 39.2 and 288 -> 257, 12,288 71.7 -> 43.6 and 289 -> 281,
+// 19,200 74.0 -> 53.6 but 303 -> 342.  Eight lanes: 37.0 and 257 at 5184 paths, 51.5 and 368 at 12,288.
+constexpr int kPathLanes = 4;
+constexpr uint32_t kSplitPaths = kSMs * 80;
 template <int G>
 static void launch_path_of(const TracerDev& T, cudaStream_t st) {
-    if (T.nflat) (void)launch_dependent(k_path<G, true>, bounce_grid(T), kTB, 0, st, T);
-    else (void)launch_dependent(k_path<G, false>, bounce_grid(T), kTB, 0, st, T);
+    if (T.nflat && T.npath <= kSplitPaths)
+        (void)launch_dependent(k_path<G, true, kPathLanes>, (T.npath * kPathLanes + kTB - 1) / kTB, kTB, 0, st, T);
+    else if (T.nflat) (void)launch_dependent(k_path<G, true, 1>, bounce_grid(T), kTB, 0, st, T);
+    else (void)launch_dependent(k_path<G, false, 1>, bounce_grid(T), kTB, 0, st, T);
 }
 static void launch_wave(rtpg_tracer* h, cudaStream_t st) {
     TracerDev& T = h->dev;

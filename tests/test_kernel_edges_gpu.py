@@ -201,6 +201,34 @@ def test_whole_path_waves_equal_bounce_waves(cuda, w, h, spp):
     assert cnt == ref.counters()
 
 
+@pytest.mark.parametrize("w,h,ris", [(3, 1, 1), (9, 1, 0), (148, 80, 0), (149, 80, 1)])
+@pytest.mark.parametrize("ntri", [36, 35, 1])
+def test_lanes_that_share_a_path(cuda, w, h, ris, ntri):
+    """Both sides of the limit of four lanes per path (80 paths per SM), an odd number of triangles and
+    fewer pairs than lanes, coincident triangles: images, depths and counters as from a launch per
+    bounce."""
+    from rtlib_b200 import scenes
+    from rtlib_b200.tracer import FLAG_NEE, FLAG_RIS, Tracer
+    sc = scenes.cornell_box(w, h)
+    sc["tri_v"] = sc["tri_v"].copy()
+    sc["tri_v"][20:24] = sc["tri_v"][4:8]  # equal distances: the lowest index wins
+    light = int(sc["light_tris"][0])
+    keep = np.r_[np.arange(ntri - 1), light]
+    sc = dict(sc, tri_v=sc["tri_v"][keep], tri_mat=sc["tri_mat"][keep], tri_uv=sc["tri_uv"][keep],
+              light_tris=np.array([ntri - 1], np.uint32), light_first=np.zeros(1, np.uint32),
+              light_count=np.ones(1, np.uint32))
+    flags = FLAG_NEE | (FLAG_RIS if ris else 0)
+    got = []
+    for timing in (False, True):  # measured waves are always a launch per bounce
+        tr = Tracer(sc, cuda, max_depth=6, width=w, height=h, seed=8)
+        tr.set_timing(timing)
+        tr.render(3, flags)
+        got.append((tr.image64().cpu().numpy(), tr.path_depths().cpu().numpy(), tr.counters()))
+    np.testing.assert_array_equal(got[0][0], got[1][0])
+    np.testing.assert_array_equal(got[0][1], got[1][1])
+    assert got[0][2] == got[1][2]
+
+
 @pytest.mark.parametrize("counts", [[578], [1, 6, 571], [2] * 256 + [3, 63], [1] * 64])
 def test_packed_lights_sample_like_indexed_ones(cuda, counts):
     """Light meshes of one and of many triangles, powers of two and not.  Entries in front of the
