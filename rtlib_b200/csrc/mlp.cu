@@ -8,6 +8,8 @@
 // the mixture to the recorded radiance distribution).
 #include <algorithm>
 #include <cmath>
+#include <map>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -84,21 +86,23 @@ __global__ void __launch_bounds__(kMlpThreads, 4) k_mlp_eval(MlpDev P, int64_t n
 
 // ------------------------------------------------------------------ training
 // d(loss)/d(raw outputs) of one record: loss = -w log q(wi) (scaled by inv_wsum), q the mixture
-// of mlp_head.  Each of the record's two threads forms its half of the lobes; q is the sum of both
-// halves, exchanged through s_q.  The thread's 20 gradients go to g; returns -log q.
-__device__ __forceinline__ float head_grad(const float* o, bool hi, float3 wi, float scale, float* s_q, float* g) {
+// of mlp_head_half's lobes.  Each of the record's two threads forms its half of the lobes and hands their
+// terms to the other through s_f (lobe-major): both add the eight terms of q in order.  The thread's
+// 20 gradients go to g; returns -log q.
+__device__ __forceinline__ float head_grad(const float* o, bool hi, float3 wi, float scale, float (*s_f)[kMlpTile], float* g) {
     VmfLobe L[kMlpLobes / 2];
     mlp_head_half(o, hi, L);
+    const int row = threadIdx.x & (kMlpTile - 1);
     float fk[kMlpLobes / 2], q = 0.0f;
 #pragma unroll
     for (int k = 0; k < kMlpLobes / 2; ++k) {
         fk[k] = vmf_pdf(L[k], wi);
-        q += L[k].weight * fk[k];
+        s_f[hi ? k + 4 : k][row] = __fmul_rn(L[k].weight, fk[k]);
     }
-    s_q[threadIdx.x] = q;
     __syncthreads();
-    const int row = threadIdx.x & (kMlpTile - 1);
-    q = fmaxf(s_q[row] + s_q[row + kMlpTile], 1e-30f);
+#pragma unroll
+    for (int k = 0; k < kMlpLobes; ++k) q = __fadd_rn(q, s_f[k][row]);
+    q = fmaxf(q, 1e-30f);
 #pragma unroll
     for (int k = 0; k < kMlpLobes / 2; ++k) {
         const float r = L[k].weight * fk[k] / q;  // responsibility
@@ -122,16 +126,28 @@ __device__ __forceinline__ float head_grad(const float* o, bool hi, float3 wi, f
     return -__logf(q);
 }
 
+// Sum of the first `parts` floats of p, the same in every lane (fixed order).  The whole warp calls it.
+__device__ __forceinline__ float warp_sum_parts(const float* p, int parts) {
+    float s = 0.0f;
+    for (int k = threadIdx.x & 31; k < parts; k += 32) s += p[k];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
 // One pass over n records: forward, loss gradient, backward; dW of all layers accumulate in
-// TMEM across the CTA's tiles and are added to grads (fp32, [in][out] per layer) at the end.
+// TMEM across the CTA's tiles and go to the CTA's row of grad_rows (fp32, [in][out] per layer) at the
+// end, its share of the loss to loss_rows; k_mlp_adam or k_mlp_add_grads sums the rows.  wsum: the
+// minibatch's weight sum in wparts parts (k_wsum).  No sum depends on the order in which CTAs finish:
+// Adam divides a gradient by its own size, so what the order of float atomics left in the last bits
+// grew to 4e-4 of the parameters within 16 steps.
 // A minibatch gives each CTA one tile, so its time is that tile's chain of phases: features, eight
 // dependent MMA phases with an epilogue each, the gradient flush.  Launched as a dependent of the
 // previous step's Adam it forms the first tile's features, which do not depend on the weights, while
 // that still runs (records and wsum are ready before the first launch of a call).  16 steps of 16384
 // records: 574 us with 128 threads per tile and a memset, a weight sum and an Adam launched one after
 // the other around it, 320 us now.
-__global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t n, Records R, const float* wsum,
-                                                            float* __restrict__ grads, float* __restrict__ loss_sum) {
+__global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t n, Records R, const float* wsum, int wparts,
+                                                            float* __restrict__ grad_rows, float* __restrict__ loss_rows) {
     extern __shared__ __align__(128) uint8_t sm[];
     __nv_bfloat16* ws = reinterpret_cast<__nv_bfloat16*>(sm);
     __nv_bfloat16* x0 = reinterpret_cast<__nv_bfloat16*>(sm + kSmemW);
@@ -140,7 +156,8 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t 
     __nv_bfloat16* dy = reinterpret_cast<__nv_bfloat16*>(sm + kSmemW + kSmemX + 3 * kSmemH);
     uint64_t* mbar = reinterpret_cast<uint64_t*>(sm + kSmemW + kSmemX + 4 * kSmemH);
     uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + kSmemW + kSmemX + 4 * kSmemH + 8);
-    __shared__ float s_q[kMlpThreads];
+    __shared__ float s_f[kMlpLobes][kMlpTile];
+    __shared__ float s_loss[kMlpTile / 32];
     grid_launch_dependents();
     const int t = threadIdx.x, row = t & (kMlpTile - 1);
     const bool hi = t >= kMlpTile;
@@ -148,10 +165,11 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t 
     if (t == 0) mbar_init(mbar, 1);
     const uint32_t sw = smem_u32(ws), sx = smem_u32(x0), sdy = smem_u32(dy);
     const uint32_t sh[3] = {smem_u32(hs[0]), smem_u32(hs[1]), smem_u32(hs[2])};
-    const float scale = (wsum && *wsum > 0.0f) ? 1.0f / *wsum : 0.0f;
+    const float total = warp_sum_parts(wsum, wparts);
+    const float scale = total > 0.0f ? 1.0f / total : 0.0f;
     // record weights are Monte Carlo estimates with a heavy tail: clamp at kWeightClamp times
     // their mean so that single rare paths do not dominate a step
-    const float wmax = (wsum && n > 0) ? kWeightClamp * (*wsum / (float)n) : 0.0f;
+    const float wmax = kWeightClamp * (total / (float)n);
     uint32_t phase = 0, tmem = 0;
     bool ok = true, first = true;
     float lsum = 0.0f;
@@ -194,7 +212,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t 
         {
             float o[kMlpOut], g[20];
             ld_row<kMlpOut>(tmem, kColD, o);
-            const float nl = head_grad(o, hi, wi, w * scale, s_q, g);
+            const float nl = head_grad(o, hi, wi, w * scale, s_f, g);
             if (w > 0.0f && !hi) lsum += w * nl;
             const int c0 = hi ? 20 : 0;
 #pragma unroll
@@ -243,10 +261,13 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t 
         first = false;
     }
     // flush dW^T (M = 64 rows in lanes 16w .. 16w+15 of warp w's quarter, the two warps of a quarter
-    // taking alternate column groups) into grads; after a wait gave up the accumulators are
-    // incomplete and nothing is flushed
+    // taking alternate column groups) into the CTA's row; after a wait gave up the accumulators are
+    // incomplete and the row is zero
     const bool done = mma_barrier(ok);
-    if (!first && done) {
+    float* const grads = grad_rows + size_t(blockIdx.x) * kMlpParams;
+    if (!done) {
+        for (int i = t; i < kMlpParams; i += kMlpThreads) grads[i] = 0.0f;
+    } else {
         const int warp = t >> 5, lane = t & 31;
         const int out = 16 * (warp & 3) + lane;  // output feature
         const uint32_t cols[4] = {kColW0, kColW1, kColW2, kColW3};
@@ -258,14 +279,13 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t 
                 float v[16];
                 ld_row<16>(tmem, cols[l] + c, v);
                 if (lane < 16 && out < nout[l])
-                    for (int k = 0; k < 16; ++k)
-                        if (v[k] != 0.0f) atomicAdd(grads + off[l] + (c + k) * nout[l] + out, v[k]);
+                    for (int k = 0; k < 16; ++k) grads[off[l] + (c + k) * nout[l] + out] = v[k];
             }
         }
     }
     // loss
     for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    if ((t & 31) == 0 && lsum != 0.0f) atomicAdd(loss_sum, lsum * scale);
+    if ((t & 31) == 0 && !hi) s_loss[t >> 5] = lsum * scale;
     if (!done) {
         if (t == 0) atomicOr(P.status, RTPG_STATUS_TIMEOUT);
         mma_drain(mbar, phase, P.poll_limit);
@@ -273,18 +293,28 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t 
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if (t == 0) loss_rows[blockIdx.x] = s_loss[0] + s_loss[1] + s_loss[2] + s_loss[3];
     if (t < 32) tmem_dealloc(*tslot, kTrainCols);
 }
 
-// sums of the nonnegative weights of gridDim.y minibatches of `batch` records (the last shorter)
-__global__ void k_wsum(int64_t n, int64_t batch, const float* w, float* out) {
+// Sums of the nonnegative weights of gridDim.y minibatches of `batch` records (the last shorter), each
+// in gridDim.x parts, kWsumParts apart.
+constexpr int kWsumParts = 64, kWsumBlock = 256;
+__global__ void __launch_bounds__(kWsumBlock) k_wsum(int64_t n, int64_t batch, const float* w, float* out) {
+    __shared__ float s_w[kWsumBlock / 32];
     const int64_t b0 = blockIdx.y * batch, m = min(batch, n - b0);
     float s = 0.0f;
-    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < m; i += int64_t(gridDim.x) * blockDim.x)
+    for (int64_t i = blockIdx.x * int64_t(kWsumBlock) + threadIdx.x; i < m; i += int64_t(gridDim.x) * kWsumBlock)
         s += fmaxf(w[b0 + i], 0.0f);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0 && s != 0.0f) atomicAdd(out + blockIdx.y, s);
+    if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        s = warp_sum_parts(s_w, kWsumBlock / 32);
+        if (threadIdx.x == 0) out[blockIdx.y * kWsumParts + blockIdx.x] = s;
+    }
 }
+static int wsum_parts(int64_t batch) { return (int)std::min<int64_t>(kWsumParts, (batch + 1023) / 1024); }
 
 // fp32 master [in][out] -> bf16 core-matrix layout of each matrix
 __device__ __forceinline__ uint32_t packed_index(int i) {
@@ -298,22 +328,64 @@ __global__ void k_mlp_pack(const float* w, __nv_bfloat16* wq) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpParams; i += gridDim.x * blockDim.x)
         wq[packed_index(i)] = __float2bfloat16_rn(w[i]);
 }
-// Adam (Kingma & Ba 2015) with bias correction; grads zeroed after use
-__global__ void k_mlp_adam(float* w, float* g, float* m, float* v, __nv_bfloat16* wq, float lr, float b1, float b2,
-                           float eps, float c1, float c2) {
+// What the CTAs of one k_mlp_train left: its gradient rows and shares of the loss.
+struct GradRows {
+    const float *grads, *loss;
+    int count;
+};
+// Launches of kGradCtas CTAs of 256 threads: the first kMlpParams / 32 have a parameter per lane, whose
+// rows their eight warps sum side by side, the last sums the loss.  Sums in double, in a fixed order.
+// 16 steps of 16384 records (128 rows, 8.4 MB a step that stay in the L2): 317 us, as with float
+// atomics into one accumulator.
+constexpr int kGradCtas = kMlpParams / 32 + 1, kGradWarps = 8;
+// The sum over all rows of parameter i = blockIdx.x * 32 + lane, in warp 0 (false elsewhere and in
+// the CTA of the loss).  All threads call it.
+__device__ __forceinline__ bool sum_rows(const GradRows& r, float* __restrict__ loss, int& i, float& sum) {
+    __shared__ double s_part[kGradWarps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (blockIdx.x == kMlpParams / 32) {
+        if (warp) return false;
+        double s = 0.0;
+        for (int k = lane; k < r.count; k += 32) s += (double)r.loss[k];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) *loss = (float)s;
+        return false;
+    }
+    i = blockIdx.x * 32 + lane;
+    double s = 0.0;
+#pragma unroll 8
+    for (int k = warp; k < r.count; k += kGradWarps) s += (double)r.grads[size_t(k) * kMlpParams + i];
+    s_part[warp][lane] = s;
+    __syncthreads();
+    if (warp) return false;
+    for (int k = 1; k < kGradWarps; ++k) s += s_part[k][lane];
+    sum = (float)s;
+    return true;
+}
+// gradients of one pass added to g
+__global__ void __launch_bounds__(32 * kGradWarps) k_mlp_add_grads(GradRows r, float* g, float* loss) {
+    int i;
+    float s;
+    if (sum_rows(r, loss, i, s)) g[i] += s;
+}
+// Adam (Kingma & Ba 2015) with bias correction; g (gradients added before) zeroed after use
+__global__ void __launch_bounds__(32 * kGradWarps) k_mlp_adam(GradRows r, float* loss, float* w, float* g, float* m, float* v,
+                                                              __nv_bfloat16* wq, float lr, float b1, float b2, float eps,
+                                                              float c1, float c2) {
     grid_launch_dependents();
     grid_dependency_wait();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpParams; i += gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-        w[i] = wi;
-        g[i] = 0.0f;
-        wq[packed_index(i)] = __float2bfloat16_rn(wi);
-    }
+    int i;
+    float s;
+    if (!sum_rows(r, loss, i, s)) return;
+    const float gi = g[i] + s;
+    const float mi = __fmaf_rn(1.0f - b1, gi, __fmul_rn(b1, m[i]));
+    const float vi = __fmaf_rn(__fmul_rn(1.0f - b2, gi), gi, __fmul_rn(b2, v[i]));
+    m[i] = mi;
+    v[i] = vi;
+    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    w[i] = wi;
+    g[i] = 0.0f;
+    wq[packed_index(i)] = __float2bfloat16_rn(wi);
 }
 
 }  // namespace rtpg
@@ -321,15 +393,20 @@ __global__ void k_mlp_adam(float* w, float* g, float* m, float* v, __nv_bfloat16
 using namespace rtpg;
 
 constexpr int64_t kMlpGroup = 256;  // minibatches whose weights are summed in one launch
+// scratch of training: weight sums of a group of minibatches in parts, a CTA's share of the loss and
+// gradient row each for a launch of k_mlp_train (9.8 MB)
+constexpr size_t kLossRows = kMlpGroup * kWsumParts, kGradRowsAt = kLossRows + 256,
+                 kTrainScratch = kGradRowsAt + size_t(kSMs) * kMlpParams;
+static_assert(kSMs <= 256, "loss shares");
 
 struct rtpg_mlp {
     MlpDev dev{};
     float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
-    float* scratch = nullptr;  // of kMlpGroup minibatches: weight sums, then losses
+    float* loss = nullptr;     // of the newest step, behind the gradients
+    float* scratch = nullptr;  // kTrainScratch floats (scratch_alloc)
     __nv_bfloat16* wq = nullptr;
     float lr = 1e-3f, b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     uint32_t step = 0;
-    int64_t last = 0;  // the newest loss's place in scratch's second half
     float mn[3], mx[3];
     // record buffer (filled by the tracer or rtpg_mlp_add_records)
     uint32_t capacity = 0;
@@ -351,8 +428,42 @@ struct rtpg_mlp {
     }
     ~rtpg_mlp() {
         for (void* p : allocs) cudaFree(p);
+        if (scratch) {
+            cudaDeviceSynchronize();  // memory of a pool is freed without waiting for its last use
+            cudaFree(scratch);
+        }
     }
 };
+
+// Training scratch comes from a pool of its own on each device: mapping and unmapping 9.8 MB by cudaMalloc
+// and cudaFree costs 0.7 ms a guide, as much as all else in creating it.  The pool keeps at most
+// kScratchKept bytes that no guide uses.
+constexpr uint64_t kScratchKept = 32u << 20;
+static int scratch_alloc(rtpg_mlp* h) {
+    static std::mutex mu;
+    static std::map<int, cudaMemPool_t> pools;
+    int dev = 0;
+    RTPG_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    cudaMemPool_t& pool = pools[dev];
+    if (!pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        uint64_t kept = kScratchKept;
+        RTPG_CUDA(cudaMemPoolCreate(&pool, &props));
+        RTPG_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept));
+    }
+    const cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&h->scratch), sizeof(float) * kTrainScratch, pool, nullptr);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        h->scratch = nullptr;
+        return fail(RTPG_ENOMEM, "rtpg_mlp_create: %zu bytes of training scratch: %s", sizeof(float) * kTrainScratch,
+                    cudaGetErrorString(e));
+    }
+    return RTPG_OK;
+}
 
 namespace rtpg {
 MlpView mlp_view(const rtpg_mlp* h) {
@@ -391,8 +502,8 @@ int rtpg_mlp_create(const float* aabb_min, const float* aabb_max, uint32_t seed,
     h->lr = learning_rate > 0.0f ? learning_rate : 1e-3f;
     h->capacity = record_capacity;
     const size_t C = std::max<uint32_t>(record_capacity, 1);
-    if ((r = h->alloc(&h->w, kMlpParams)) || (r = h->alloc(&h->g, kMlpParams)) || (r = h->alloc(&h->m, kMlpParams)) ||
-        (r = h->alloc(&h->v, kMlpParams)) || (r = h->alloc(&h->wq, kMlpParams)) || (r = h->alloc(&h->scratch, 2 * kMlpGroup)) ||
+    if ((r = h->alloc(&h->w, kMlpParams)) || (r = h->alloc(&h->g, kMlpParams + 1)) || (r = h->alloc(&h->m, kMlpParams)) ||
+        (r = h->alloc(&h->v, kMlpParams)) || (r = h->alloc(&h->wq, kMlpParams)) || (r = scratch_alloc(h)) ||
         (r = h->alloc(&h->r_pos, 3 * C)) || (r = h->alloc(&h->r_nrm, 3 * C)) || (r = h->alloc(&h->r_wo, 3 * C)) ||
         (r = h->alloc(&h->r_wi, 3 * C)) || (r = h->alloc(&h->r_w, C)) || (r = h->alloc(&h->r_pdf, C)) ||
         (r = h->alloc(&h->r_count, 1)) ||
@@ -400,6 +511,7 @@ int rtpg_mlp_create(const float* aabb_min, const float* aabb_max, uint32_t seed,
         delete h;
         return r;
     }
+    h->loss = h->g + kMlpParams;
     for (int k = 0; k < 3; ++k) {
         h->mn[k] = aabb_min[k];
         h->mx[k] = aabb_max[k];
@@ -429,7 +541,7 @@ int rtpg_mlp_create(const float* aabb_min, const float* aabb_max, uint32_t seed,
     }
     cudaError_t e;
     if ((e = cudaMemcpy(h->w, w.data(), sizeof(float) * kMlpParams, cudaMemcpyHostToDevice)) ||
-        (e = cudaMemset(h->g, 0, sizeof(float) * kMlpParams)) || (e = cudaMemset(h->m, 0, sizeof(float) * kMlpParams)) ||
+        (e = cudaMemset(h->g, 0, sizeof(float) * (kMlpParams + 1))) || (e = cudaMemset(h->m, 0, sizeof(float) * kMlpParams)) ||
         (e = cudaMemset(h->v, 0, sizeof(float) * kMlpParams)) || (e = cudaMemset(h->r_count, 0, 4)) ||
         (e = cudaMemset(h->status, 0, 4))) {
         delete h;
@@ -482,42 +594,44 @@ int rtpg_mlp_eval(rtpg_mlp* h, int64_t n, const float* pos, const float* nrm, co
     return RTPG_OK;
 }
 
-// Gradient of the loss over n records (device arrays) ADDED to host_grads-sized device buffer
-// `grads` (16384 floats, NULL: the handle's own accumulator); returns the loss through
-// host_loss (NULL: none).  The loss is -sum w log q(wi) / sum w.
-// weight sums of up to kMlpGroup minibatches of `batch` records (n records in all), losses zeroed
+// weight sums of up to kMlpGroup minibatches of `batch` records (n records in all)
 static int mlp_group(rtpg_mlp* h, int64_t n, int64_t batch, const float* w, cudaStream_t st) {
     const int64_t nb = (n + batch - 1) / batch;
-    RTPG_CUDA(cudaMemsetAsync(h->scratch, 0, sizeof(float) * 2 * kMlpGroup, st));
-    k_wsum<<<dim3((unsigned)std::max<int64_t>(1, grid_for(std::min(n, batch), 256, 4) / nb), (unsigned)nb), 256, 0, st>>>(
-        n, batch, w, h->scratch);
+    k_wsum<<<dim3((unsigned)wsum_parts(batch), (unsigned)nb), kWsumBlock, 0, st>>>(n, batch, w, h->scratch);
     RTPG_LAUNCH_CHECK();
     return RTPG_OK;
 }
-// gradient over minibatch k of the group; chained: a dependent of the previous step's Adam, before
-// which records and weight sums were complete
-static int mlp_grad(rtpg_mlp* h, int64_t k, int64_t n, const Records& R, float* grads, bool chained, cudaStream_t st) {
+// gradient over the n records of minibatch k of the group, left in rows; chained: a dependent of the
+// previous step's Adam, before which records and weight sums were complete
+static int mlp_grad(rtpg_mlp* h, int64_t k, int64_t n, int64_t batch, const Records& R, bool chained, GradRows& rows,
+                    cudaStream_t st) {
     const int g = (int)std::min<int64_t>((n + kMlpTile - 1) / kMlpTile, kSMs);
-    const float* const wsum = h->scratch + k;
-    float* const loss = h->scratch + kMlpGroup + k;
+    const float* const wsum = h->scratch + k * kWsumParts;
+    float *const grads = h->scratch + kGradRowsAt, *const loss = h->scratch + kLossRows;
     if (chained) {
-        RTPG_CUDA(launch_dependent(k_mlp_train, g, kMlpThreads, kSmemTrain, st, h->dev, n, R, wsum, grads, loss));
+        RTPG_CUDA(launch_dependent(k_mlp_train, g, kMlpThreads, kSmemTrain, st, h->dev, n, R, wsum, wsum_parts(batch), grads, loss));
     } else {
-        k_mlp_train<<<g, kMlpThreads, kSmemTrain, st>>>(h->dev, n, R, wsum, grads, loss);
+        k_mlp_train<<<g, kMlpThreads, kSmemTrain, st>>>(h->dev, n, R, wsum, wsum_parts(batch), grads, loss);
         RTPG_LAUNCH_CHECK();
     }
+    rows = GradRows{grads, loss, g};
     return RTPG_OK;
 }
 
+// Gradient of the loss over n records (device arrays) ADDED to the device buffer `grads` (16384
+// floats, NULL: the handle's own accumulator); returns the loss through host_loss (NULL: none).
+// The loss is -sum w log q(wi) / sum w.
 int rtpg_mlp_loss_grad(rtpg_mlp* h, int64_t n, const float* pos, const float* nrm, const float* wo, const float* wi,
                        const float* w, float* grads, float* host_loss, void* stream) {
     if (!h || n <= 0 || !pos || !nrm || !wo || !wi || !w) return fail(RTPG_EINVAL, "rtpg_mlp_loss_grad: bad arguments");
     cudaStream_t st = as_stream(stream);
-    h->last = 0;
+    GradRows rows;
     int r = mlp_group(h, n, n, w, st);
-    if (r || (r = mlp_grad(h, 0, n, Records{pos, nrm, wo, wi, w}, grads ? grads : h->g, false, st))) return r;
+    if (r || (r = mlp_grad(h, 0, n, n, Records{pos, nrm, wo, wi, w}, false, rows, st))) return r;
+    k_mlp_add_grads<<<kGradCtas, 32 * kGradWarps, 0, st>>>(rows, grads ? grads : h->g, h->loss);
+    RTPG_LAUNCH_CHECK();
     if (host_loss) {
-        RTPG_CUDA(cudaMemcpyAsync(host_loss, h->scratch + kMlpGroup, 4, cudaMemcpyDeviceToHost, st));
+        RTPG_CUDA(cudaMemcpyAsync(host_loss, h->loss, 4, cudaMemcpyDeviceToHost, st));
         RTPG_CUDA(cudaStreamSynchronize(st));
     }
     return RTPG_OK;
@@ -545,18 +659,18 @@ int rtpg_mlp_train(rtpg_mlp* h, int64_t n, const float* pos, const float* nrm, c
             if (r) return r;
             for (int64_t b = 0; b < in_group; b += batch) {
                 const int64_t at = g0 + b;
-                h->last = b / batch;
-                r = mlp_grad(h, h->last, std::min<int64_t>(batch, in_group - b),
-                             Records{pos + 3 * at, nrm + 3 * at, wo + 3 * at, wi + 3 * at, w + at}, h->g, b > 0, st);
+                GradRows rows;
+                r = mlp_grad(h, b / batch, std::min<int64_t>(batch, in_group - b), batch,
+                             Records{pos + 3 * at, nrm + 3 * at, wo + 3 * at, wi + 3 * at, w + at}, b > 0, rows, st);
                 if (r) return r;
                 ++h->step;
                 const float c1 = 1.0f - std::pow(h->b1, (float)h->step), c2 = 1.0f - std::pow(h->b2, (float)h->step);
-                RTPG_CUDA(launch_dependent(k_mlp_adam, 64, 256, 0, st, h->w, h->g, h->m, h->v, h->wq, h->lr, h->b1, h->b2,
+                RTPG_CUDA(launch_dependent(k_mlp_adam, kGradCtas, 32 * kGradWarps, 0, st, rows, h->loss, h->w, h->g, h->m, h->v, h->wq, h->lr, h->b1, h->b2,
                                            h->eps, c1, c2));
             }
         }
     if (host_last_loss) {
-        RTPG_CUDA(cudaMemcpyAsync(host_last_loss, h->scratch + kMlpGroup + h->last, 4, cudaMemcpyDeviceToHost, st));
+        RTPG_CUDA(cudaMemcpyAsync(host_last_loss, h->loss, 4, cudaMemcpyDeviceToHost, st));
         RTPG_CUDA(cudaStreamSynchronize(st));
     }
     return RTPG_OK;

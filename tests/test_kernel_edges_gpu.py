@@ -430,3 +430,36 @@ def test_sampling_thresholds_near_and_past_boundaries(cuda, oracle):
         wa, wp = o.sample_pdf(q["pos"], q["seeds"])[:2]
         np.testing.assert_array_equal(a.cpu().numpy(), wa)
         np.testing.assert_array_equal(p.cpu().numpy(), wp)
+
+
+def _records(n, seed, dev):
+    rng = np.random.default_rng(seed)
+    unit = lambda: (lambda v: (v / np.linalg.norm(v, axis=1, keepdims=True)).astype(np.float32))(rng.normal(size=(n, 3)))
+    return [_t(a, dev) for a in (rng.random((n, 3), dtype=np.float32), unit(), unit(), unit(),
+                                 rng.lognormal(0, 2, n).astype(np.float32))]
+
+
+@pytest.mark.parametrize("n,batch", [(1, 4096), (700, 256), (40000, 16384), (148 * 128 * 2 + 5, 148 * 128 + 1), (5000, 1 << 20)])
+def test_training_repeats_bit_for_bit(cuda, n, batch):
+    """Weight sums, gradients and loss are added in a fixed order whatever order the CTAs finish in: the
+    same records give the same parameters, gradient and loss each time (one tile, one and several per
+    CTA, ragged last minibatches).  Gradients are added to what is there."""
+    import torch
+    from rtlib_b200.mlp import MLPGuide
+    rec = _records(n, n, cuda)
+    got = []
+    for _ in range(4):
+        g = MLPGuide((0, 0, 0), (1, 1, 1), seed=9)
+        loss, grad = g.loss_grad(*rec)
+        got.append((g.train(rec, batch=batch, epochs=3), g.params(), loss, grad))
+        assert g.status() == 0
+    for loss, params, l0, g0 in got[1:]:
+        assert loss == got[0][0] and l0 == got[0][2]
+        np.testing.assert_array_equal(params, got[0][1])
+        assert torch.equal(g0, got[0][3])
+    # the same gradient added to ones, in the caller's buffer
+    from rtlib_b200._lib import call, ptr, stream_ptr
+    g = MLPGuide((0, 0, 0), (1, 1, 1), seed=9)
+    more = torch.ones(16384, device=cuda)
+    call("rtpg_mlp_loss_grad", g.h, n, *[ptr(x) for x in rec], ptr(more), None, stream_ptr())
+    assert torch.equal(more, got[0][3] + 1.0)
