@@ -323,10 +323,13 @@ struct Records {
 };
 
 // ------------------------------------------------------------------ shared building blocks
+// The weights by coherent loads: a training launch starts while the previous step's Adam still writes
+// them, and what is read after grid_dependency_wait may not come through the read-only path, whose
+// data must not change while the kernel runs.
 __device__ __forceinline__ void load_weights(__nv_bfloat16* ws, const __nv_bfloat16* wq) {
     const uint4* s = reinterpret_cast<const uint4*>(wq);
     uint4* d = reinterpret_cast<uint4*>(ws);
-    for (int i = threadIdx.x; i < kMlpParams / 8; i += blockDim.x) d[i] = __ldg(s + i);
+    for (int i = threadIdx.x; i < kMlpParams / 8; i += blockDim.x) d[i] = __ldcg(s + i);
 }
 // All threads: make the shared-memory operands written by this CTA visible to the tensor cores and
 // order earlier TMEM loads before the next MMA.  ok: the thread's last wait; returns whether no

@@ -463,3 +463,19 @@ def test_training_repeats_bit_for_bit(cuda, n, batch):
     more = torch.ones(16384, device=cuda)
     call("rtpg_mlp_loss_grad", g.h, n, *[ptr(x) for x in rec], ptr(more), None, stream_ptr())
     assert torch.equal(more, got[0][3] + 1.0)
+
+
+@pytest.mark.parametrize("batch,steps", [(100, 40), (5000, 12), (148 * 128 + 1, 5)])
+def test_chained_steps_see_the_step_before(cuda, batch, steps):
+    """Within a call a step's launch starts while the previous step's Adam runs; its CTAs read the
+    weights that Adam leaves: the steps of one call equal calls of one step each, bit for bit, with one
+    tile, many CTAs and several tiles per CTA."""
+    from rtlib_b200.mlp import MLPGuide
+    n = batch * steps - batch // 3
+    rec = _records(n, steps, cuda)
+    a, b = MLPGuide((0, 0, 0), (1, 1, 1), seed=9), MLPGuide((0, 0, 0), (1, 1, 1), seed=9)
+    la = a.train(rec, batch=batch, epochs=1)
+    for s in range(0, n, batch):
+        lb = b.train([x[s:s + batch].contiguous() for x in rec], batch=batch, epochs=1)
+    np.testing.assert_array_equal(a.params(), b.params())
+    assert la == lb and a.status() == 0 and b.status() == 0
