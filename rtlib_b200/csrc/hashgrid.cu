@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "hash_stage.h"
 #include "limits.cuh"
 #include "hashgrid_dev.cuh"
 
@@ -120,11 +121,6 @@ struct StageDev {
     uint8_t* occ;               // per point: occupied slots of its bucket
     uint32_t size;              // a power of two, at least 1.5 points
 };
-static uint32_t stage_size(uint32_t points) {
-    uint32_t h = 32;
-    while (h < points + points / 2) h <<= 1;
-    return h;
-}
 static size_t stage_ones(uint32_t size, uint32_t nbuckets) { return size_t(size) * 12 + size_t(nbuckets) * 4; }
 static size_t stage_bytes(uint32_t cap, uint32_t nbuckets) {
     return ((stage_ones(stage_size(cap), nbuckets) + 255) & ~size_t(255)) + size_t(stage_size(cap)) * 4 + size_t(cap) * 13;
@@ -205,11 +201,8 @@ __global__ void __launch_bounds__(256) k_hash_give(StageDev s, int64_t base, uin
         if (e != kFull) out_slot[base + j] = s.slot[e];
     }
 }
-// One batch.  A bucket's list is as long as the distinct new keys that fall into it, walked once per
-// key: with at most kStagePerSlot points per slot that is at most 128 on average.  2^19 points (373 k
-// cells) into 2^20 slots: 253 us with two 64-bit radix sorts, 48 us here.
-constexpr uint32_t kStagePerSlot = 4;
-static bool stage_fits(const HashGridDev& g, int64_t n) { return (uint64_t)n <= (uint64_t)g.nslots * kStagePerSlot; }
+// One batch (where stage_fits).  2^19 points (373 k cells) into 2^20 slots: 253 us with two 64-bit radix
+// sorts, 48 us here.
 static int stage_insert(const HashGridDev& g, unsigned char* scratch, int64_t base, uint32_t n, const float* pos,
                         uint32_t* out_slot, uint64_t* out_key, cudaStream_t st) {
     const StageDev s = stage_view(scratch, n, g.nbuckets);
@@ -316,8 +309,7 @@ int rtpg_hashgrid_create(const float* aabb_min, const float* aabb_max, const uin
         delete h;
         return fail(RTPG_ECUDA, "cub temp size: %s", cudaGetErrorString(e));
     }
-    // a staged batch may be as large as max_batch
-    const uint32_t stage_cap = (uint32_t)std::min<uint64_t>(B, (uint64_t)num_slots * kStagePerSlot);
+    const size_t staged = stage_bytes(stage_cap(B, num_slots), g.nbuckets);
     for (int pass = 0; pass < 2; ++pass) {  // sizes, then places
         size_t at = 0;
         auto take = [&](auto** p, size_t count) {
@@ -335,7 +327,7 @@ int rtpg_hashgrid_create(const float* aabb_min, const float* aabb_max, const uin
         take(&h->occ_of, B);
         take(&h->temp, tb);
         if (!pass && ((r = h->alloc(&g.cur, num_slots)) || (r = h->alloc(&g.prv, num_slots)) || (r = h->alloc(&g.status, 1)) ||
-                      (r = h->alloc(&h->stage, std::max(at, stage_bytes(stage_cap, g.nbuckets)))))) {
+                      (r = h->alloc(&h->stage, std::max(at, staged))))) {
             delete h;
             return r;
         }
@@ -382,7 +374,7 @@ int rtpg_hashgrid_insert(rtpg_hashgrid* h, int64_t n, const float* pos, uint32_t
     // chunks are inserted in order, which keeps the sequential-insertion semantics
     for (int64_t base = 0; base < n; base += h->max_batch) {
         const int64_t m = std::min<int64_t>(h->max_batch, n - base);
-        if (stage_fits(h->dev, m)) {
+        if (stage_fits((uint64_t)m, h->dev.nslots)) {
             const int r = stage_insert(h->dev, h->stage, base, (uint32_t)m, pos, out_slot, out_key, st);
             if (r) return r;
             continue;
@@ -561,7 +553,7 @@ extern "C" int rtpg_hashgrid_insert_noalloc(const float* aabb_min, const float* 
     auto* occ_of = reinterpret_cast<uint8_t*>(s + kNA_occ);
     void* temp = s + kNA_temp;
     // the staging scratch lies where the sort's would (the status word apart)
-    if (stage_fits(g, n) && stage_bytes((uint32_t)n, g.nbuckets) <= kNA_status)
+    if (stage_fits((uint64_t)n, g.nslots) && stage_bytes((uint32_t)n, g.nbuckets) <= kNA_status)
         return stage_insert(g, s, 0, (uint32_t)n, pos, out_slot, nullptr, as_stream(stream));
     // every scratch word read below is written earlier in the same call, so nothing left
     // by a previous call needs clearing
