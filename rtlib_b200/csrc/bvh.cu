@@ -79,10 +79,8 @@ __device__ __forceinline__ int bvh_delta(const unsigned long long* __restrict__ 
 }
 
 // Karras 2012: node i covers a key range whose split is found by binary search
-// (count: leaves of every node)
 __global__ void k_scene_hierarchy(const unsigned long long* __restrict__ keys, int n, BvhNode* __restrict__ nodes,
-                                  uint32_t* __restrict__ parent_i, uint32_t* __restrict__ parent_l,
-                                  uint32_t* __restrict__ count) {
+                                  uint32_t* __restrict__ parent_i, uint32_t* __restrict__ parent_l) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n - 1; i += gridDim.x * blockDim.x) {
         const int d = (bvh_delta(keys, n, i, i + 1) - bvh_delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
         const int dmin = bvh_delta(keys, n, i, i - d);
@@ -108,7 +106,6 @@ __global__ void k_scene_hierarchy(const unsigned long long* __restrict__ keys, i
         nodes[i].child[0] = c0;
         nodes[i].child[1] = c1;
         nodes[i].pad[0] = nodes[i].pad[1] = 0;
-        count[i] = (uint32_t)(hi - lo + 1);
     }
 }
 
@@ -221,9 +218,13 @@ __global__ void k_scene_boxes(const float* __restrict__ v, const uint32_t* __res
 // around its centroid and so inflates every box above it; here it waits until large clusters are
 // left and ends up near the root.  Equal areas are told apart by the smaller i ^ j, which is symmetric
 // and distinct for a cluster's candidates, so the least pair always merges.
+// Boxes that contain one another in order merge one pair a round: each one's best partner is a
+// smaller one.  Clusters that are left after kPlocRounds rounds pair with their neighbour in order
+// (i with i ^ 1, which halves them each round).  The 1.05 M-triangle rooms take 74 rounds, soups of random
+// triangles 49 for 200,000.
 constexpr int kPlocRadius = 16;
 constexpr int kPlocBlock = 256;
-constexpr uint32_t kPlocMaxRounds = 120;  // a round adds at most one level (see k_wide_level)
+constexpr uint32_t kPlocRounds = 88;  // a round adds at most one level (see k_wide_level)
 
 __device__ __forceinline__ float box_area(float4 alo, float4 ahi, float4 blo, float4 bhi) {
     const float x = fmaxf(ahi.x, bhi.x) - fminf(alo.x, blo.x), y = fmaxf(ahi.y, bhi.y) - fminf(alo.y, blo.y),
@@ -239,7 +240,7 @@ __global__ void k_ploc_init(const float4* __restrict__ leaf_box, uint32_t n, flo
     }
 }
 __global__ void __launch_bounds__(kPlocBlock) k_ploc_nearest(const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                                             uint32_t n, uint32_t* __restrict__ nearest) {
+                                                             uint32_t n, int radius, uint32_t* __restrict__ nearest) {
     __shared__ float4 s_lo[kPlocBlock + 2 * kPlocRadius], s_hi[kPlocBlock + 2 * kPlocRadius];
     const int base = (int)(blockIdx.x * kPlocBlock) - kPlocRadius;
     for (int k = threadIdx.x; k < kPlocBlock + 2 * kPlocRadius; k += kPlocBlock) {
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_nearest(const float4* __res
     float best = INFINITY;
     uint32_t arg = i ^ 1u;
     if (arg >= n) arg = i - 1;
-    for (int d = -kPlocRadius; d <= kPlocRadius; ++d) {
+    for (int d = -radius; d <= radius; ++d) {
         const int j = (int)i + d;
         if (d == 0 || j < 0 || j >= (int)n) continue;
         const float a = box_area(mlo, mhi, s_lo[me + d], s_hi[me + d]);
@@ -307,7 +308,7 @@ __global__ void k_ploc_compact(const float4* __restrict__ lo, const float4* __re
 // the child with most triangles is opened instead, which bounds the depth: on the way to any
 // triangle a level then either descends seven binary levels or at least halves the triangles
 // (at most 31 times), so a binary hierarchy of D levels takes at most kCountLevel + 31 + (D - 31) / 7
-// levels: 56 for the linear one (95: 63 key bits and the index), 60 for 120 rounds of clustering.
+// levels: 60 for a clustered hierarchy (kPlocRounds rounds and at most 31 that halve the clusters).
 // Nodes with fewer than eight children have leaves only, at least two, so there are at most 5/8 as
 // many nodes as triangles.
 constexpr uint32_t kCountLevel = 16;
@@ -569,7 +570,7 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
     unsigned* flags = nullptr;
     BvhTri* tris = nullptr;  // the triangles in leaf order, and their scene indices
     uint32_t *prim = nullptr, *root = nullptr, *counts = nullptr;
-    uint32_t *count = nullptr, *pcount = nullptr, *nearest = nullptr, *keep = nullptr, *at = nullptr;
+    uint32_t *pcount = nullptr, *nearest = nullptr, *keep = nullptr, *at = nullptr;
     BvhNode* pnodes = nullptr;
     float4 *clo[2] = {nullptr, nullptr}, *chi[2] = {nullptr, nullptr};
     uint8_t *sort_temp = nullptr, *scan_temp = nullptr;
@@ -624,7 +625,6 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
             take(&flags, n);
             take(&root, wide_cap);
             take(&counts, 5);
-            take(&count, n);
             take(&pcount, n);
             take(&nearest, n);
             take(&keep, n);
@@ -656,7 +656,7 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
         if (flat) {
             k_scene_flat<<<1, 64, 0, st>>>(tris, prim, n, s->flat);
         } else {
-            k_scene_hierarchy<<<g, 256, 0, st>>>(dk.Current(), (int)n, s->nodes, pi, pl, count);
+            k_scene_hierarchy<<<g, 256, 0, st>>>(dk.Current(), (int)n, s->nodes, pi, pl);
             if ((e = cudaMemsetAsync(flags, 0, 4ull * n, st))) break;
             k_scene_boxes<<<g, 256, 0, st>>>(vertices, indices, prim, n, s->nodes, pi, pl, ibox, flags);
             // counts: wide nodes, triangles, largest absolute coordinate, clustered nodes, clusters
@@ -665,9 +665,10 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
             k_scene_leaf_boxes<<<g, 256, 0, st>>>(vertices, indices, prim, n, s->leaf_box, counts + 2);
             k_ploc_init<<<g, 256, 0, st>>>(s->leaf_box, n, clo[0], chi[0]);
             uint32_t clusters = n, rounds = 0;
-            for (; clusters > 1 && rounds < kPlocMaxRounds && !e; ++rounds) {
+            for (; clusters > 1 && !e; ++rounds) {
                 const int a = rounds & 1, b = a ^ 1, gc = grid_for(clusters, 256, 8);
-                k_ploc_nearest<<<(clusters + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, st>>>(clo[a], chi[a], clusters, nearest);
+                const int radius = rounds < kPlocRounds ? kPlocRadius : 0;
+                k_ploc_nearest<<<(clusters + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, st>>>(clo[a], chi[a], clusters, radius, nearest);
                 k_ploc_merge<<<gc, 256, 0, st>>>(clo[a], chi[a], clusters, nearest, pnodes, pcount, counts + 3, keep);
                 if ((e = cub::DeviceScan::ExclusiveSum(scan_temp, scan_bytes, keep, at, (int)clusters, st))) break;
                 k_ploc_compact<<<gc, 256, 0, st>>>(clo[a], chi[a], clusters, keep, at, clo[b], chi[b], counts + 4);
@@ -675,12 +676,7 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
                 e = cudaStreamSynchronize(st);
             }
             if (e) break;
-            // the clustered hierarchy (its root was made last) or, where clustering took too many
-            // rounds (coincident triangles), the linear one
-            const bool clustered = clusters == 1;
-            const BvhNode* const bin = clustered ? pnodes : s->nodes;
-            const uint32_t* const bin_count = clustered ? pcount : count;
-            const uint32_t bin_root = clustered ? n - 2 : 0;
+            const uint32_t bin_root = n - 2;  // made last
             if ((e = cudaMemcpyAsync(root, &bin_root, 4, cudaMemcpyHostToDevice, st))) break;
             uint32_t begin = 0, end = 1, now[3] = {1, 0, 0};
             for (uint32_t level = 0; begin < end; ++level) {
@@ -688,7 +684,7 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
                     rc = fail(RTPG_ECAPACITY, "rtpg_scene_create: hierarchy of %u nodes in %u levels exceeds its bounds", end, level);
                     break;
                 }
-                k_wide_level<<<(end - begin + 127) / 128, 128, 0, st>>>(bin, bin_count, tris, prim, begin, end, level, root,
+                k_wide_level<<<(end - begin + 127) / 128, 128, 0, st>>>(pnodes, pcount, tris, prim, begin, end, level, root,
                                                                        wide_cap, s->wide, s->wtris, counts);
                 if ((e = cudaMemcpyAsync(now, counts, sizeof(now), cudaMemcpyDeviceToHost, st))) break;
                 if ((e = cudaStreamSynchronize(st))) break;

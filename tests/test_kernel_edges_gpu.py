@@ -479,3 +479,33 @@ def test_chained_steps_see_the_step_before(cuda, batch, steps):
         lb = b.train([x[s:s + batch].contiguous() for x in rec], batch=batch, epochs=1)
     np.testing.assert_array_equal(a.params(), b.params())
     assert la == lb and a.status() == 0 and b.status() == 0
+
+
+@pytest.mark.parametrize("nested,others", [(130, 0), (200, 0), (200, 3000), (1000, 500)])
+def test_hierarchy_of_nested_triangles(cuda, oracle, nested, others):
+    """Boxes that contain one another merge one pair a round, so clustering runs out of rounds and
+    pairs what is left by order: hits equal brute force, alone and beside other triangles."""
+    import torch
+    from rtlib_b200.tracer import Scene
+    rng = np.random.default_rng(nested + others)
+    size = (1.0 + 0.02 * np.arange(nested, dtype=np.float32))[:, None, None]
+    tri = np.array([[[-1, -1, -1], [2, -1, -1], [-1, 2, 2]]], np.float32) * size
+    soup = rng.normal(size=(others, 3, 3)) * 0.2 + rng.uniform(-9, 9, (others, 1, 3))
+    tri = np.concatenate([tri, soup.astype(np.float32)]).reshape(-1, 9)
+    tri = tri[rng.permutation(len(tri))]
+    q = 20000
+    org, d = rng.uniform(-10, 10, (q, 3)).astype(np.float32), rng.normal(size=(q, 3)).astype(np.float32)
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    sc = Scene(_t(tri, cuda))
+    t, p, occ = torch.empty(q, device=cuda), torch.empty(q, dtype=torch.int32, device=cuda), torch.empty(q, dtype=torch.int32, device=cuda)
+    sc.intersect(_t(org, cuda), _t(d, cuda), out_t=t, out_prim=p)
+    sc.intersect(_t(org, cuda), _t(d, cuda), any_hit=True, out_prim=occ)
+    want_t, want_p = oracle.intersect(tri, org, d, 0.0, 1e20)[:2]
+    hit, got_p = want_p != 0xFFFFFFFF, p.cpu().numpy().view(np.uint32)
+    np.testing.assert_array_equal(got_p != 0xFFFFFFFF, hit)
+    np.testing.assert_array_equal(t.cpu().numpy()[hit], want_t[hit])
+    np.testing.assert_array_equal(occ.cpu().numpy() != -1, hit)
+    # the triangles share a plane: another one than the lowest index may answer, at the same distance
+    for i in np.flatnonzero(got_p != want_p):
+        alone = oracle.intersect(tri[got_p[i]:got_p[i] + 1], org[i:i + 1], d[i:i + 1], 0.0, 1e20)[0]
+        assert alone[0] == want_t[i]
