@@ -239,9 +239,47 @@ __global__ void k_ploc_init(const float4* __restrict__ leaf_box, uint32_t n, flo
         hi[k] = make_float4(a.w, b.x, b.y, 0.0f);
     }
 }
+// The partner of cluster i of n: lo, hi point at it among its neighbours.
+__device__ __forceinline__ uint32_t ploc_partner(const float4* lo, const float4* hi, uint32_t i, uint32_t n, int radius) {
+    const float4 mlo = *lo, mhi = *hi;
+    float best = INFINITY;
+    uint32_t arg = i ^ 1u;
+    if (arg >= n) arg = i - 1;
+    for (int d = -radius; d <= radius; ++d) {
+        const int j = (int)i + d;
+        if (d == 0 || j < 0 || j >= (int)n) continue;
+        const float a = box_area(mlo, mhi, lo[d], hi[d]);
+        if (a < best || (a == best && ((uint32_t)j ^ i) < (arg ^ i))) {
+            best = a;
+            arg = (uint32_t)j;
+        }
+    }
+    return arg;
+}
+// clusters a and b become a node (a: the merged cluster)
+__device__ __forceinline__ void ploc_merge(float4& alo, float4& ahi, float4 blo, float4 bhi, BvhNode* nodes, uint32_t* count,
+                                           uint32_t* next) {
+    const uint32_t ra = __float_as_uint(alo.w), rb = __float_as_uint(blo.w), id = atomicAdd(next, 1u);
+    BvhNode nd;
+    nd.a = make_float4(alo.x, alo.y, alo.z, ahi.x);
+    nd.b = make_float4(ahi.y, ahi.z, blo.x, blo.y);
+    nd.c = make_float4(blo.z, bhi.x, bhi.y, bhi.z);
+    nd.child[0] = ra;
+    nd.child[1] = rb;
+    nd.pad[0] = nd.pad[1] = 0;
+    nodes[id] = nd;
+    count[id] = ((ra & kBvhLeafBit) ? 1u : count[ra]) + ((rb & kBvhLeafBit) ? 1u : count[rb]);
+    alo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), __uint_as_float(id));
+    ahi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
+}
+// A round over many clusters, three kernels and a scan; their number is on the device (the host only
+// knows a bound, the grids' size).
 __global__ void __launch_bounds__(kPlocBlock) k_ploc_nearest(const float4* __restrict__ lo, const float4* __restrict__ hi,
-                                                             uint32_t n, int radius, uint32_t* __restrict__ nearest) {
+                                                             const uint32_t* __restrict__ clusters, int radius,
+                                                             uint32_t* __restrict__ nearest) {
     __shared__ float4 s_lo[kPlocBlock + 2 * kPlocRadius], s_hi[kPlocBlock + 2 * kPlocRadius];
+    const uint32_t n = *clusters;
+    if (blockIdx.x * kPlocBlock >= n) return;
     const int base = (int)(blockIdx.x * kPlocBlock) - kPlocRadius;
     for (int k = threadIdx.x; k < kPlocBlock + 2 * kPlocRadius; k += kPlocBlock) {
         const int g = min(max(base + k, 0), (int)n - 1);
@@ -249,55 +287,85 @@ __global__ void __launch_bounds__(kPlocBlock) k_ploc_nearest(const float4* __res
         s_hi[k] = hi[g];
     }
     __syncthreads();
-    const uint32_t i = blockIdx.x * kPlocBlock + threadIdx.x;
-    if (i >= n) return;
-    const int me = threadIdx.x + kPlocRadius;
-    const float4 mlo = s_lo[me], mhi = s_hi[me];
-    float best = INFINITY;
-    uint32_t arg = i ^ 1u;
-    if (arg >= n) arg = i - 1;
-    for (int d = -radius; d <= radius; ++d) {
-        const int j = (int)i + d;
-        if (d == 0 || j < 0 || j >= (int)n) continue;
-        const float a = box_area(mlo, mhi, s_lo[me + d], s_hi[me + d]);
-        if (a < best || (a == best && ((uint32_t)j ^ i) < (arg ^ i))) {
-            best = a;
-            arg = (uint32_t)j;
-        }
-    }
-    nearest[i] = arg;
+    const uint32_t i = blockIdx.x * kPlocBlock + threadIdx.x, me = threadIdx.x + kPlocRadius;
+    if (i < n) nearest[i] = ploc_partner(s_lo + me, s_hi + me, i, n, radius);
 }
-__global__ void k_ploc_merge(float4* lo, float4* hi, uint32_t n, const uint32_t* __restrict__ nearest,
-                             BvhNode* __restrict__ nodes, uint32_t* __restrict__ count, uint32_t* __restrict__ next,
+__global__ void k_ploc_merge(float4* lo, float4* hi, const uint32_t* __restrict__ clusters, uint32_t bound,
+                             const uint32_t* __restrict__ nearest, BvhNode* nodes, uint32_t* count, uint32_t* next,
                              uint32_t* __restrict__ keep) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t j = nearest[i];
-        const bool pair = nearest[j] == i;
-        keep[i] = !pair || i < j;
+    const uint32_t n = *clusters;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < bound; i += gridDim.x * blockDim.x) {
+        const uint32_t j = i < n ? nearest[i] : 0u;
+        const bool pair = i < n && nearest[j] == i;
+        keep[i] = i < n && (!pair || i < j);
         if (!pair || i > j) continue;
-        const float4 alo = lo[i], ahi = hi[i], blo = lo[j], bhi = hi[j];
-        const uint32_t ra = __float_as_uint(alo.w), rb = __float_as_uint(blo.w), id = atomicAdd(next, 1u);
-        BvhNode nd;
-        nd.a = make_float4(alo.x, alo.y, alo.z, ahi.x);
-        nd.b = make_float4(ahi.y, ahi.z, blo.x, blo.y);
-        nd.c = make_float4(blo.z, bhi.x, bhi.y, bhi.z);
-        nd.child[0] = ra;
-        nd.child[1] = rb;
-        nd.pad[0] = nd.pad[1] = 0;
-        nodes[id] = nd;
-        count[id] = ((ra & kBvhLeafBit) ? 1u : count[ra]) + ((rb & kBvhLeafBit) ? 1u : count[rb]);
-        lo[i] = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), __uint_as_float(id));
-        hi[i] = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
+        float4 alo = lo[i], ahi = hi[i];
+        ploc_merge(alo, ahi, lo[j], hi[j], nodes, count, next);
+        lo[i] = alo;
+        hi[i] = ahi;
     }
 }
-__global__ void k_ploc_compact(const float4* __restrict__ lo, const float4* __restrict__ hi, uint32_t n,
-                               const uint32_t* __restrict__ keep, const uint32_t* __restrict__ at, float4* __restrict__ lo2,
-                               float4* __restrict__ hi2, uint32_t* __restrict__ left) {
+__global__ void k_ploc_compact(const float4* __restrict__ lo, const float4* __restrict__ hi,
+                               const uint32_t* __restrict__ clusters, const uint32_t* __restrict__ keep,
+                               const uint32_t* __restrict__ at, float4* __restrict__ lo2, float4* __restrict__ hi2,
+                               uint32_t* __restrict__ left) {
+    const uint32_t n = *clusters;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         if (i == n - 1) *left = at[i] + keep[i];
         if (!keep[i]) continue;
         lo2[at[i]] = lo[i];
         hi2[at[i]] = hi[i];
+    }
+}
+// All rounds from kPlocFinish clusters or fewer on, by one CTA in shared memory.  Launches and the look at
+// the number of clusters are most of a round's time there (45 us): creating a scene of 66 / 3000 /
+// 20,000 / 200,000 triangles took 1.12 / 1.89 / 3.42 / 4.66 ms with a look per round and five allocations,
+// 0.60 / 0.98 / 1.88 / 2.48 now.
+constexpr uint32_t kPlocFinish = 2048;
+constexpr int kPlocFinishBlock = 1024;
+constexpr size_t kPlocFinishSmem = kPlocFinish * (2 * sizeof(float4) + sizeof(uint32_t));
+__global__ void __launch_bounds__(kPlocFinishBlock) k_ploc_finish(const float4* __restrict__ lo, const float4* __restrict__ hi,
+                                                                  const uint32_t* __restrict__ clusters, uint32_t rounds,
+                                                                  BvhNode* nodes, uint32_t* count, uint32_t* next) {
+    extern __shared__ float4 s_box[];
+    float4 *const s_lo = s_box, *const s_hi = s_box + kPlocFinish;
+    uint32_t* const s_near = reinterpret_cast<uint32_t*>(s_box + 2 * kPlocFinish);
+    __shared__ uint32_t s_warp[kPlocFinishBlock / 32];
+    uint32_t n = *clusters;
+    for (uint32_t k = threadIdx.x; k < n; k += kPlocFinishBlock) {
+        s_lo[k] = lo[k];
+        s_hi[k] = hi[k];
+    }
+    __syncthreads();
+    for (; n > 1; ++rounds) {
+        const int radius = rounds < kPlocRounds ? kPlocRadius : 0;
+        const uint32_t per = n > kPlocFinishBlock ? 2 : 1, i0 = threadIdx.x * per;
+        for (uint32_t k = 0; k < per; ++k)
+            if (i0 + k < n) s_near[i0 + k] = ploc_partner(s_lo + i0 + k, s_hi + i0 + k, i0 + k, n, radius);
+        __syncthreads();
+        float4 vlo[2], vhi[2];
+        bool keep[2] = {false, false};
+#pragma unroll
+        for (uint32_t k = 0; k < 2; ++k) {
+            const uint32_t i = i0 + k;
+            if (k >= per || i >= n) continue;
+            const uint32_t j = s_near[i];
+            const bool pair = s_near[j] == i;
+            keep[k] = !pair || i < j;
+            if (!keep[k]) continue;
+            vlo[k] = s_lo[i];
+            vhi[k] = s_hi[i];
+            if (pair) ploc_merge(vlo[k], vhi[k], s_lo[j], s_hi[j], nodes, count, next);
+        }
+        uint32_t left, at = block_exclusive_scan<kPlocFinishBlock>(uint32_t(keep[0]) + uint32_t(keep[1]), s_warp, left);
+#pragma unroll
+        for (uint32_t k = 0; k < 2; ++k)
+            if (keep[k]) {
+                s_lo[at] = vlo[k];
+                s_hi[at++] = vhi[k];
+            }
+        n = left;
+        __syncthreads();
     }
 }
 
@@ -335,15 +403,19 @@ __device__ __forceinline__ WideChild wide_child(const BvhNode& nd, const uint32_
     c.count = (c.ref & kBvhLeafBit) ? 1u : count[c.ref];
     return c;
 }
-// counts: [0] nodes allocated, [1] triangles placed, [2] bits of the largest coordinate; root: the binary node of every wide node
-__global__ void __launch_bounds__(128) k_wide_level(const BvhNode* __restrict__ nodes, const uint32_t* __restrict__ count,
-                                                    const BvhTri* __restrict__ tris, const uint32_t* __restrict__ prim,
-                                                    uint32_t begin, uint32_t end, uint32_t level, uint32_t* __restrict__ root,
-                                                    uint32_t cap, WideNode* __restrict__ wide, WideTri* __restrict__ wtris,
-                                                    uint32_t* __restrict__ counts) {
-    const uint32_t w = begin + blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= end) return;
-    const float max_abs = __uint_as_float(counts[2]);
+// The build's numbers on the device: nodes allocated, triangles placed, bits of the largest coordinate,
+// clustered nodes, clusters of even and odd rounds; first node of every level of the collapse
+// (first[level + 1] ends it), CTAs of a level's launch that are done.
+struct BuildCounts {
+    uint32_t nodes, tris, max_abs, merged, clusters[2];
+    uint32_t first[kWideStack + 2], done[kWideStack];
+};
+// root: the binary node of every wide node
+__device__ __forceinline__ void wide_node(const BvhNode* __restrict__ nodes, const uint32_t* __restrict__ count,
+                                          const BvhTri* __restrict__ tris, const uint32_t* __restrict__ prim, uint32_t w,
+                                          uint32_t level, uint32_t* root, uint32_t cap, WideNode* __restrict__ wide,
+                                          WideTri* __restrict__ wtris, BuildCounts* counts) {
+    const float max_abs = __uint_as_float(counts->max_abs);
     WideChild c[8];
     int n = 2;
     {
@@ -426,8 +498,8 @@ __global__ void __launch_bounds__(128) k_wide_level(const BvhNode* __restrict__ 
     nd.lmask = lmask;
     nd.pad0 = 0;
     for (int q = 0; q < 4; ++q) nd.pad1[q] = 0;
-    nd.child_base = imask ? atomicAdd(counts, (uint32_t)__popc(imask)) : 0u;
-    nd.tri_base = lmask ? atomicAdd(counts + 1, (uint32_t)__popc(lmask)) : 0u;
+    nd.child_base = imask ? atomicAdd(&counts->nodes, (uint32_t)__popc(imask)) : 0u;
+    nd.tri_base = lmask ? atomicAdd(&counts->tris, (uint32_t)__popc(lmask)) : 0u;
     uint32_t child = nd.child_base, tri = nd.tri_base;
     for (int q = 0; q < 8; ++q) {
         const int k = in_slot[q];
@@ -456,6 +528,24 @@ __global__ void __launch_bounds__(128) k_wide_level(const BvhNode* __restrict__ 
     }
     wide[w] = nd;
 }
+__global__ void __launch_bounds__(128) k_wide_level(const BvhNode* __restrict__ nodes, const uint32_t* __restrict__ count,
+                                                    const BvhTri* __restrict__ tris, const uint32_t* __restrict__ prim,
+                                                    uint32_t level, uint32_t* root, uint32_t cap,
+                                                    WideNode* __restrict__ wide, WideTri* __restrict__ wtris,
+                                                    BuildCounts* counts) {
+    const uint32_t end = min(counts->first[level + 1], cap);
+    for (uint32_t w = counts->first[level] + blockIdx.x * blockDim.x + threadIdx.x; w < end; w += gridDim.x * blockDim.x)
+        wide_node(nodes, count, tris, prim, w, level, root, cap, wide, wtris, counts);
+    // the last CTA to finish tells where the level after the next begins
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(counts->done + level, 1u) == gridDim.x - 1)
+        counts->first[level + 2] = atomicAdd(&counts->nodes, 0u);
+}
+
+// rounds of clustering, or levels of the collapse, between two looks of the host at how far they are
+constexpr int kBuildLook = 4;
+static_assert(kWideStack % kBuildLook == 0 && (kPlocFinish >> kBuildLook) > 1, "looks end at the bounds");
 
 struct HitOut {
     float* t;
@@ -569,7 +659,8 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
     float4* ibox = nullptr;
     unsigned* flags = nullptr;
     BvhTri* tris = nullptr;  // the triangles in leaf order, and their scene indices
-    uint32_t *prim = nullptr, *root = nullptr, *counts = nullptr;
+    uint32_t *prim = nullptr, *root = nullptr;
+    BuildCounts* counts = nullptr;
     uint32_t *pcount = nullptr, *nearest = nullptr, *keep = nullptr, *at = nullptr;
     BvhNode* pnodes = nullptr;
     float4 *clo[2] = {nullptr, nullptr}, *chi[2] = {nullptr, nullptr};
@@ -579,11 +670,26 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
     // small scenes are a flat list; the others get both hierarchies
     const bool flat = n <= kFlatTris;
     const uint32_t wide_cap = n / 8 * 5 + 8;
-    if (n > 0 && (flat ? (r = s->alloc(&s->flat, flat_pairs(n)))
-                       : (r = s->alloc(&s->nodes, n - 1)) || (r = s->alloc(&s->leaf_box, 2 * size_t(n))) ||
-                             (r = s->alloc(&s->wide, wide_cap)) || (r = s->alloc(&s->wtris, n)))) {
+    if (n > 0 && flat && (r = s->alloc(&s->flat, flat_pairs(n)))) {
         delete s;
         return r;
+    }
+    // one allocation holds what rays read: each of more than 1 MB costs 0.3 ms
+    char* arrays = nullptr;
+    for (int pass = 0; pass < 2 && n > 0 && !flat; ++pass) {  // sizes, then places
+        size_t at_byte = 0;
+        auto take = [&](auto** p, size_t count) {
+            if (pass) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(arrays + at_byte);
+            at_byte += (count * sizeof(**p) + 255) & ~size_t(255);
+        };
+        take(&s->nodes, n - 1);
+        take(&s->leaf_box, 2 * size_t(n));
+        take(&s->wide, wide_cap);
+        take(&s->wtris, n);
+        if (!pass && (r = s->alloc(&arrays, at_byte))) {
+            delete s;
+            return r;
+        }
     }
     s->dev.nodes = s->nodes;
     s->dev.leaf_box = s->leaf_box;
@@ -624,7 +730,7 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
             take(&ibox, 2 * size_t(n));
             take(&flags, n);
             take(&root, wide_cap);
-            take(&counts, 5);
+            take(&counts, 1);
             take(&pcount, n);
             take(&nearest, n);
             take(&keep, n);
@@ -659,40 +765,48 @@ int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32
             k_scene_hierarchy<<<g, 256, 0, st>>>(dk.Current(), (int)n, s->nodes, pi, pl);
             if ((e = cudaMemsetAsync(flags, 0, 4ull * n, st))) break;
             k_scene_boxes<<<g, 256, 0, st>>>(vertices, indices, prim, n, s->nodes, pi, pl, ibox, flags);
-            // counts: wide nodes, triangles, largest absolute coordinate, clustered nodes, clusters
-            const uint32_t init_counts[5] = {1u, 0u, 0u, 0u, n};
-            if ((e = cudaMemcpyAsync(counts, init_counts, sizeof(init_counts), cudaMemcpyHostToDevice, st))) break;
-            k_scene_leaf_boxes<<<g, 256, 0, st>>>(vertices, indices, prim, n, s->leaf_box, counts + 2);
+            BuildCounts now{};
+            now.nodes = now.first[1] = 1;
+            now.clusters[0] = n;
+            if ((e = cudaMemcpyAsync(counts, &now, sizeof(now), cudaMemcpyHostToDevice, st))) break;
+            k_scene_leaf_boxes<<<g, 256, 0, st>>>(vertices, indices, prim, n, s->leaf_box, &counts->max_abs);
             k_ploc_init<<<g, 256, 0, st>>>(s->leaf_box, n, clo[0], chi[0]);
-            uint32_t clusters = n, rounds = 0;
-            for (; clusters > 1 && !e; ++rounds) {
-                const int a = rounds & 1, b = a ^ 1, gc = grid_for(clusters, 256, 8);
-                const int radius = rounds < kPlocRounds ? kPlocRadius : 0;
-                k_ploc_nearest<<<(clusters + kPlocBlock - 1) / kPlocBlock, kPlocBlock, 0, st>>>(clo[a], chi[a], clusters, radius, nearest);
-                k_ploc_merge<<<gc, 256, 0, st>>>(clo[a], chi[a], clusters, nearest, pnodes, pcount, counts + 3, keep);
-                if ((e = cub::DeviceScan::ExclusiveSum(scan_temp, scan_bytes, keep, at, (int)clusters, st))) break;
-                k_ploc_compact<<<gc, 256, 0, st>>>(clo[a], chi[a], clusters, keep, at, clo[b], chi[b], counts + 4);
-                if ((e = cudaMemcpyAsync(&clusters, counts + 4, 4, cudaMemcpyDeviceToHost, st))) break;
+            // a round at most halves the clusters, so kBuildLook of them leave more than one
+            uint32_t bound = n, rounds = 0;
+            while (bound > kPlocFinish && !e) {
+                const int gn = (int)((bound + kPlocBlock - 1) / kPlocBlock), gc = grid_for(bound, 256, 8);
+                for (int k = 0; k < kBuildLook && !e; ++k, ++rounds) {
+                    const int a = rounds & 1, b = a ^ 1, radius = rounds < kPlocRounds ? kPlocRadius : 0;
+                    k_ploc_nearest<<<gn, kPlocBlock, 0, st>>>(clo[a], chi[a], counts->clusters + a, radius, nearest);
+                    k_ploc_merge<<<gc, 256, 0, st>>>(clo[a], chi[a], counts->clusters + a, bound, nearest, pnodes, pcount,
+                                                     &counts->merged, keep);
+                    if ((e = cub::DeviceScan::ExclusiveSum(scan_temp, scan_bytes, keep, at, (int)bound, st))) break;
+                    k_ploc_compact<<<gc, 256, 0, st>>>(clo[a], chi[a], counts->clusters + a, keep, at, clo[b], chi[b],
+                                                       counts->clusters + b);
+                }
+                if (e || (e = cudaMemcpyAsync(&bound, counts->clusters + (rounds & 1), 4, cudaMemcpyDeviceToHost, st))) break;
                 e = cudaStreamSynchronize(st);
             }
-            if (e) break;
+            if (e || (e = cudaFuncSetAttribute(k_ploc_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlocFinishSmem))) break;
+            k_ploc_finish<<<1, kPlocFinishBlock, kPlocFinishSmem, st>>>(clo[rounds & 1], chi[rounds & 1],
+                                                                      counts->clusters + (rounds & 1), rounds, pnodes, pcount,
+                                                                      &counts->merged);
             const uint32_t bin_root = n - 2;  // made last
             if ((e = cudaMemcpyAsync(root, &bin_root, 4, cudaMemcpyHostToDevice, st))) break;
-            uint32_t begin = 0, end = 1, now[3] = {1, 0, 0};
-            for (uint32_t level = 0; begin < end; ++level) {
-                if (level >= (uint32_t)kWideStack || end > wide_cap) {
-                    rc = fail(RTPG_ECAPACITY, "rtpg_scene_create: hierarchy of %u nodes in %u levels exceeds its bounds", end, level);
-                    break;
-                }
-                k_wide_level<<<(end - begin + 127) / 128, 128, 0, st>>>(pnodes, pcount, tris, prim, begin, end, level, root,
-                                                                       wide_cap, s->wide, s->wtris, counts);
-                if ((e = cudaMemcpyAsync(now, counts, sizeof(now), cudaMemcpyDeviceToHost, st))) break;
+            const int gw = (int)std::min<uint32_t>((wide_cap + 127) / 128, kSMs * 16);
+            uint32_t level = 0;
+            do {
+                for (int k = 0; k < kBuildLook; ++k, ++level)
+                    k_wide_level<<<gw, 128, 0, st>>>(pnodes, pcount, tris, prim, level, root, wide_cap, s->wide, s->wtris, counts);
+                if ((e = cudaMemcpyAsync(&now, counts, sizeof(now), cudaMemcpyDeviceToHost, st))) break;
                 if ((e = cudaStreamSynchronize(st))) break;
-                begin = end;
-                end = now[0];
+            } while (now.first[level + 1] > now.first[level] && now.nodes <= wide_cap && level < (uint32_t)kWideStack);
+            if (e) break;
+            if (now.first[level + 1] > now.first[level] || now.nodes > wide_cap) {
+                rc = fail(RTPG_ECAPACITY, "rtpg_scene_create: hierarchy of %u nodes in %u levels exceeds its bounds", now.nodes, level);
+                break;
             }
-            if (e || rc) break;
-            memcpy(&s->dev.max_abs, &now[2], 4);
+            memcpy(&s->dev.max_abs, &now.max_abs, 4);
         }
         if ((e = cudaGetLastError())) break;
         if ((e = cudaStreamSynchronize(st))) break;

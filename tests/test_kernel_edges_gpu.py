@@ -509,3 +509,26 @@ def test_hierarchy_of_nested_triangles(cuda, oracle, nested, others):
     for i in np.flatnonzero(got_p != want_p):
         alone = oracle.intersect(tri[got_p[i]:got_p[i] + 1], org[i:i + 1], d[i:i + 1], 0.0, 1e20)[0]
         assert alone[0] == want_t[i]
+
+
+@pytest.mark.parametrize("n", [65, 1024, 1025, 2048, 2049, 4097, 33000])
+def test_hierarchy_build_sizes(cuda, oracle, n):
+    """Clustering by one CTA (up to 2048 clusters, one or two a thread) and by launches of all SMs before
+    that: every triangle is found."""
+    import torch
+    from rtlib_b200.tracer import Scene
+    rng = np.random.default_rng(n)
+    centre = rng.uniform(-3, 3, (n, 1, 3))
+    tri = (rng.normal(size=(n, 3, 3)) * 0.02 + centre).astype(np.float32).reshape(n, 9)
+    q = min(n, 3000)
+    aim = rng.permutation(n)[:q]  # rays at as many triangles
+    org = rng.uniform(-4, 4, (q, 3)).astype(np.float32)
+    d = tri[aim].reshape(q, 3, 3).mean(1) - org
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    sc = Scene(_t(tri, cuda))
+    t, p = torch.empty(q, device=cuda), torch.empty(q, dtype=torch.int32, device=cuda)
+    sc.intersect(_t(org, cuda), _t(d, cuda), out_t=t, out_prim=p)
+    want_t, want_p = oracle.intersect(tri, org, d, 0.0, 1e20)[:2]
+    np.testing.assert_array_equal(p.cpu().numpy().view(np.uint32), want_p)
+    np.testing.assert_array_equal(t.cpu().numpy(), want_t)
+    assert (want_p != 0xFFFFFFFF).mean() > 0.99
