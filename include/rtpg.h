@@ -283,7 +283,8 @@ int rtpg_mlp_eval(rtpg_mlp* h, int64_t n, const float* pos, const float* nrm, co
 int rtpg_mlp_loss_grad(rtpg_mlp* h, int64_t n, const float* pos, const float* nrm, const float* wo, const float* wi,
                        const float* w, float* grads, float* host_loss, void* stream);
 /* epochs x (n / batch) Adam steps on the given records, or on the record buffer when pos is
- * NULL; host_last_loss: the last minibatch's loss (NULL: not read) */
+ * NULL; host_last_loss: the last minibatch's loss (NULL: not read).  The same records in the same
+ * order give the same parameters and loss bit for bit. */
 int rtpg_mlp_train(rtpg_mlp* h, int64_t n, const float* pos, const float* nrm, const float* wo, const float* wi,
                    const float* w, uint32_t batch, uint32_t epochs, float* host_last_loss, void* stream);
 /* records written so far (may exceed the capacity: the excess was dropped); clear = 1 empties */
@@ -302,15 +303,19 @@ int rtpg_mlp_set_wait_test(rtpg_mlp* h, int skip_mma, uint32_t poll_limit);
 
 /* ================================================================ scene / hit queries
  * The integrator's closest-hit and any-hit queries (RTLib: optixTrace inside TraceRadiance /
- * TraceOccluded, RTLib/Src/Ext/OPX7/Test/cuda/SimpleKernel.h:347-366, "SK.h") answered by a
- * linear BVH built on the GPU.  vertices: num_vertices x float3; indices: num_triangles x
- * uint3 (device).  Creation synchronises the stream. */
+ * TraceOccluded, RTLib/Src/Ext/OPX7/Test/cuda/SimpleKernel.h:347-366, "SK.h").  Scenes of at most
+ * 64 triangles are a flat list, larger ones an eight-wide hierarchy built on the GPU (about 220
+ * bytes a triangle).  vertices: num_vertices x float3; indices: num_triangles x uint3 (device).
+ * Creation synchronises the stream. */
 typedef struct rtpg_scene rtpg_scene;
 int rtpg_scene_create(const float* vertices, uint32_t num_vertices, const uint32_t* indices, uint32_t num_triangles,
                       void* stream, rtpg_scene** out);
 int rtpg_scene_destroy(rtpg_scene* s);
 /* Batched queries: ray n has origin org[3n..], direction dir[3n..], interval (tmin, tmax)
- * (NULL = 0 / 1e20).  any_hit = 0: closest hit (TraceRadiance), 1: any hit (TraceOccluded).
+ * (NULL = 0 / 1e20).  any_hit = 0: closest hit (TraceRadiance); of triangles at exactly the same
+ * distance the lowest index in a flat list, in a hierarchy the one that a near-first walk of the
+ * linear (Morton-order) hierarchy meets first.  any_hit = 1: some hit (TraceOccluded); where a ray
+ * hits several triangles any of them may be reported.
  * out_t = -1 and out_prim = UINT32_MAX on a miss; out_uv: barycentrics (u, v) of vertices
  * 1 and 2 (float2).  Outputs optional. */
 int rtpg_scene_intersect(rtpg_scene* s, int64_t n, const float* org, const float* dir, const float* tmin,
@@ -414,10 +419,11 @@ int rtpg_tracer_set_light_emission(rtpg_tracer* h, const float* host_rgb, uint32
  *   grad_texture        3 floats per texel of diffuse texture texture_index (-1: none);
  *   grad_light_emission 3 floats per light mesh (NULL: none).
  * flags: 0 or RTPG_TRACE_FLAG_NEE (RIS resampling depends on the radiances, guiding on
- * recorded radiance; neither is differentiated).  Per sample, one primal wave recomputes every
- * path's radiance and one adjoint wave replays the path, subtracting each term as it passes
- * it: nothing per vertex is stored.  The accumulation is not touched; the streams advance
- * as the render would advance them. */
+ * recorded radiance; neither is differentiated).  One launch per sample: a primal pass forms every
+ * path's radiance and keeps what its rays hit (in the trace-vertex arrays of the last recording
+ * wave, which it overwrites), then the path is replayed from that, subtracting each term as it passes
+ * it.  The accumulation is not touched; the streams advance as the render would advance
+ * them. */
 int rtpg_tracer_render_adjoint(rtpg_tracer* h, uint32_t spp, uint32_t flags, const float* d_image,
                                int32_t texture_index, float* grad_texture, float* grad_light_emission, void* stream);
 /* mean radiance per pixel, width x height x RGB float (device) */
@@ -432,7 +438,10 @@ int rtpg_tracer_counters(rtpg_tracer* h, uint64_t* host_path_bounces, uint64_t* 
 /* Measurement mode: enable = 1 makes rtpg_tracer_render launch waves without the CUDA graph,
  * bracket every kernel with CUDA events on the stream and synchronise per wave; the summed
  * device milliseconds of raygen / bounce / finish (and their launch counts) are read into
- * three-element arrays with rtpg_tracer_timings.  Enabling or disabling resets the sums. */
+ * three-element arrays with rtpg_tracer_timings.  Enabling or disabling resets the sums.  The mode
+ * always launches a kernel per bounce; without it, images of at most 132,608 paths (seven CTAs of
+ * 128 per SM) run a path per thread in one kernel unless the learned guide is used, with the same
+ * results, which the mode does not time. */
 int rtpg_tracer_set_timing(rtpg_tracer* h, int enable);
 /* Debug view: the final bounce index of every path of the last wave (uint32 per pixel,
  * device); with recording on, a path commits min(depth, 10) trace vertices. */

@@ -124,13 +124,6 @@ __device__ __forceinline__ void tmem_ld8_async(uint32_t taddr, uint32_t* r) {
                  : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-    uint32_t r[16];
-    tmem_ld16_async(taddr, r);
-    tmem_wait_ld();
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
 // N (a multiple of 8, at most 64) columns with the loads in flight together
 template <int N>
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, float* v) {
@@ -194,26 +187,8 @@ struct VmfLobe {
     float3 mu;
     float kappa, weight;
 };
-// raw network outputs of one sample -> lobes (normalised mean, kappa = exp(clamped), softmax)
-__device__ __forceinline__ void mlp_head(const float* o, VmfLobe* L) {
-    float mx = -1e30f;
-#pragma unroll
-    for (int k = 0; k < kMlpLobes; ++k) mx = fmaxf(mx, o[5 * k + 4]);
-    float se = 0.0f;
-#pragma unroll
-    for (int k = 0; k < kMlpLobes; ++k) {
-        const float3 m = f3(o[5 * k], o[5 * k + 1], o[5 * k + 2]);
-        const float len = sqrtf(dot3(m, m));
-        L[k].mu = len > 1e-12f ? m * (1.0f / len) : f3(0.f, 0.f, 1.f);
-        L[k].kappa = __expf(fminf(fmaxf(o[5 * k + 3], kLogKappaMin), kLogKappaMax));
-        L[k].weight = __expf(o[5 * k + 4] - mx);
-        se += L[k].weight;
-    }
-    const float inv = 1.0f / se;
-#pragma unroll
-    for (int k = 0; k < kMlpLobes; ++k) L[k].weight *= inv;
-}
-// the same for the four lobes of one half (k = 4 half .. 4 half + 3) only
+// Raw network outputs of one sample -> the four lobes of one half (k = 4 half .. 4 half + 3):
+// normalised mean, kappa = exp(clamped), weight by the softmax over all eight.
 __device__ __forceinline__ void mlp_head_half(const float* o, bool hi, VmfLobe* L) {
     float mx = -1e30f;
 #pragma unroll
