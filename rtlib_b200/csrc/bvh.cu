@@ -483,21 +483,20 @@ __device__ __forceinline__ void wide_node(const BvhNode* __restrict__ nodes, con
         (c[k].count > 1 ? imask : lmask) |= 1u << slot_of[k];
     }
     WideNode nd;
-    // planes: a step of at least 2 ulp of the coordinates, origin one step below the box
+    // planes: q = 0 and q = 255 on the box, a step of at least 2 ulp of the coordinates
     double step[3];
-    nd.exp = imask << 24;
+    nd.imask = imask;
     for (int a = 0; a < 3; ++a) {
-        int e = -100, m = 0;
-        if (hi[a] > lo[a]) frexp(((double)hi[a] - (double)lo[a]) / 250.0, &e);
+        int m = 0;
         frexp(fmax(fabs((double)lo[a]), fabs((double)hi[a])), &m);
-        e = max(max(e, m - 22), -100);
-        step[a] = ldexp(1.0, e);
-        nd.org[a] = (float)((double)lo[a] - step[a]);
-        nd.exp |= uint32_t(min(e + 127, 254)) << (8 * a);
+        const float least = fmaxf((float)ldexp(1.0, m - 22), 0x1p-100f);
+        nd.step[a] = fmaxf(__double2float_ru(((double)hi[a] - (double)lo[a]) / 255.0), least);
+        step[a] = nd.step[a];
+        nd.org[a] = lo[a];
     }
     nd.lmask = lmask;
     nd.pad0 = 0;
-    for (int q = 0; q < 4; ++q) nd.pad1[q] = 0;
+    nd.pad1 = 0;
     nd.child_base = imask ? atomicAdd(&counts->nodes, (uint32_t)__popc(imask)) : 0u;
     nd.tri_base = lmask ? atomicAdd(&counts->tris, (uint32_t)__popc(lmask)) : 0u;
     uint32_t child = nd.child_base, tri = nd.tri_base;
@@ -510,8 +509,8 @@ __device__ __forceinline__ void wide_node(const BvhNode* __restrict__ nodes, con
         if (k < 0) continue;
         for (int a = 0; a < 3; ++a) {
             const double x0 = ((double)c[k].lo[a] - (double)nd.org[a]) / step[a], x1 = ((double)c[k].hi[a] - (double)nd.org[a]) / step[a];
-            nd.qlo[a][q] = (uint8_t)fmin(fmax(floor(x0 - 0.015625), 0.0), 255.0);
-            nd.qhi[a][q] = (uint8_t)fmin(fmax(ceil(x1 + 0.015625), 0.0), 255.0);
+            nd.qlo[a][q] = (uint8_t)fmin(fmax(floor(x0), 0.0), 255.0);
+            nd.qhi[a][q] = (uint8_t)fmin(fmax(ceil(x1), 0.0), 255.0);
         }
         if (imask >> q & 1u) {
             if (child < cap) root[child] = c[k].ref;

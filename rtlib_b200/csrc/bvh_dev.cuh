@@ -67,19 +67,26 @@ __host__ __device__ constexpr uint32_t flat_pairs(uint32_t n) { return (n + 1) /
 // Traversal on GPUs Through Compressed Wide BVHs" (HPG 2017): up to eight children in slots that
 // follow the octants of the node, so that visiting slot (k xor octant) for descending k is about
 // front to back for every ray octant, without sorting.  96 bytes = three 32-byte loads.
-//   org, exp   child box plane q of axis a lies at org[a] + q * 2^(exp byte a - 127)
-//   imask      (top byte of exp) slots that hold interior children, stored one after the other
-//              from child_base in slot order
+//   org, step  planes of axis a: a lower one at org[a] + (q - kPlaneMargin) * step[a], an upper one at
+//              org[a] + (q + kPlaneMargin) * step[a]; q = 0 and 255 lie on the node's own box, so that walls
+//              there stay thin
+//   imask      slots that hold interior children, stored one after the other from child_base in
+//              slot order
 //   lmask      slots that hold a triangle, stored one after the other from tri_base in slot order
-//   qlo, qhi   per axis and slot, rounded outwards by at least 1/64 of a step
+//   qlo, qhi   per axis and slot, rounded outwards
 // A leaf is one triangle: more of them per leaf cost more tests than they save nodes (closest hits
 // of 2^20 rays in 1.05 M triangles: 1493 us with one, 1492 with two, 1596 with three).
+// With steps that are powers of two and planes rounded outwards by up to a step, a wall of a node's box was
+// a slab as thick as two steps, entered by every ray that starts or ends on it: next event estimation in Cornell
+// boxes whose light is 32 / 512 / 2048 triangles took 1-6 % longer than with two exact boxes a node (1280 x 720,
+// 8 samples: 8.63 / 9.31 / 10.40 ms): 8.81 / 9.61 / 11.04 then, 8.46 / 9.11 / 10.53 now.
+constexpr float kPlaneMargin = 0.03125f;
 struct __align__(32) WideNode {
     float org[3];
-    uint32_t exp;
-    uint32_t child_base, tri_base, lmask, pad0;
+    uint32_t imask, child_base, tri_base, lmask, pad0;
     uint8_t qlo[3][8], qhi[3][8];
-    uint32_t pad1[4];
+    float step[3];
+    uint32_t pad1;
 };
 static_assert(sizeof(WideNode) == 96, "three 32-byte sectors");
 // A leaf triangle of the walked hierarchy: its rows, its leaf in the binary hierarchy and its scene
@@ -287,20 +294,18 @@ __device__ __forceinline__ float plane(uint32_t w) {
 // by what rounding can do.  Whatever leaf box passes box_hit must not be lost to a quantised box
 // around it: box_hit's slab distances are off by at most 2^-23 (|o| + |plane|) |1/d|, the ones
 // here by as much again, so planes are moved apart by 2^-21 (|o| + max_abs), (a ten-thousandth
-// of a millimetre per metre of scene).  The step 32768 q adds 2^-9 of a quantisation step, which
-// the boxes' 1/64 covers.
+// of a millimetre per metre of scene).  Forming 32768 + q and the products with the step adds less than
+// 2^-7 of a quantisation step, which kPlaneMargin covers.
 struct WideRay {
     RayInv inv;
-    float nx, ny, nz, fx, fy, fz;  // origin product, plus (near planes) and minus (far) the widening
+    float px, py, pz, ex, ey, ez;  // origin product, widening
     uint32_t octinv;               // 7 - octant: bit a set where the direction is positive
     __device__ __forceinline__ WideRay(const SceneDev& s, float ox, float oy, float oz, float dx, float dy, float dz)
         : inv(dx, dy, dz) {
-        const float ex = 0x1p-21f * (fabsf(ox) + s.max_abs) * fabsf(inv.ix);
-        const float ey = 0x1p-21f * (fabsf(oy) + s.max_abs) * fabsf(inv.iy);
-        const float ez = 0x1p-21f * (fabsf(oz) + s.max_abs) * fabsf(inv.iz);
-        const float px = ox * inv.ix, py = oy * inv.iy, pz = oz * inv.iz;
-        nx = px + ex; ny = py + ey; nz = pz + ez;
-        fx = px - ex; fy = py - ey; fz = pz - ez;
+        ex = 0x1p-21f * (fabsf(ox) + s.max_abs) * fabsf(inv.ix);
+        ey = 0x1p-21f * (fabsf(oy) + s.max_abs) * fabsf(inv.iy);
+        ez = 0x1p-21f * (fabsf(oz) + s.max_abs) * fabsf(inv.iz);
+        px = ox * inv.ix; py = oy * inv.iy; pz = oz * inv.iz;
         octinv = (inv.ix < 0.0f ? 0u : 1u) | (inv.iy < 0.0f ? 0u : 2u) | (inv.iz < 0.0f ? 0u : 4u);
     }
 };
@@ -315,17 +320,15 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
     asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
-// Slots of the node's children whose box the ray may hit in [tmin, tmax]; v: the node's first 80
-// bytes.  The mask is summed in the mantissa of a float, off the integer pipe that the byte
+// Slots of the node's children whose box the ray may hit in [tmin, tmax]; v: the node.  The mask is summed in the mantissa of a float, off the integer pipe that the byte
 // permutes and the min / max keep busy.
 __device__ __forceinline__ uint32_t wide_hits(const WideRay& r, const uint32_t* v, float tmin, float tmax) {
     const float px = __uint_as_float(v[0]), py = __uint_as_float(v[1]), pz = __uint_as_float(v[2]);
-    const float sx = __uint_as_float((v[3] & 0xffu) << 23) * r.inv.ix;
-    const float sy = __uint_as_float((v[3] >> 8 & 0xffu) << 23) * r.inv.iy;
-    const float sz = __uint_as_float((v[3] >> 16 & 0xffu) << 23) * r.inv.iz;
-    const float nx = __fmaf_rn(-32768.0f, sx, __fmaf_rn(px, r.inv.ix, -r.nx)), fx = __fmaf_rn(-32768.0f, sx, __fmaf_rn(px, r.inv.ix, -r.fx));
-    const float ny = __fmaf_rn(-32768.0f, sy, __fmaf_rn(py, r.inv.iy, -r.ny)), fy = __fmaf_rn(-32768.0f, sy, __fmaf_rn(py, r.inv.iy, -r.fy));
-    const float nz = __fmaf_rn(-32768.0f, sz, __fmaf_rn(pz, r.inv.iz, -r.nz)), fz = __fmaf_rn(-32768.0f, sz, __fmaf_rn(pz, r.inv.iz, -r.fz));
+    const float sx = __uint_as_float(v[20]) * r.inv.ix, sy = __uint_as_float(v[21]) * r.inv.iy, sz = __uint_as_float(v[22]) * r.inv.iz;
+    const float mx = kPlaneMargin * fabsf(sx), my = kPlaneMargin * fabsf(sy), mz = kPlaneMargin * fabsf(sz);
+    const float ox = __fmaf_rn(-32768.0f, sx, __fmaf_rn(px, r.inv.ix, -r.px)), oy = __fmaf_rn(-32768.0f, sy, __fmaf_rn(py, r.inv.iy, -r.py)),
+                oz = __fmaf_rn(-32768.0f, sz, __fmaf_rn(pz, r.inv.iz, -r.pz));
+    const float nx = ox - (mx + r.ex), fx = ox + (mx + r.ex), ny = oy - (my + r.ey), fy = oy + (my + r.ey), nz = oz - (mz + r.ez), fz = oz + (mz + r.ez);
     const bool bx = r.inv.ix < 0.0f, by = r.inv.iy < 0.0f, bz = r.inv.iz < 0.0f;
     float hits = 8388608.0f;  // 2^23: its last eight bits are the mask
 #pragma unroll
@@ -388,11 +391,8 @@ struct WideWalk {
             const char* const p = reinterpret_cast<const char*>(s.wide + node);
             ld32(p, v);
             ld32(p + 32, v + 8);
-            {
-                const uint4 w = __ldg(reinterpret_cast<const uint4*>(p + 64));
-                v[16] = w.x; v[17] = w.y; v[18] = w.z; v[19] = w.w;
-            }
-            const uint32_t hits = wide_hits(r, v, tmin, h.t), imask = v[3] >> 24;
+            ld32(p + 64, v + 16);
+            const uint32_t hits = wide_hits(r, v, tmin, h.t), imask = v[3];
             g = make_uint2(v[4], octant_order(hits & imask, r.octinv) << 24 | imask);
             tri_base = v[5];
             lmask = v[6];

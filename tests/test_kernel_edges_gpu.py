@@ -532,3 +532,48 @@ def test_hierarchy_build_sizes(cuda, oracle, n):
     np.testing.assert_array_equal(p.cpu().numpy().view(np.uint32), want_p)
     np.testing.assert_array_equal(t.cpu().numpy(), want_t)
     assert (want_p != 0xFFFFFFFF).mean() > 0.99
+
+
+@pytest.mark.parametrize("scale,offset", [(1.0, 0.0), (1e-3, 0.0), (1e3, 0.0), (1.0, 50.0), (1e-3, 0.05)])
+def test_hierarchy_planes_keep_every_hit(cuda, oracle, scale, offset):
+    """Quantised boxes of nodes whose children lie on their walls (a room of many small tiles, flat boxes
+    that share planes), at several scales and away from the origin; rays start on the walls and run
+    along them: hits equal brute force."""
+    import torch
+    from rtlib_b200.tracer import Scene
+    rng = np.random.default_rng(int(scale * 1000) + int(offset * 100))
+    k = 12
+    g = (np.stack(np.meshgrid(np.arange(k), np.arange(k), indexing="ij"), -1).reshape(-1, 2) / k).astype(np.float32)
+    quads = []
+    for axis in range(3):
+        for side in (0.0, 1.0):
+            c = np.empty((len(g), 4, 3), np.float32)
+            for j, (du, dv) in enumerate(((0, 0), (1, 0), (1, 1), (0, 1))):
+                c[:, j, axis] = side
+                c[:, j, (axis + 1) % 3] = g[:, 0] + du / k
+                c[:, j, (axis + 2) % 3] = g[:, 1] + dv / k
+            quads.append(c)
+    c = np.concatenate(quads)
+    tri = np.concatenate([c[:, [0, 1, 2]], c[:, [0, 2, 3]]])
+    inner = rng.normal(size=(300, 3, 3)) * 0.05 + rng.uniform(0.2, 0.8, (300, 1, 3))
+    tri = (np.concatenate([tri, inner.astype(np.float32)]) * np.float32(scale) + np.float32(offset)).astype(np.float32).reshape(-1, 9)
+    q = 6000
+    on = tri.reshape(-1, 3, 3)[rng.integers(0, len(tri), (2, q))]
+    b = rng.dirichlet((1, 1, 1), (2, q, 1))[:, :, 0, :, None]
+    p = (on * b).sum(2).astype(np.float32)  # points of two triangles: from one towards the other
+    org, d = p[0], p[1] - p[0]
+    far = np.linalg.norm(d, axis=1)
+    keep = far > 1e-2 * scale
+    org, d = org[keep], (d[keep] / far[keep, None]).astype(np.float32)
+    sc = Scene(_t(tri, cuda))
+    n = len(org)
+    t, prim, occ = torch.empty(n, device=cuda), torch.empty(n, dtype=torch.int32, device=cuda), torch.empty(n, dtype=torch.int32, device=cuda)
+    tmin, tmax = np.float32(1e-4 * scale), np.float32(10.0 * scale)
+    lo, hi = _t(np.full(n, tmin), cuda), _t(np.full(n, tmax), cuda)
+    sc.intersect(_t(org, cuda), _t(d, cuda), lo, hi, out_t=t, out_prim=prim)
+    sc.intersect(_t(org, cuda), _t(d, cuda), lo, hi, any_hit=True, out_prim=occ)
+    want_t, want_p = oracle.intersect(tri, org, d, tmin, tmax)[:2]
+    hit = want_p != 0xFFFFFFFF
+    np.testing.assert_array_equal(prim.cpu().numpy().view(np.uint32) != 0xFFFFFFFF, hit)
+    np.testing.assert_array_equal(t.cpu().numpy()[hit], want_t[hit])
+    np.testing.assert_array_equal(occ.cpu().numpy() != -1, hit)
