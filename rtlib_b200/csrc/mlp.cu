@@ -335,8 +335,8 @@ struct GradRows {
 };
 // Launches of kGradCtas CTAs of 256 threads: the first kMlpParams / 32 have a parameter per lane, whose
 // rows their eight warps sum side by side, the last sums the loss.  Sums in double, in a fixed order.
-// 16 steps of 16384 records (128 rows, 8.4 MB a step that stay in the L2): 317 us, as with float
-// atomics into one accumulator.
+// 16 steps of 16384 records (128 rows, 8.4 MB a step that stay in the L2): 319 us, 317 with float
+// atomics into one accumulator (303 and 293 from a flushed L2).
 constexpr int kGradCtas = kMlpParams / 32 + 1, kGradWarps = 8;
 // The sum over all rows of parameter i = blockIdx.x * 32 + lane, in warp 0 (false elsewhere and in
 // the CTA of the loss).  All threads call it.
