@@ -404,6 +404,7 @@ struct rtpg_mlp {
     float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
     float* loss = nullptr;     // of the newest step, behind the gradients
     float* scratch = nullptr;  // kTrainScratch floats (scratch_alloc)
+    int device = 0;            // of scratch
     __nv_bfloat16* wq = nullptr;
     float lr = 1e-3f, b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     uint32_t step = 0;
@@ -429,8 +430,12 @@ struct rtpg_mlp {
     ~rtpg_mlp() {
         for (void* p : allocs) cudaFree(p);
         if (scratch) {
+            int cur = device;
+            cudaGetDevice(&cur);
+            if (cur != device) cudaSetDevice(device);
             cudaDeviceSynchronize();  // memory of a pool is freed without waiting for its last use
             cudaFree(scratch);
+            if (cur != device) cudaSetDevice(cur);
         }
     }
 };
@@ -455,6 +460,7 @@ static int scratch_alloc(rtpg_mlp* h) {
         RTPG_CUDA(cudaMemPoolCreate(&pool, &props));
         RTPG_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept));
     }
+    h->device = dev;
     const cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&h->scratch), sizeof(float) * kTrainScratch, pool, nullptr);
     if (e != cudaSuccess) {
         cudaGetLastError();

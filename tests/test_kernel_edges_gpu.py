@@ -577,3 +577,29 @@ def test_hierarchy_planes_keep_every_hit(cuda, oracle, scale, offset):
     np.testing.assert_array_equal(prim.cpu().numpy().view(np.uint32) != 0xFFFFFFFF, hit)
     np.testing.assert_array_equal(t.cpu().numpy()[hit], want_t[hit])
     np.testing.assert_array_equal(occ.cpu().numpy() != -1, hit)
+
+
+def test_training_scratch_is_given_back(cuda):
+    """Forty guides at once hold 9.8 MB of training scratch each; when they are gone at most the 32 MB that
+    the pool keeps stay with the process (and what the allocator rounds up to), and new guides train on
+    it as on new memory."""
+    import torch
+    from rtlib_b200.mlp import MLPGuide
+    rec = _records(5000, 3, cuda)
+    def train():
+        g = MLPGuide((0, 0, 0), (1, 1, 1), seed=9)
+        return g.train(rec, batch=2000, epochs=1), g.params()
+    want = train()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    guides = [MLPGuide((0, 0, 0), (1, 1, 1), seed=k) for k in range(40)]
+    for g in guides:
+        g.train(rec, batch=2000, epochs=1)
+    held = before - torch.cuda.mem_get_info()[0]
+    del guides, g
+    torch.cuda.synchronize()
+    kept = before - torch.cuda.mem_get_info()[0]
+    assert held > 300e6 and kept < 80e6, (held, kept)
+    got = train()
+    assert got[0] == want[0]
+    np.testing.assert_array_equal(got[1], want[1])
