@@ -301,12 +301,27 @@ __global__ void __launch_bounds__(256) k_mqt_pdf(MqtDev t, int64_t n, const uint
     }
 }
 
+// ------------------------------------------------------------------ export
+// Floats [at, at + m) of the pyramids without their rows' shift.  Rows copied to host memory one by one
+// (a strided copy) take twice to seven times as long as one run of bytes, so a chunk is packed first:
+// 2^20 trees of level 3 with their leaves 348 -> 188 ms, 2^18 of level 2 60.7 -> 8.7 ms (178 and 7.9 as
+// one run).
+constexpr size_t kExportFloats = 1u << 18;  // 1 MB: allocations past that cost 0.3 ms
+__global__ void __launch_bounds__(256) k_mqt_pack(MqtDev t, uint64_t at, uint32_t m, float* __restrict__ out) {
+    const uint32_t per = mqt_level_offset(t.level + 1);
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
+        const uint64_t c = (at + k) / per;
+        out[k] = t.pyramid[c * mqt_stride(t.level) + kMqtShift + ((at + k) - c * per)];
+    }
+}
+
 }  // namespace rtpg
 
 using namespace rtpg;
 
 struct rtpg_mqt {
     MqtDev dev{};
+    float* staging = nullptr;  // of exports: kExportFloats, or all there are
     std::vector<void*> allocs;
     size_t bytes = 0;
     template <class T>
@@ -346,7 +361,8 @@ int rtpg_mqt_create(uint32_t num_cells, uint32_t level, float fraction, int32_t 
     const size_t nleaf = (size_t)num_cells << (2 * level), npyr = (size_t)num_cells * mqt_stride(level);
     int r;
     if ((r = h->alloc(&t.leaves, nleaf)) || (r = h->alloc(&t.pyramid, npyr)) || (r = h->alloc(&t.status, 1)) ||
-        (r = h->alloc(&t.touched, num_cells)) || (r = h->alloc(&t.live, num_cells))) {
+        (r = h->alloc(&t.touched, num_cells)) || (r = h->alloc(&t.live, num_cells)) ||
+        (r = h->alloc(&h->staging, std::min<size_t>(kExportFloats, (size_t)num_cells * mqt_level_offset(level + 1))))) {
         delete h;
         return r;
     }
@@ -463,9 +479,13 @@ int rtpg_mqt_export(rtpg_mqt* h, int64_t* host_leaves, float* host_pyramid, void
     if (host_leaves)
         RTPG_CUDA(cudaMemcpyAsync(host_leaves, t.leaves, ((size_t)t.ncells << (2 * t.level)) * 8, cudaMemcpyDeviceToHost, st));
     if (host_pyramid) {
-        const size_t row = (size_t)mqt_level_offset(t.level + 1) * 4;
-        RTPG_CUDA(cudaMemcpy2DAsync(host_pyramid, row, t.pyramid + kMqtShift, (size_t)mqt_stride(t.level) * 4, row, t.ncells,
-                                    cudaMemcpyDeviceToHost, st));
+        const uint64_t n = (uint64_t)t.ncells * mqt_level_offset(t.level + 1);
+        for (uint64_t at = 0; at < n; at += kExportFloats) {
+            const uint32_t m = (uint32_t)std::min<uint64_t>(kExportFloats, n - at);
+            k_mqt_pack<<<grid_for(m, 256, 8), 256, 0, st>>>(t, at, m, h->staging);
+            RTPG_LAUNCH_CHECK();
+            RTPG_CUDA(cudaMemcpyAsync(host_pyramid + at, h->staging, (size_t)m * 4, cudaMemcpyDeviceToHost, st));
+        }
     }
     RTPG_CUDA(cudaStreamSynchronize(st));
     return RTPG_OK;

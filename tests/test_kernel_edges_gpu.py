@@ -603,3 +603,23 @@ def test_training_scratch_is_given_back(cuda):
     got = train()
     assert got[0] == want[0]
     np.testing.assert_array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("ncell,level", [(1, 1), (52429, 1), (12483, 2), (50000, 2), (3084, 3), (13, 7)])
+def test_morton_export_chunks(cuda, oracle, ncell, level):
+    """Pyramids leave the device in chunks of 2^18 floats: less than one, exactly one cell past one, and
+    several whose ends lie inside cells."""
+    from rtlib_b200.hashgrid import MortonQuadTrees
+    rng = np.random.default_rng(ncell)
+    n = 20000
+    m = MortonQuadTrees(ncell, level=level)
+    cell, uv, val = rng.integers(0, ncell, n).astype(np.uint32), rng.random((n, 2), dtype=np.float32), rng.random(n, dtype=np.float32)
+    cell[:2] = 0, ncell - 1
+    leaves = np.zeros(ncell << (2 * level), np.int64)
+    m.record(_t(cell, cuda), _t(uv, cuda), _t(val, cuda))
+    oracle.mqt_record(level, 24, leaves, cell, uv, val)
+    np.testing.assert_array_equal(m.export()[0], leaves)
+    m.update()
+    got_leaves, got = m.export()
+    assert not got_leaves.any()
+    np.testing.assert_array_equal(got, oracle.mqt_build(ncell, level, 24, leaves))
