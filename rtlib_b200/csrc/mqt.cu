@@ -43,8 +43,8 @@ __device__ __forceinline__ unsigned long long mqt_record_key(const MqtDev& t, in
 // queue up in L2 behind one another (and a look at the byte first finds the L1 line of the first
 // look), so each CTA remembers the cells it marked in a direct-mapped table in shared memory; large
 // CTAs share one table among many records.  2^22 records into 377 k / 1474 cells of 4^4 leaves:
-// 258 / 255 us aggregated and without
-// marks, 150 / 97 us now (139 / 75 us without marks).
+// 258 / 255 us aggregated and without marks, 150 / 97 us here with the cells' flags side by side (139 / 75 us
+// without marks); mqt_touched_shift spreads them since.
 constexpr int kRecThreads = 1024;
 constexpr uint32_t kRecTags = 8192;  // 32 KB, two CTAs per SM
 __global__ void __launch_bounds__(kRecThreads) k_mqt_record(MqtDev t, int64_t n, const uint32_t* __restrict__ cell,
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(kRecThreads) k_mqt_record_private(MqtDev t, in
         const unsigned long long v = ((unsigned long long)hi[k] << 32) | lo[k];
         if (!v) continue;
         atomicAdd(t.leaves + k, v);
-        t.touched[k >> (2 * t.level)] = 1;
+        t.touched[size_t(k >> (2 * t.level)) << t.touched_shift] = 1;
     }
 }
 
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(32 * kMqtWarps) k_mqt_build_small(MqtDev t) {
     const uint32_t nw = gridDim.x * kMqtWarps, per = 32 / G;
     for (uint32_t base = (blockIdx.x * kMqtWarps + (threadIdx.x >> 5)) * per; base < t.ncells; base += nw * per) {
         const uint32_t c = base + lane / G;
-        const bool touched = c < t.ncells && t.touched[c], live = c < t.ncells && t.live[c];
+        const bool touched = c < t.ncells && t.touched[size_t(c) << t.touched_shift], live = c < t.ncells && t.live[c];
         if (!__any_sync(0xffffffffu, touched || live)) continue;
         unsigned long long v[4] = {0ull, 0ull, 0ull, 0ull};
         unsigned long long* lf = t.leaves + size_t(c) * NLEAF + 4 * g;
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(32 * kMqtWarps) k_mqt_build_small(MqtDev t) {
         }
         __syncwarp();
         if (out && g == 0) {
-            t.touched[c] = 0;
+            t.touched[size_t(c) << t.touched_shift] = 0;
             t.live[c] = touched ? 1 : 0;
         }
     }
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(32 * kMqtWarps) k_mqt_build_warp(MqtDev t) {
     for (uint32_t base = (blockIdx.x * kMqtWarps + (threadIdx.x >> 5)) * 8; base < t.ncells; base += nw * 8) {
         const uint32_t c0 = base + lane;
         const bool mine = lane < 8 && c0 < t.ncells;
-        const bool touched = mine && t.touched[c0], live = mine && t.live[c0];
+        const bool touched = mine && t.touched[size_t(c0) << t.touched_shift], live = mine && t.live[c0];
         const unsigned read = __ballot_sync(0xffffffffu, touched);
         for (unsigned todo = __ballot_sync(0xffffffffu, touched || live); todo; todo &= todo - 1) {
             const uint32_t k = __ffs(todo) - 1;
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(32 * kMqtWarps) k_mqt_build_warp(MqtDev t) {
                                  (read >> k) & 1u, t.fx);
         }
         if (touched || live) {
-            t.touched[c0] = 0;
+            t.touched[size_t(c0) << t.touched_shift] = 0;
             t.live[c0] = touched ? 1 : 0;
         }
     }
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(L == 6 ? 128 : 512) k_mqt_build_block(MqtDev t
     __shared__ unsigned long long s_sum[W];
     const uint32_t warp = threadIdx.x >> 5;
     for (uint32_t c = blockIdx.x; c < t.ncells; c += gridDim.x) {
-        const bool touched = t.touched[c], live = t.live[c];
+        const bool touched = t.touched[size_t(c) << t.touched_shift], live = t.live[c];
         if (!touched && !live) continue;
         float* w = t.pyramid + size_t(c) * mqt_stride(L);
         const unsigned long long s = mqt_build_subtree<5>(t.leaves + (size_t(c) << (2 * L)) + size_t(warp) * 1024, w, TOP, warp,
@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(L == 6 ? 128 : 512) k_mqt_build_block(MqtDev t
             unsigned long long r = 0;
             for (uint32_t k = 0; k < W; ++k) r += s_sum[k];
             w[mqt_base(0)] = fx_to_float(r, t.fx);
-            t.touched[c] = 0;
+            t.touched[size_t(c) << t.touched_shift] = 0;
             t.live[c] = touched ? 1 : 0;
         }
         __syncthreads();
@@ -356,18 +356,19 @@ int rtpg_mqt_create(uint32_t num_cells, uint32_t level, float fraction, int32_t 
     t.ncells = num_cells;
     t.level = level;
     t.fraction = fraction;
+    t.touched_shift = mqt_touched_shift(num_cells);
     t.fx.scale = ldexpf(1.0f, fixed_point_bits);
     t.fx.inv_scale = ldexpf(1.0f, -fixed_point_bits);
     const size_t nleaf = (size_t)num_cells << (2 * level), npyr = (size_t)num_cells * mqt_stride(level);
     int r;
     if ((r = h->alloc(&t.leaves, nleaf)) || (r = h->alloc(&t.pyramid, npyr)) || (r = h->alloc(&t.status, 1)) ||
-        (r = h->alloc(&t.touched, num_cells)) || (r = h->alloc(&t.live, num_cells)) ||
+        (r = h->alloc(&t.touched, (size_t)num_cells << t.touched_shift)) || (r = h->alloc(&t.live, num_cells)) ||
         (r = h->alloc(&h->staging, std::min<size_t>(kExportFloats, (size_t)num_cells * mqt_level_offset(level + 1))))) {
         delete h;
         return r;
     }
     if (cudaMemset(t.leaves, 0, nleaf * 8) != cudaSuccess || cudaMemset(t.pyramid, 0, npyr * 4) != cudaSuccess ||
-        cudaMemset(t.status, 0, 4) != cudaSuccess || cudaMemset(t.touched, 0, num_cells) != cudaSuccess ||
+        cudaMemset(t.status, 0, 4) != cudaSuccess || cudaMemset(t.touched, 0, (size_t)num_cells << t.touched_shift) != cudaSuccess ||
         cudaMemset(t.live, 0, num_cells) != cudaSuccess) {
         delete h;
         return fail(RTPG_ECUDA, "rtpg_mqt_create: memset failed");
@@ -395,7 +396,7 @@ int rtpg_mqt_clear(rtpg_mqt* h, void* stream) {
     const MqtDev& t = h->dev;
     RTPG_CUDA(cudaMemsetAsync(t.leaves, 0, ((size_t)t.ncells << (2 * t.level)) * 8, st));
     RTPG_CUDA(cudaMemsetAsync(t.pyramid, 0, (size_t)t.ncells * mqt_stride(t.level) * 4, st));
-    RTPG_CUDA(cudaMemsetAsync(t.touched, 0, t.ncells, st));
+    RTPG_CUDA(cudaMemsetAsync(t.touched, 0, (size_t)t.ncells << t.touched_shift, st));
     RTPG_CUDA(cudaMemsetAsync(t.live, 0, t.ncells, st));
     RTPG_CUDA(cudaMemsetAsync(t.status, 0, 4, st));
     return RTPG_OK;

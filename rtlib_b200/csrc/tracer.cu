@@ -999,7 +999,7 @@ __global__ void __launch_bounds__(kCommitThreads) k_commit(TracerDev T) {
             if (k_s != ~0ull) {
                 atomicAdd(T.mqt.leaves + k_s, v_s);
                 // a look first: a wave's vertices meet a cell a few times each, not thousands
-                uint8_t* const touched = T.mqt.touched + (k_s >> (2 * T.mqt.level));
+                uint8_t* const touched = T.mqt.touched + ((k_s >> (2 * T.mqt.level)) << T.mqt.touched_shift);
                 if (!*touched) *touched = 1;
             }
         } else {
