@@ -1190,9 +1190,15 @@ static int timed_wave(rtpg_tracer* h, cudaStream_t st) {
 // Whether waves of this tracer run a path per thread (k_path) instead of a launch per bounce: while
 // the paths fit seven of the eight CTAs an SM holds.  Guided Cornell passes (63 spp): 65 k paths 12.7
 // -> 10.5 ms, 144 k 16.4 -> 16.8 ms; hash-grid passes over 100 k triangles: 14 k paths 18.2 -> 14.0
-// ms, 130 k 29.2 -> 27.1 ms.  The learned guide needs its network between bounces.
-constexpr uint32_t kWholePaths = kSMs * 7 * kTB;
-static bool whole_paths(const TracerDev& T) { return T.npath <= kWholePaths && guide_of(T.flags) != kGuideMlp; }
+// ms, 130 k 29.2 -> 27.1 ms.  The learned guide needs its network between bounces.  RIS in flat scenes (32
+// candidates of arithmetic where others wait for the closest hit) gains from compaction earlier, above five
+// CTAs: 4 samples of the Cornell box at 90 k paths 1718 -> 1682 us, at 102 k 1841 -> 1933, at 116 k 1974 -> 2216;
+// guided passes (15 spp) at 90 k 8.31 -> 7.89 ms, at 102 k 8.84 -> 8.92, at 116 k 9.57 -> 10.3.
+constexpr uint32_t kWholePaths = kSMs * 7 * kTB, kWholePathsRis = kSMs * 5 * kTB;
+static bool whole_paths(const TracerDev& T) {
+    const bool ris = T.nflat && (T.flags & RTPG_TRACE_FLAG_RIS);
+    return T.npath <= (ris ? kWholePathsRis : kWholePaths) && guide_of(T.flags) != kGuideMlp;
+}
 // In flat scenes of so few paths that an SM holds ten warps of them at most, four lanes share a path:
 // each tests a quarter of the triangles, all of them shade (what else would these schedulers issue).
 // One sample of the Cornell box with a lane a path -> four, NEE and RIS with 32 candidates: 256 paths

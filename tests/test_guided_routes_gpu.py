@@ -67,9 +67,10 @@ def _same_render(a, b):
     assert a.counters() == b.counters() and a.stats() == b.stats()
 
 
-# four lanes a path; a lane a path; a launch per bounce (past 7 CTAs of 128 paths per SM); and scenes
-# that rays walk a hierarchy in
-ROUTES = [("flat", 48, 48), ("flat", 149, 80), ("flat", 148 * 7, 129), ("rooms", 64, 36), ("rooms", 300, 200)]
+# four lanes a path; a lane a path; both sides of the limit for RIS (5 CTAs of 128 paths per SM); a launch
+# per bounce (past 7 of them); and scenes that rays walk a hierarchy in
+ROUTES = [("flat", 48, 48), ("flat", 149, 80), ("flat", 148 * 5, 128), ("flat", 148 * 5, 129), ("flat", 148 * 7, 129),
+          ("rooms", 64, 36), ("rooms", 300, 200)]
 
 
 @pytest.mark.parametrize("kind,w,h", ROUTES)
