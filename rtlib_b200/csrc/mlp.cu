@@ -126,9 +126,9 @@ __device__ __forceinline__ float head_grad(const float* o, bool hi, float3 wi, f
     return -__logf(q);
 }
 
-// Sum of the first `parts` floats of p, the same in every lane (fixed order).  The whole warp calls it.
-__device__ __forceinline__ float warp_sum_parts(const float* p, int parts) {
-    float s = 0.0f;
+// Sum of the first `parts` of p, the same in every lane (fixed order).  The whole warp calls it.
+__device__ __forceinline__ double warp_sum_parts(const double* p, int parts) {
+    double s = 0.0;
     for (int k = threadIdx.x & 31; k < parts; k += 32) s += p[k];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     return s;
@@ -137,7 +137,8 @@ __device__ __forceinline__ float warp_sum_parts(const float* p, int parts) {
 // One pass over n records: forward, loss gradient, backward; dW of all layers accumulate in
 // TMEM across the CTA's tiles and go to the CTA's row of grad_rows (fp32, [in][out] per layer) at the
 // end, its share of the loss to loss_rows; k_mlp_adam or k_mlp_add_grads sums the rows.  wsum: the
-// minibatch's weight sum in wparts parts (k_wsum).  No sum depends on the order in which CTAs finish:
+// minibatch's weight sum in wparts parts (k_wsum), in double: one unit in the last place of the float it
+// becomes moves some twenty of a minibatch's output gradients to another bf16 value.  No sum depends on the order in which CTAs finish:
 // Adam divides a gradient by its own size, so what the order of float atomics left in the last bits
 // grew to 4e-4 of the parameters within 16 steps.
 // A minibatch gives each CTA one tile, so its time is that tile's chain of phases: features, eight
@@ -146,7 +147,7 @@ __device__ __forceinline__ float warp_sum_parts(const float* p, int parts) {
 // that still runs (records and wsum are ready before the first launch of a call).  16 steps of 16384
 // records: 574 us with 128 threads per tile and a memset, a weight sum and an Adam launched one after
 // the other around it, 320 us now.
-__global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t n, Records R, const float* wsum, int wparts,
+__global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t n, Records R, const double* wsum, int wparts,
                                                             float* __restrict__ grad_rows, float* __restrict__ loss_rows) {
     extern __shared__ __align__(128) uint8_t sm[];
     __nv_bfloat16* ws = reinterpret_cast<__nv_bfloat16*>(sm);
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t 
     if (t == 0) mbar_init(mbar, 1);
     const uint32_t sw = smem_u32(ws), sx = smem_u32(x0), sdy = smem_u32(dy);
     const uint32_t sh[3] = {smem_u32(hs[0]), smem_u32(hs[1]), smem_u32(hs[2])};
-    const float total = warp_sum_parts(wsum, wparts);
+    const float total = (float)warp_sum_parts(wsum, wparts);
     const float scale = total > 0.0f ? 1.0f / total : 0.0f;
     // record weights are Monte Carlo estimates with a heavy tail: clamp at kWeightClamp times
     // their mean so that single rare paths do not dominate a step
@@ -300,12 +301,12 @@ __global__ void __launch_bounds__(kMlpThreads, 1) k_mlp_train(MlpDev P, int64_t 
 // Sums of the nonnegative weights of gridDim.y minibatches of `batch` records (the last shorter), each
 // in gridDim.x parts, kWsumParts apart.
 constexpr int kWsumParts = 64, kWsumBlock = 256;
-__global__ void __launch_bounds__(kWsumBlock) k_wsum(int64_t n, int64_t batch, const float* w, float* out) {
-    __shared__ float s_w[kWsumBlock / 32];
+__global__ void __launch_bounds__(kWsumBlock) k_wsum(int64_t n, int64_t batch, const float* w, double* out) {
+    __shared__ double s_w[kWsumBlock / 32];
     const int64_t b0 = blockIdx.y * batch, m = min(batch, n - b0);
-    float s = 0.0f;
+    double s = 0.0;
     for (int64_t i = blockIdx.x * int64_t(kWsumBlock) + threadIdx.x; i < m; i += int64_t(gridDim.x) * kWsumBlock)
-        s += fmaxf(w[b0 + i], 0.0f);
+        s += (double)fmaxf(w[b0 + i], 0.0f);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) s_w[threadIdx.x >> 5] = s;
     __syncthreads();
@@ -393,18 +394,18 @@ __global__ void __launch_bounds__(32 * kGradWarps) k_mlp_adam(GradRows r, float*
 using namespace rtpg;
 
 constexpr int64_t kMlpGroup = 256;  // minibatches whose weights are summed in one launch
-// scratch of training: weight sums of a group of minibatches in parts, a CTA's share of the loss and
-// gradient row each for a launch of k_mlp_train (9.8 MB)
-constexpr size_t kLossRows = kMlpGroup * kWsumParts, kGradRowsAt = kLossRows + 256,
-                 kTrainScratch = kGradRowsAt + size_t(kSMs) * kMlpParams;
+// scratch of training: weight sums of a group of minibatches in parts (double), a CTA's share of the loss and
+// gradient row each for a launch of k_mlp_train (float; 9.9 MB in all, in doubles)
+constexpr size_t kLossRows = kMlpGroup * kWsumParts, kGradRowsAt = kLossRows + 128,
+                 kTrainScratch = kGradRowsAt + size_t(kSMs) * kMlpParams / 2;
 static_assert(kSMs <= 256, "loss shares");
 
 struct rtpg_mlp {
     MlpDev dev{};
     float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
-    float* loss = nullptr;     // of the newest step, behind the gradients
-    float* scratch = nullptr;  // kTrainScratch floats (scratch_alloc)
-    int device = 0;            // of scratch
+    float* loss = nullptr;      // of the newest step, behind the gradients
+    double* scratch = nullptr;  // kTrainScratch (scratch_alloc)
+    int device = 0;             // of scratch
     __nv_bfloat16* wq = nullptr;
     float lr = 1e-3f, b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     uint32_t step = 0;
@@ -440,7 +441,7 @@ struct rtpg_mlp {
     }
 };
 
-// Training scratch comes from a pool of its own on each device: mapping and unmapping 9.8 MB by cudaMalloc
+// Training scratch comes from a pool of its own on each device: mapping and unmapping 9.9 MB by cudaMalloc
 // and cudaFree costs 0.7 ms a guide, as much as all else in creating it.  The pool keeps at most
 // kScratchKept bytes that no guide uses.
 constexpr uint64_t kScratchKept = 32u << 20;
@@ -461,11 +462,11 @@ static int scratch_alloc(rtpg_mlp* h) {
         RTPG_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept));
     }
     h->device = dev;
-    const cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&h->scratch), sizeof(float) * kTrainScratch, pool, nullptr);
+    const cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&h->scratch), sizeof(double) * kTrainScratch, pool, nullptr);
     if (e != cudaSuccess) {
         cudaGetLastError();
         h->scratch = nullptr;
-        return fail(RTPG_ENOMEM, "rtpg_mlp_create: %zu bytes of training scratch: %s", sizeof(float) * kTrainScratch,
+        return fail(RTPG_ENOMEM, "rtpg_mlp_create: %zu bytes of training scratch: %s", sizeof(double) * kTrainScratch,
                     cudaGetErrorString(e));
     }
     return RTPG_OK;
@@ -612,8 +613,8 @@ static int mlp_group(rtpg_mlp* h, int64_t n, int64_t batch, const float* w, cuda
 static int mlp_grad(rtpg_mlp* h, int64_t k, int64_t n, int64_t batch, const Records& R, bool chained, GradRows& rows,
                     cudaStream_t st) {
     const int g = (int)std::min<int64_t>((n + kMlpTile - 1) / kMlpTile, kSMs);
-    const float* const wsum = h->scratch + k * kWsumParts;
-    float *const grads = h->scratch + kGradRowsAt, *const loss = h->scratch + kLossRows;
+    const double* const wsum = h->scratch + k * kWsumParts;
+    float *const grads = reinterpret_cast<float*>(h->scratch + kGradRowsAt), *const loss = reinterpret_cast<float*>(h->scratch + kLossRows);
     if (chained) {
         RTPG_CUDA(launch_dependent(k_mlp_train, g, kMlpThreads, kSmemTrain, st, h->dev, n, R, wsum, wsum_parts(batch), grads, loss));
     } else {
